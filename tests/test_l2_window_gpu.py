@@ -1,6 +1,8 @@
 """L2 persistence windows: tables that fit in the device's persisting-L2
 maximum launch with an access-policy window, larger ones without, and the
 answers are the same with windows on and off."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -96,3 +98,17 @@ def test_windows_share_the_set_aside():
     del tables[0]
     extra = wc.SingleValueHashTable((16 << 20) // 8 - 4096, key_bytes=4)
     assert extra.l2_window()[0] > 0
+
+
+def test_set_aside_leaves_l2_to_the_other_tables():
+    # the set-aside shrinks L2 for the writes of every other array: a small
+    # table's window must not take more than a quarter of it (a sixth is
+    # asked for, rounded up by the device to its step)
+    t = wc.SingleValueHashTable(1 << 16, key_bytes=4)
+    assert t.l2_window()[0] > 0
+    limit = ctypes.c_size_t()
+    CU_LIMIT_PERSISTING_L2_CACHE_SIZE = 6
+    assert ctypes.CDLL("libcuda.so.1").cuCtxGetLimit(
+        ctypes.byref(limit), CU_LIMIT_PERSISTING_L2_CACHE_SIZE) == 0
+    l2 = torch.cuda.get_device_properties(0).L2_cache_size
+    assert t.l2_window()[0] <= limit.value <= l2 // 4
