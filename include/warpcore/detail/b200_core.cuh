@@ -156,6 +156,35 @@ __host__ __device__ __forceinline__ uint64_t fast_mod(uint64_t x, uint64_t d, ui
     return r >= d ? r - d : r;
 }
 
+__host__ __device__ __forceinline__ uint32_t mulhi32(uint32_t a, uint32_t b)
+{
+#ifdef __CUDA_ARCH__
+    return __umulhi(a, b);
+#else
+    return uint32_t((uint64_t(a) * b) >> 32);
+#endif
+}
+
+/* the same for a 32-bit x (every hash of a 4-byte key): the upper half of
+ * the 64-bit magic is floor((2^32 - 1) / d), so the reduction takes one
+ * 32-bit multiply-high instead of a 64-bit one (which is four multiplies
+ * and their carries); x is below a divisor of more than 32 bits */
+__host__ __device__ __forceinline__ uint64_t fast_mod32(uint32_t x, uint64_t d, uint64_t magic)
+{
+    if (d >> 32) return x;
+    const uint32_t d32 = uint32_t(d);
+    const uint32_t r = x - mulhi32(x, uint32_t(magic >> 32)) * d32;
+    return r >= d32 ? r - d32 : r;
+}
+
+/* the hash of a key reduced modulo d: hash_key of a 4-byte key is below 2^32 */
+template <class K>
+__host__ __device__ __forceinline__ uint64_t mod_hash(uint64_t h, uint64_t d, uint64_t magic)
+{
+    if constexpr (sizeof(K) == 4) return fast_mod32(uint32_t(h), d, magic);
+    else return fast_mod(h, d, magic);
+}
+
 /* ------------------------------------------------------------------ */
 /* table view and bucket probing                                        */
 /* ------------------------------------------------------------------ */
@@ -189,7 +218,7 @@ template <class K>
 __host__ __device__ __forceinline__ uint64_t probe_begin(const TableView &t, K key)
 {
     const K k = K(key + K(t.seed));
-    return fast_mod(hash_key<K>(t.hasher1, k), t.num_buckets, t.magic_nb);
+    return mod_hash<K>(hash_key<K>(t.hasher1, k), t.num_buckets, t.magic_nb);
 }
 
 template <class K>
@@ -197,7 +226,7 @@ __host__ __device__ __forceinline__ uint64_t probe_step(const TableView &t, K ke
 {
     if (t.probing != kProbeDouble || t.num_buckets < 2) return 1;
     const K k = K(key + K(t.seed) + K(1));
-    return fast_mod(hash_key<K>(t.hasher2, k), t.num_buckets - 1, t.magic_nb1) + 1;
+    return mod_hash<K>(hash_key<K>(t.hasher2, k), t.num_buckets - 1, t.magic_nb1) + 1;
 }
 
 /* advance to the next bucket; `step` grows by one per window for

@@ -308,7 +308,7 @@ int wc_mvht_num_values(wc_table *t, const void *keys_in, uint64_t num_in, uint64
  * values_out[begin_offsets_out[i] .. end_offsets_out[i]); *num_out (host)
  * gets the total.  With values_out NULL it is a dry run: end_offsets_out
  * gets the per-key counts (not summed), every status is dry_run.  The
- * offsets are uint64; synchronises `stream` before the values pass. */
+ * offsets are uint64; synchronises `stream`. */
 int wc_mvht_retrieve(wc_table *t, const void *keys_in, uint64_t num_in,
                      uint64_t *begin_offsets_out, uint64_t *end_offsets_out, void *values_out,
                      uint64_t *num_out, wc_stream_t stream, uint64_t probing_length,

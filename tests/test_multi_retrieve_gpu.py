@@ -1,0 +1,98 @@
+"""The one-pass lookup of the multi-value, multi-bucket and bucket-list
+tables at the edges of its tiles: query counts around a block's threads, a
+full tile and a full wave, more windows with values than a tile can note,
+and a key with more values than a note's position holds."""
+import numpy as np
+import pytest
+import torch
+
+import warpcore_b200 as wc
+from oracle import oracle as o
+from tests.wc_helpers import dev, empty_dev, host
+
+pytestmark = pytest.mark.gpu
+
+DT = {4: np.uint32, 8: np.uint64}
+
+
+def make(kind, kb, vb, nkeys, per, load=0.8):
+    if kind == "mv":
+        return wc.MultiValueHashTable(int(nkeys * per / load), key_bytes=kb, value_bytes=vb)
+    if kind == "mb":
+        return wc.MultiBucketHashTable(int(nkeys * -(-per // 4) / load), key_bytes=kb,
+                                       value_bytes=vb, bucket_size=4)
+    return wc.BucketListHashTable(int(nkeys / load), 4 * nkeys * per, key_bytes=kb, value_bytes=vb)
+
+
+def retrieve(t, queries, total, vb, joined=False):
+    n = len(queries)
+    off = torch.full((n + 1,), -7, dtype=torch.int64, device="cuda")
+    begin, end = off[:n], off[1:]
+    if not joined:
+        begin = torch.full((n,), -7, dtype=torch.int64, device="cuda")
+    out = empty_dev(max(total, 1), vb)
+    st = empty_dev(n, 4)
+    num = t.retrieve(dev(queries), begin, end, out, status_out=st)
+    return num, host(begin).astype(np.int64), host(end).astype(np.int64), host(out)[:num], host(st)
+
+
+@pytest.mark.parametrize("kind", ["mv", "mb", "bl"])
+@pytest.mark.parametrize("kb,vb", [(4, 4), (8, 8), (4, 8), (8, 4)])
+def test_tile_edges(kind, kb, vb):
+    nkeys, per = 3000, 5
+    both = o.gen_unique_keys(kb, 2 * nkeys, 77)
+    keys = both[:nkeys]
+    rng = np.random.default_rng(5)
+    values = rng.integers(1, 2**31, size=(nkeys, per)).astype(DT[vb])
+    t = make(kind, kb, vb, nkeys, per)
+    for j in range(per):  # one value of each key per round: the order is known
+        t.insert(dev(keys), dev(np.ascontiguousarray(values[:, j])))
+    # a bucket list is read newest bucket first: buckets of 1, 2, 3 values
+    order = [3, 4, 1, 2, 0] if kind == "bl" else range(per)
+    for n in (1, 31, 255, 256, 257, 1024, 1025, 148 * 4 * 256 + 1, 148 * 4 * 1024 + 1025):
+        at = rng.integers(0, 2 * nkeys, size=n)
+        hit = at < nkeys
+        cnt = np.where(hit, per, 0)
+        num, b, e, v, st = retrieve(t, both[at], int(cnt.sum()), vb, joined=n % 2 == 1)
+        assert num == cnt.sum()
+        assert np.array_equal(e, np.cumsum(cnt))
+        assert np.array_equal(b, np.cumsum(cnt) - cnt)
+        assert np.array_equal(v.view(DT[vb]), values[at[hit]][:, list(order)].reshape(-1))
+        assert np.array_equal(st, np.where(hit, 0, 1 << 5))
+        counts = torch.zeros(n, dtype=torch.int64, device="cuda")
+        assert t.num_values(dev(both[at]), counts) == num
+        assert np.array_equal(host(counts).astype(np.int64), cnt)
+
+
+@pytest.mark.parametrize("kind", ["mv", "mb"])
+@pytest.mark.parametrize("kb", [4, 8])
+def test_more_windows_than_notes(kind, kb):
+    # 60 values in windows of 8 (or buckets of 4 in such windows): more than
+    # the two notes per key that a tile holds, so keys are walked again
+    nkeys, per = 2048, 60
+    keys = o.gen_unique_keys(kb, nkeys, 78)
+    rng = np.random.default_rng(6)
+    values = rng.integers(1, 2**31, size=(nkeys, per)).astype(DT[kb])
+    t = make(kind, kb, kb, nkeys, per, load=0.9)
+    for j in range(per):
+        t.insert(dev(keys), dev(np.ascontiguousarray(values[:, j])))
+    q = np.concatenate([keys] * 80)  # full tiles, every query present
+    num, b, e, v, _ = retrieve(t, q, len(q) * per, kb)
+    assert num == len(q) * per
+    assert np.array_equal(e, (np.arange(len(q)) + 1) * per)
+    assert np.array_equal(v.view(DT[kb]), np.concatenate([values.reshape(-1)] * 80))
+
+
+def test_key_with_more_values_than_a_note_counts():
+    n, extra = 40000, 1000
+    keys = o.gen_unique_keys(4, extra + 1, 79)
+    t = wc.MultiValueHashTable(int((n + extra) / 0.5), key_bytes=4)
+    vals = np.arange(1, n + 1, dtype=np.uint32)
+    t.insert(dev(keys[1:]), dev(vals[:extra]))
+    t.insert(dev(np.full(n, keys[0], dtype=np.uint32)), dev(vals))
+    q = np.concatenate([keys[1:], keys[:1], keys[1:]])
+    num, b, e, v, _ = retrieve(t, q, n + 2 * extra, 4)
+    assert num == n + 2 * extra
+    assert np.array_equal(v[:extra], vals[:extra])
+    assert np.array_equal(np.sort(v[extra:extra + n].view(np.uint32)), vals)
+    assert np.array_equal(v[extra + n:], vals[:extra])

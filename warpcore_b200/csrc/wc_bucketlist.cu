@@ -48,30 +48,9 @@ int bl_fail(int code, const char *msg) { return host_fail(code, msg); }
 
 uint64_t kmask(uint32_t bytes) { return bytes == 4 ? 0xffffffffull : ~0ull; }
 
-struct BlArgs {
+struct BlArgs : MultiArgs {
     BlView v;
-    const void *keys;
-    const void *values;              /* insert */
-    void *values_out;                /* retrieve */
-    const unsigned long long *begin;
-    const unsigned long long *end;
-    unsigned long long *counts_out;
-    unsigned long long *total;
-    void *status_out;
-    uint64_t n;
-    uint64_t max_windows;
-    uint32_t bool_mask;
-    int handler;
 };
-
-__device__ __forceinline__ void bl_write_status(const BlArgs &a, uint64_t i, uint32_t st)
-{
-    if (!a.status_out) return;
-    if (a.handler == kHandlerStatus)
-        reinterpret_cast<uint32_t *>(a.status_out)[i] = st;
-    else if (a.handler == kHandlerBoolean)
-        reinterpret_cast<unsigned char *>(a.status_out)[i] = (unsigned char)((st & a.bool_mask) != 0);
-}
 
 /* bulk insert (:235-326).  Unlike the reference kernel, which leaves the
  * status of a key without a slot (invalid key, probing length exceeded)
@@ -87,48 +66,130 @@ __global__ void __launch_bounds__(256, WC_MULTI_MIN_BLOCKS) bl_insert_kernel(con
                                                     reinterpret_cast<const V *>(a.values)[i],
                                                     a.max_windows, j);
         join |= j;
-        bl_write_status(a, i, st);
+        multi_write_status(a, i, st);
     }
     const uint32_t wj = __reduce_or_sync(0xffffffffu, join); /* every lane arrives */
     if ((threadIdx.x & 31) == 0) join_status(a.v.t.status, wj);
 }
 
-/* num_values (kValues false) or retrieve (gpu_engine.cuh:305-346) */
-template <class K, class V, int kW, bool kValues>
-__global__ void __launch_bounds__(256, WC_MULTI_MIN_BLOCKS) bl_find_kernel(const BlArgs a)
-{
-    uint32_t join = 0;
-    unsigned long long total = 0;
-    const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < a.n; i += stride) {
-        uint64_t num = 0;
-        const K key = reinterpret_cast<const K *>(a.keys)[i];
-        if constexpr (kValues) {
-            /* The counting pass looked every key up and wrote its status;
-             * this pass only reads lists.  A key counted at 0 needs no
-             * lookup.  Values go inside the key's own segment only. */
-            const uint64_t room = a.end[i] - a.begin[i];
-            if (room == 0) continue;
-            V *const out = reinterpret_cast<V *>(a.values_out) + a.begin[i];
-            bl_for_each_one<K, V, kW, true>(a.v, key, a.max_windows, num, [&](V x, uint64_t j) {
-                if (j < room) out[j] = x;
-            });
-        } else {
-            const uint32_t st = bl_for_each_one<K, V, kW, false>(a.v, key, a.max_windows, num,
-                                                                 [](V, uint64_t) {});
-            join |= st;
-            if (a.counts_out) a.counts_out[i] = num;
-            total += num;
-            bl_write_status(a, i, st);
+/* the key's slot (as bl_find looks for it), then its handle, which holds the
+ * list's count, then for the values the list's buckets, newest first (as
+ * bl_walk reads them): a bucket's header and its first four values are read
+ * together, so a list costs one memory latency per bucket */
+template <class K, class V, int kW>
+struct BlWalk {
+    using key_t = K;
+    using val_t = V;
+    using Args = BlArgs;
+    struct State {
+        uint64_t bucket, step, wins, num;
+        uint64_t at;    /* the key's slot, then the list bucket's pool index */
+        uint64_t count; /* list: values in all; num: values read */
+        uint64_t size, read; /* list: values in the bucket (phase 3: at most), read of it */
+        int phase;      /* 0 windows, 1 handle, 2 list, 3 list, size still in the header */
+    };
+
+    static __device__ __forceinline__ const TableView &view(const Args &a) { return a.v.t; }
+
+    static __device__ __forceinline__ void start(const Args &a, K key, State &s)
+    {
+        s.bucket = probe_begin<K>(a.v.t, key);
+        s.step = 0;
+        s.wins = 0;
+        s.num = 0;
+        s.phase = 0;
+    }
+
+    static __device__ __forceinline__ bool count_step(const Args &a, K key, State &s, uint32_t &st)
+    {
+        if (s.phase == 0) return window(a, key, s, st);
+        s.num = bl_unpack(a.v, a.v.handles[s.at]).count;
+        st = kStNone;
+        return true;
+    }
+
+    static __device__ __forceinline__ bool value_step(const Args &a, K key, State &s, V *out,
+                                                      uint64_t room)
+    {
+        const BlView &v = a.v;
+        if (s.phase == 0) {
+            uint32_t st;
+            return window(a, key, s, st);
         }
+        if (s.phase == 1) {
+            const BlHandle c = bl_unpack(v, v.handles[s.at]);
+            if (c.state != kBlInit || c.index == bl_head(v.ib)) return true;
+            s.at = c.index;
+            s.count = c.count;
+            s.size = c.tail;
+            s.read = 0;
+            s.phase = 2;
+            return s.at >= v.capacity ||
+                   s.at + (c.count <= v.min_bucket ? 0 : 1) + c.tail > v.capacity;
+        }
+        /* the list's first bucket (the last one read) has no header; an
+         * older bucket is no larger than a newer one, so no value is read
+         * that lies beyond what the bucket may hold */
+        const bool last = s.count - s.num + s.read <= v.min_bucket;
+        const uint64_t first = s.at + (last ? 0 : 1);
+        if (last && s.phase == 3) s.size = v.min_bucket;
+        unsigned long long x[4];
+        const unsigned long long header = v.pool[s.at];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint64_t p = first + s.read + uint64_t(u);
+            x[u] = s.read + uint64_t(u) < s.size && p < v.capacity ? v.pool[p] : 0ull;
+        }
+        if (s.phase == 3) {
+            if (!last) s.size = bl_header_size(v, header);
+            s.phase = 2;
+            if (first + s.size > v.capacity) return true;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (s.read < s.size && s.num < s.count) {
+                if (s.num < room) out[s.num] = V(x[u]);
+                ++s.num;
+                ++s.read;
+            }
+        }
+        if (s.num >= s.count) return true;
+        if (s.read >= s.size) {
+            s.size = bl_header_size(v, header);
+            s.at = bl_header_prev(v, header);
+            s.read = 0;
+            s.phase = 3;
+            return s.at >= v.capacity;
+        }
+        return false;
     }
-    const uint32_t wj = __reduce_or_sync(0xffffffffu, join);
-    const unsigned long long sum = warp_sum_u64(total);
-    if ((threadIdx.x & 31) == 0) {
-        if (a.total && sum) atomicAdd(a.total, sum);
-        join_status(a.v.t.status, wj);
+
+    static __device__ __forceinline__ bool window(const Args &a, K key, State &s, uint32_t &st)
+    {
+        const TableView &t = a.v.t;
+        const uint32_t W = kW ? uint32_t(kW) : t.cg_size;
+        uint32_t hits;
+        bool free;
+        key_window<K, kW>(reinterpret_cast<const K *>(t.slots) + s.bucket * W, W, key,
+                          K(t.empty_key), hits, free);
+        if (hits) {
+            s.at = s.bucket * W + uint64_t(__ffs(hits) - 1);
+            s.phase = 1;
+            return false;
+        }
+        if (free) {
+            st = kStKeyNotFound;
+            return true;
+        }
+        if (++s.wins >= a.max_windows) {
+            st = kStProbingLengthExceeded;
+            return true;
+        }
+        if (s.wins == 1) s.step = probe_step<K>(t, key);
+        s.bucket = probe_next(t, s.bucket, s.step);
+        return false;
     }
-}
+};
 
 /* init: keys empty, handles uninitialized, pool headers {head, min}, next free 0 */
 template <class K>
@@ -169,15 +230,16 @@ __global__ void __launch_bounds__(256) bl_scan_keys_kernel(const BlView v, uint6
 }
 
 struct BlKernels {
-    const void *insert, *count, *values, *init, *scan;
+    const void *insert, *count, *offsets, *values, *init, *scan;
 };
 
 template <class K, class V, int kW>
 BlKernels bl_kernels_of()
 {
     return {reinterpret_cast<const void *>(bl_insert_kernel<K, V, kW>),
-            reinterpret_cast<const void *>(bl_find_kernel<K, V, kW, false>),
-            reinterpret_cast<const void *>(bl_find_kernel<K, V, kW, true>),
+            reinterpret_cast<const void *>(multi_find_kernel<BlWalk<K, V, kW>, false>),
+            reinterpret_cast<const void *>(multi_find_kernel<BlWalk<K, V, kW>, true>),
+            reinterpret_cast<const void *>(multi_values_kernel<BlWalk<K, V, kW>>),
             reinterpret_cast<const void *>(bl_init_kernel<K>),
             reinterpret_cast<const void *>(bl_scan_keys_kernel<K>)};
 }
@@ -267,19 +329,8 @@ int read_counter(const unsigned long long *d, cudaStream_t s, uint64_t *out)
 int count(wc_blht *t, const void *keys, uint64_t n, uint64_t *counts_dev, uint64_t *total,
           cudaStream_t s, uint64_t probing_length, void *status_out, int handler, uint32_t ignore)
 {
-    unsigned long long *tmp = t->counters + 1;
-    BL_CUDA(cudaMemsetAsync(tmp, 0, sizeof(unsigned long long), s));
     BlArgs a = args_of(t, keys, n, probing_length, status_out, handler, ignore);
-    a.counts_out = reinterpret_cast<unsigned long long *>(counts_dev);
-    a.total = tmp;
-    int rc = launch(bl_kernels(t).count, n, a, s);
-    if (rc) return rc;
-    return read_counter(tmp, s, total);
-}
-
-int scan(wc_blht *t, uint64_t *begin, uint64_t *end, uint64_t n, cudaStream_t s)
-{
-    return host_offsets_scan(&t->scan, &t->scan_bytes, begin, end, n, s);
+    return host_multi_count(bl_kernels(t).count, &a, &a, t->counters + 8, counts_dev, total, s);
 }
 
 int join_host(wc_blht *t, uint32_t bits, cudaStream_t s)
@@ -458,23 +509,18 @@ int wc_blht_retrieve(wc_blht *t, const void *keys_in, uint64_t num_in,
     if (!keys_in || !end_offsets_out || (values_out && !begin_offsets_out))
         return bl_fail(WC_ERR_INVALID_ARGUMENT, "NULL buffer");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    /* pass 1: counts, and each key's status (the values pass reads lists only) */
-    rc = count(t, keys_in, num_in, end_offsets_out, num_out, s, probing_length,
-               values_out ? status_out : nullptr, values_out ? status_handler : WC_HANDLER_NOTHING,
-               ignore);
-    if (rc) return rc;
     if (!values_out) {
+        rc = count(t, keys_in, num_in, end_offsets_out, num_out, s, probing_length, nullptr,
+                   WC_HANDLER_NOTHING, ignore);
+        if (rc) return rc;
         rc = host_dry_run_status(status_out, num_in, status_handler, ignore, s);
         if (rc) return rc;
         return join_host(t, kStDryRun, s);
     }
-    rc = scan(t, begin_offsets_out, end_offsets_out, num_in, s);
-    if (rc) return rc;
     BlArgs a = args_of(t, keys_in, num_in, probing_length, status_out, status_handler, ignore);
-    a.values_out = values_out;
-    a.begin = reinterpret_cast<const unsigned long long *>(begin_offsets_out);
-    a.end = reinterpret_cast<const unsigned long long *>(end_offsets_out);
-    return launch(bl_kernels(t).values, num_in, a, s);
+    const BlKernels k = bl_kernels(t);
+    return host_multi_retrieve(k.offsets, k.values, &a, &a, &t->scan, &t->scan_bytes,
+                               begin_offsets_out, end_offsets_out, values_out, num_out, s);
 }
 
 int wc_blht_retrieve_all_keys(wc_blht *t, void *keys_out, uint64_t *num_out, wc_stream_t stream)

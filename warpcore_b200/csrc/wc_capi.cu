@@ -379,15 +379,64 @@ uint64_t warpcore::b200::host_valid_capacity(uint64_t min_capacity, uint64_t cg)
     return valid_capacity(min_capacity, cg);
 }
 
-/* counts in end -> end = inclusive prefix sums, begin = exclusive ones (the
- * reference's cub::DeviceScan::InclusiveSum step): tile sums, tile offsets,
- * apply.  The tile-sum buffer grows on demand. */
-int warpcore::b200::host_offsets_scan(void **scratch, uint64_t *scratch_bytes, uint64_t *begin,
-                                      uint64_t *end, uint64_t n, cudaStream_t s)
+namespace {
+
+/* A tile is at most kMultiTile keys and small enough that every resident
+ * block gets one, in steps of a block's threads: a small call then walks one
+ * key per lane on all SMs, and a large one draws four keys per lane. */
+int multi_launch(const void *kernel, MultiArgs *a, void *args, cudaStream_t s)
 {
-    const MvScanKernels k = mv_scan_kernels();
-    const uint64_t ntiles = (n + kScanTile - 1) / kScanTile;
-    const uint64_t need = ntiles * sizeof(unsigned long long);
+    void *kargs[] = {args};
+    const uint64_t wave = uint64_t(device_props().sms) * blocks_per_sm(kernel, kMultiThreads);
+    const uint64_t ntiles = (a->n + a->tile - 1) / a->tile;
+    WC_CUDA(cudaLaunchKernel(kernel, dim3(unsigned(ntiles < wave ? ntiles : wave)),
+                             dim3(kMultiThreads), kargs, 0, s));
+    note_launches(1);
+    return WC_OK;
+}
+
+uint32_t multi_tile(const void *kernel, uint64_t n)
+{
+    const uint64_t wave = uint64_t(device_props().sms) * blocks_per_sm(kernel, kMultiThreads);
+    uint64_t tile = (n + wave - 1) / wave;
+    tile = (tile + kMultiThreads - 1) / kMultiThreads * kMultiThreads;
+    return uint32_t(tile < kMultiTile ? tile : kMultiTile);
+}
+
+/* the sum of the counts, read back */
+int multi_total(const MultiArgs *a, uint64_t *total, cudaStream_t s)
+{
+    unsigned long long h[kLookFailed + 1] = {0};
+    WC_CUDA(cudaMemcpyAsync(h, a->look, sizeof(h), cudaMemcpyDeviceToHost, s));
+    WC_CUDA(cudaStreamSynchronize(s));
+    if (h[kLookFailed])
+        return fail(WC_ERR_TIMEOUT, "retrieve: the wait for an earlier tile's offsets ran out");
+    *total = h[kLookTotal];
+    return WC_OK;
+}
+
+} // namespace
+
+int warpcore::b200::host_multi_count(const void *count_kernel, MultiArgs *a, void *args,
+                                     unsigned long long *look, uint64_t *counts, uint64_t *total,
+                                     cudaStream_t s)
+{
+    a->tile = multi_tile(count_kernel, a->n);
+    a->look = look;
+    a->counts_out = reinterpret_cast<unsigned long long *>(counts);
+    WC_CUDA(cudaMemsetAsync(look, 0, kLookTiles * sizeof(unsigned long long), s));
+    const int rc = multi_launch(count_kernel, a, args, s);
+    return rc ? rc : multi_total(a, total, s);
+}
+
+int warpcore::b200::host_multi_retrieve(const void *offsets_kernel, const void *values_kernel,
+                                        MultiArgs *a, void *args, void **scratch,
+                                        uint64_t *scratch_bytes, uint64_t *begin, uint64_t *end,
+                                        void *values_out, uint64_t *total, cudaStream_t s)
+{
+    a->tile = multi_tile(offsets_kernel, a->n);
+    const uint64_t ntiles = (a->n + a->tile - 1) / a->tile;
+    const uint64_t need = (kLookTiles + ntiles) * sizeof(unsigned long long);
     if (need > *scratch_bytes) {
         WC_CUDA(cudaStreamSynchronize(s));
         if (*scratch) cudaFree(*scratch);
@@ -396,21 +445,23 @@ int warpcore::b200::host_offsets_scan(void **scratch, uint64_t *scratch_bytes, u
         WC_CUDA(cudaMalloc(scratch, need));
         *scratch_bytes = need;
     }
-    auto *e = reinterpret_cast<unsigned long long *>(end);
-    auto *b = reinterpret_cast<unsigned long long *>(begin);
-    auto *ts = reinterpret_cast<unsigned long long *>(*scratch);
-    uint64_t nn = n, nt = ntiles;
-    void *a1[] = {&e, &nn, &ts};
-    WC_CUDA(cudaLaunchKernel(k.tile_sums, dim3(unsigned(ntiles)), dim3(kScanThreads), a1, 0, s));
-    void *a2[] = {&ts, &nt};
-    WC_CUDA(cudaLaunchKernel(k.tile_offsets, dim3(1), dim3(kScanThreads), a2, 0, s));
-    /* end == begin + 1: the scan writes end only, begin[0] is zero */
-    int write_begin = e == b + 1 ? 0 : 1;
-    if (!write_begin) WC_CUDA(cudaMemsetAsync(b, 0, sizeof(unsigned long long), s));
-    void *a3[] = {&e, &b, &nn, &ts, &write_begin};
-    WC_CUDA(cudaLaunchKernel(k.apply, dim3(unsigned(ntiles)), dim3(kScanThreads), a3, 0, s));
-    note_launches(3);
-    return WC_OK;
+    a->look = reinterpret_cast<unsigned long long *>(*scratch);
+    a->end_out = reinterpret_cast<unsigned long long *>(end);
+    a->begin_out = reinterpret_cast<unsigned long long *>(begin);
+    a->begin_first = nullptr;
+    if (end == begin + 1) {
+        /* the reference's offsets_out, offsets_out + 1 idiom: begin[i + 1]
+         * is end[i] already, and begin[0] is zero */
+        a->begin_first = a->begin_out;
+        a->begin_out = nullptr;
+    }
+    a->values_out = values_out;
+    WC_CUDA(cudaMemsetAsync(*scratch, 0, need, s));
+    int rc = multi_launch(offsets_kernel, a, args, s);
+    if (rc) return rc;
+    a->tile = multi_tile(values_kernel, a->n);
+    rc = multi_launch(values_kernel, a, args, s);
+    return rc ? rc : multi_total(a, total, s);
 }
 
 /* join bits into a device Status word from the host (synchronises) */
@@ -430,12 +481,12 @@ int warpcore::b200::host_dry_run_status(void *status_out, uint64_t n, int handle
                                         uint32_t ignore, cudaStream_t s)
 {
     if (!status_out || handler == WC_HANDLER_NOTHING || n == 0) return WC_OK;
-    const MvScanKernels k = mv_scan_kernels();
+    const void *const k = multi_dry_status_kernel_ptr();
     uint64_t nn = n;
     int h = handler;
     uint32_t mask = (~ignore) ^ 0xFFFu;
     void *args[] = {&status_out, &nn, &h, &mask};
-    WC_CUDA(cudaLaunchKernel(k.dry_status, dim3(grid_for(k.dry_status, kBlock, n, kBlock)),
+    WC_CUDA(cudaLaunchKernel(k, dim3(grid_for(k, kBlock, n, kBlock)),
                              dim3(kBlock), args, 0, s));
     note_launches(1);
     return WC_OK;
@@ -1288,30 +1339,16 @@ int mv_launch(const void *k, wc_table *t, uint64_t items, MvArgs &a, cudaStream_
     return WC_OK;
 }
 
-/* per-key counts (and their sum, read back to the host) */
+/* per-key counts (and their sum, read back to the host); the device block
+ * has 64 bytes at t->counter */
 int mv_count(wc_table *t, const void *keys, uint64_t n, uint64_t *counts_dev, uint64_t *total,
              cudaStream_t s, uint64_t probing_length, void *status_out, int handler,
              uint32_t ignore)
 {
     const MvKernels k = mv_kernels(t->layout, int(t->cfg.cg_size));
     if (!k.count) return fail(WC_ERR_UNSUPPORTED, "no kernel for this configuration");
-    WC_CUDA(cudaMemsetAsync(t->counter, 0, sizeof(unsigned long long), s));
     MvArgs a = mv_args(t, keys, n, probing_length, true, status_out, handler, ignore);
-    a.counts_out = reinterpret_cast<unsigned long long *>(counts_dev);
-    a.total = t->counter;
-    int rc = mv_launch(k.count, t, n, a, s);
-    if (rc) return rc;
-    unsigned long long h = 0;
-    WC_CUDA(cudaMemcpyAsync(&h, t->counter, sizeof(h), cudaMemcpyDeviceToHost, s));
-    WC_CUDA(cudaStreamSynchronize(s));
-    *total = h;
-    return WC_OK;
-}
-
-/* counts in end -> end = inclusive prefix sums, begin = exclusive ones */
-int mv_scan(wc_table *t, uint64_t *begin, uint64_t *end, uint64_t n, cudaStream_t s)
-{
-    return host_offsets_scan(&t->scratch, &t->scratch_bytes, begin, end, n, s);
+    return host_multi_count(k.count, &a, &a, t->counter, counts_dev, total, s);
 }
 
 int mv_join(wc_table *t, uint32_t bits, cudaStream_t s)
@@ -1366,28 +1403,21 @@ int wc_mvht_retrieve(wc_table *t, const void *keys_in, uint64_t num_in,
     if (!keys_in || !end_offsets_out || (values_out && !begin_offsets_out))
         return fail(WC_ERR_INVALID_ARGUMENT, "NULL buffer");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    /* pass 1: counts per key into end_offsets, and each key's status (the
-     * values pass reads values only) */
-    rc = mv_count(t, keys_in, num_in, end_offsets_out, num_out, s, probing_length,
-                  values_out ? status_out : nullptr,
-                  values_out ? status_handler : WC_HANDLER_NOTHING, ignore);
-    if (rc) return rc;
     if (!values_out) {
         /* dry run: per-key counts, status dry_run for every key */
+        rc = mv_count(t, keys_in, num_in, end_offsets_out, num_out, s, probing_length, nullptr,
+                      WC_HANDLER_NOTHING, ignore);
+        if (rc) return rc;
         rc = host_dry_run_status(status_out, num_in, status_handler, ignore, s);
         if (rc) return rc;
         return mv_join(t, kStDryRun, s);
     }
-    /* pass 2: offsets; pass 3: values, each key at its begin offset */
-    rc = mv_scan(t, begin_offsets_out, end_offsets_out, num_in, s);
-    if (rc) return rc;
     const MvKernels k = mv_kernels(t->layout, int(t->cfg.cg_size));
+    if (!k.values) return fail(WC_ERR_UNSUPPORTED, "no kernel for this configuration");
     MvArgs a = mv_args(t, keys_in, num_in, probing_length, true, status_out, status_handler,
                        ignore);
-    a.values_out = values_out;
-    a.begin = reinterpret_cast<const unsigned long long *>(begin_offsets_out);
-    a.end = reinterpret_cast<const unsigned long long *>(end_offsets_out);
-    return mv_launch(k.values, t, num_in, a, s);
+    return host_multi_retrieve(k.offsets, k.values, &a, &a, &t->scratch, &t->scratch_bytes,
+                               begin_offsets_out, end_offsets_out, values_out, num_out, s);
 }
 
 int wc_mvht_retrieve_all_keys(wc_table *t, void *keys_out, uint64_t *num_out, wc_stream_t stream)

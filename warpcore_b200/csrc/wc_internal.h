@@ -76,14 +76,12 @@ const void *batch_kernel_ptr(int layout, int W, bool inline_desc);
 /* MultiValueHashTable kernels of a layout (KV32 / KV64) and window width;
  * null pointers if not built */
 struct MvKernels {
-    const void *insert = nullptr, *count = nullptr, *values = nullptr, *unique = nullptr;
+    const void *insert = nullptr, *count = nullptr, *offsets = nullptr, *values = nullptr,
+               *unique = nullptr;
 };
 MvKernels mv_kernels(int layout, int W);
 MvKernels mv_kernels_mixed(int layout, int W); /* u32/u64 and u64/u32 */
-struct MvScanKernels {
-    const void *tile_sums, *tile_offsets, *apply, *dry_status;
-};
-MvScanKernels mv_scan_kernels();
+const void *multi_dry_status_kernel_ptr();
 
 /* message returned by wc_last_error() on the calling thread */
 void set_last_error(const char *msg);
@@ -95,11 +93,16 @@ int host_fail(int code, const char *msg);
 int host_cuda_fail(cudaError_t e, const char *what);
 unsigned host_grid(const void *kernel, int block, uint64_t items, uint64_t per_block);
 uint64_t host_valid_capacity(uint64_t min_capacity, uint64_t cg);
-/* the multi-value tables' shared host steps: per-key counts (in end) to
- * begin / end offsets, a host-side Status join, a dry run's statuses, one
- * device counter read back */
-int host_offsets_scan(void **scratch, uint64_t *scratch_bytes, uint64_t *begin, uint64_t *end,
-                      uint64_t n, cudaStream_t s);
+/* the multi-value tables' shared host steps: num_values / retrieve of the
+ * keys in a (the kernels of wc_multi.cuh, whose argument is *args, which
+ * starts with a), a host-side Status join, a dry run's statuses, one device
+ * counter read back.  host_multi_count uses the kLookTiles words at `look`,
+ * host_multi_retrieve a scratch array grown on demand; both synchronise. */
+int host_multi_count(const void *count_kernel, MultiArgs *a, void *args, unsigned long long *look,
+                     uint64_t *counts, uint64_t *total, cudaStream_t s);
+int host_multi_retrieve(const void *offsets_kernel, const void *values_kernel, MultiArgs *a,
+                        void *args, void **scratch, uint64_t *scratch_bytes, uint64_t *begin,
+                        uint64_t *end, void *values_out, uint64_t *total, cudaStream_t s);
 int host_join_status(uint32_t *status, uint32_t bits, cudaStream_t s);
 int host_dry_run_status(void *status_out, uint64_t n, int handler, uint32_t ignore, cudaStream_t s);
 int host_read_counter(const unsigned long long *d, cudaStream_t s, uint64_t *out);

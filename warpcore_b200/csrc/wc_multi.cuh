@@ -1,0 +1,416 @@
+/*
+ * wc_multi.cuh -- lookups of the tables that hold several values per key
+ * (multi-value, multi-bucket, bucket-list): the bulk num_values and the
+ * bulk retrieve (multi_value_hash_table.cuh:371-520,
+ * multi_bucket_hash_table.cuh:574-680, bucket_list_hash_table.cuh:337-466).
+ * What differs between the tables, how a key's values are found and read,
+ * comes from a Walk (MvWalk, MbWalk, BlWalk).
+ *
+ * The reference counts the values of every key, scans the counts into
+ * offsets and walks every key again to copy its values.  Here two kernels
+ * do it:
+ *   multi_find_kernel counts and makes the offsets.  A block takes a tile
+ *     of keys and walks them; the tile's counts are scanned in the block,
+ *     and the values of all earlier tiles are summed by looking back over
+ *     the tiles' published sums (one 64-bit word each: a tile's own sum,
+ *     then the sum up to its end).  Tiles are handed out in order by a
+ *     ticket, so a tile waits only for tiles that already run; the wait has
+ *     a limit all the same, after which the call reports a timeout.
+ *   multi_values_kernel walks the keys that have values, up to the window
+ *     where the last of them is, and copies the values as it meets them.
+ *
+ * Both are bound by the latency of the walks' dependent reads.  A walk ends
+ * at the first window with a free slot: at load 0.8 its mean is 2 to 3
+ * windows and the longest of 32 is 8 to 9, so a warp that keeps one key per
+ * lane until all are done leaves two lanes of three waiting.  Here each
+ * lane issues one memory operation per step (a window, a bucket, a handle,
+ * a list bucket) and a lane whose key is done draws the next key of the
+ * block's tile.
+ *
+ * Shared memory is kept small on purpose: reads in flight need L1 space.
+ * A form that noted the windows with values in shared memory while
+ * counting, and copied from the notes without a second walk, needed 37 KiB
+ * per block and ran slower the more blocks were resident (multi-value,
+ * 2^23 lookups, half present with 4 values each: 736 / 859 / 1366 us with
+ * 4 / 5 / 6 blocks per SM).
+ */
+#ifndef WC_MULTI_CUH
+#define WC_MULTI_CUH
+
+#include "wc_lane_kernels.cuh"
+#include <warpcore/detail/mb_ops.cuh>
+
+namespace warpcore {
+namespace b200 {
+
+/* resident 256-thread blocks per SM these kernels are built for */
+#ifndef WC_MULTI_MIN_BLOCKS
+#define WC_MULTI_MIN_BLOCKS 4 /* inserts */
+#endif
+#ifndef WC_MULTI_COUNT_BLOCKS
+#define WC_MULTI_COUNT_BLOCKS 6
+#endif
+#ifndef WC_MULTI_VALUES_BLOCKS
+#define WC_MULTI_VALUES_BLOCKS 5
+#endif
+
+/* what the bulk calls of all these tables pass */
+struct MultiArgs {
+    const void *keys;
+    const void *values;             /* insert */
+    void *values_out;               /* retrieve */
+    unsigned long long *begin_out;  /* retrieve: offsets; NULL where begin_out
+                                       would be end_out - 1 (begin_first) */
+    unsigned long long *end_out;
+    unsigned long long *begin_first;
+    unsigned long long *counts_out; /* num_values: per key, or NULL */
+    unsigned long long *look;       /* look-back words, see kLook* */
+    void *status_out;
+    uint64_t n;
+    uint64_t max_windows;
+    uint32_t tile;                  /* keys per tile, at most kMultiTile */
+    uint32_t bool_mask;
+    int handler;
+};
+
+/* keys per tile: four per thread, so that a lane draws a few times before
+ * the tile's last walks leave lanes idle */
+constexpr int kMultiTile = 1024;
+constexpr int kMultiThreads = 256;
+
+/* look-back words: ticket, total, timeout flag, then one word per tile */
+constexpr int kLookTicket = 0, kLookTotal = 1, kLookFailed = 2, kLookTiles = 4;
+constexpr unsigned long long kLookSum = 1ull << 62;  /* the tile's own sum */
+constexpr unsigned long long kLookEnd = 2ull << 62;  /* the sum up to its end */
+constexpr unsigned long long kLookBad = 3ull << 62;  /* a wait ran out */
+constexpr unsigned long long kLookMask = (1ull << 62) - 1;
+constexpr uint32_t kLookPolls = 1u << 21; /* of at least 64 ns each */
+
+__device__ __forceinline__ void multi_write_status(const MultiArgs &a, uint64_t i, uint32_t st)
+{
+    if (!a.status_out) return;
+    if (a.handler == kHandlerStatus)
+        reinterpret_cast<uint32_t *>(a.status_out)[i] = st;
+    else if (a.handler == kHandlerBoolean)
+        reinterpret_cast<unsigned char *>(a.status_out)[i] =
+            (unsigned char)((st & a.bool_mask) != 0);
+}
+
+__device__ __forceinline__ unsigned long long look_load(const unsigned long long *p)
+{
+    return *reinterpret_cast<const volatile unsigned long long *>(p);
+}
+__device__ __forceinline__ void look_store(unsigned long long *p, unsigned long long v)
+{
+    *reinterpret_cast<volatile unsigned long long *>(p) = v;
+}
+
+/* exclusive scan over the block of one value per thread; returns the total */
+__device__ __forceinline__ unsigned long long block_exclusive_scan(unsigned long long v,
+                                                                   unsigned long long &excl)
+{
+    __shared__ unsigned long long warp_sums[32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    unsigned long long x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(kFull, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) warp_sums[wid] = x;
+    __syncthreads();
+    if (wid == 0) {
+        unsigned long long w = lane < int(blockDim.x >> 5) ? warp_sums[lane] : 0ull;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(kFull, w, o);
+            if (lane >= o) w += y;
+        }
+        warp_sums[lane] = w; /* inclusive over warps */
+    }
+    __syncthreads();
+    const unsigned long long warp_base = wid ? warp_sums[wid - 1] : 0ull;
+    excl = warp_base + x - v;
+    const unsigned long long total = warp_sums[(blockDim.x >> 5) - 1];
+    __syncthreads();
+    return total;
+}
+
+/* The sum of all tiles before `tile`, by one warp (every lane returns it):
+ * 32 tiles' words at a time, nearest first, until one holds the sum up to
+ * its end.  kLookBad if a word is not written within kLookPolls polls. */
+__device__ __forceinline__ unsigned long long look_back(const unsigned long long *words,
+                                                        uint64_t tile, int lane)
+{
+    unsigned long long sum = 0;
+    uint64_t upto = tile; /* words [.., upto) are still to be added */
+    uint32_t polls = 0;
+    while (upto > 0) {
+        const bool in = uint64_t(lane) < upto;
+        const unsigned long long w = in ? look_load(words + (upto - 1 - uint64_t(lane))) : kLookEnd;
+        const unsigned long long kind = w & ~kLookMask;
+        if (__any_sync(kFull, kind == kLookBad)) return kLookBad;
+        const unsigned ends = __ballot_sync(kFull, kind == kLookEnd);
+        const unsigned none = __ballot_sync(kFull, kind == 0);
+        const int last = ends ? __ffs(ends) - 1 : 31; /* the nearest tile whose end is known */
+        const unsigned used = last == 31 ? kFull : ((1u << (last + 1)) - 1u);
+        if (none & used) {
+            if (++polls > kLookPolls) return kLookBad;
+            __nanosleep(64);
+            continue;
+        }
+        sum += warp_sum_u64(lane <= last ? (w & kLookMask) : 0ull);
+        if (ends) break;
+        upto -= 32;
+    }
+    return sum;
+}
+
+/* the window of W keys at kw: the slots that hold key, and whether one is
+ * free.  A window of a known width comes in 32-byte loads, with one compare
+ * per slot; the mask is built only where the key is. */
+template <class K, int kW>
+__device__ __forceinline__ void key_window(const K *kw, uint32_t W, K key, K empty, uint32_t &hits,
+                                           bool &free)
+{
+    constexpr int WB = kW * int(sizeof(K));
+    hits = 0;
+    free = false;
+    if constexpr (kW > 0 && WB <= 128) {
+        using L = typename std::conditional<sizeof(K) == 4, LayoutSet32, LayoutSet64>::type;
+        uint32_t w[WB / 4];
+        load_window<WB>(reinterpret_cast<const unsigned char *>(kw), w);
+        bool any = false;
+#pragma unroll
+        for (int i = 0; i < kW; ++i) {
+            any |= K(window_key<L>(w, i)) == key;
+            free |= K(window_key<L>(w, i)) == empty;
+        }
+        if (any) {
+#pragma unroll
+            for (int i = 0; i < kW; ++i) hits |= uint32_t(K(window_key<L>(w, i)) == key) << i;
+        }
+    } else {
+        uint32_t e;
+        mb_window<K, kW>(kw, W, key, empty, hits, e);
+        free = e != 0;
+    }
+}
+
+/* A lane's next key: the lanes of a warp without a key take the next ones
+ * of the block's tile, `m` in all, in order.  `left` (uniform) turns false
+ * with the last of them.  Returns whether this lane got key number `at`. */
+__device__ __forceinline__ bool draw_key(bool has, int m, int *drawn, bool &left, int &at)
+{
+    const unsigned need = __ballot_sync(kFull, !has);
+    if (!need || !left) return false;
+    const int lane = threadIdx.x & 31;
+    int from = 0;
+    if (lane == 0) from = atomicAdd(drawn, __popc(need));
+    from = __shfl_sync(kFull, from, 0);
+    left = from + __popc(need) < m;
+    if (has) return false;
+    at = from + __popc(need & ((1u << lane) - 1u));
+    return at < m;
+}
+
+/* num_values (kOffsets false): per-key counts and their sum; the first half
+ * of retrieve (kOffsets): begin / end offsets and the sum */
+template <class Walk, bool kOffsets>
+__global__ void __launch_bounds__(kMultiThreads, WC_MULTI_COUNT_BLOCKS)
+    multi_find_kernel(const typename Walk::Args a)
+{
+    using K = typename Walk::key_t;
+    __shared__ K s_key[kMultiTile];
+    __shared__ unsigned long long s_end[kMultiTile]; /* counts, then end offsets in the tile */
+    __shared__ int s_drawn;
+    __shared__ unsigned long long s_before;
+    __shared__ uint64_t s_tile;
+
+    const int lane = threadIdx.x & 31;
+    const uint64_t ntiles = (a.n + a.tile - 1) / a.tile;
+    const K *const keys = reinterpret_cast<const K *>(a.keys);
+    const K empty = K(Walk::view(a).empty_key), tomb = K(Walk::view(a).tombstone_key);
+    uint32_t join = 0;
+
+    for (;;) {
+        if (threadIdx.x == 0) {
+            s_tile = atomicAdd(a.look + kLookTicket, 1ull);
+            s_drawn = 0;
+        }
+        __syncthreads();
+        const uint64_t tile = s_tile;
+        if (tile >= ntiles) break;
+        const uint64_t base = tile * a.tile;
+        const int m = int(a.n - base < a.tile ? a.n - base : a.tile);
+        for (int i = threadIdx.x; i < m; i += kMultiThreads) s_key[i] = ld_stream(keys + base + i);
+        __syncthreads();
+
+        /* ---- walk the keys ---- */
+        {
+            bool has = false, left = true;
+            int at = 0;
+            K key = 0;
+            typename Walk::State s;
+            for (;;) {
+                if (draw_key(has, m, &s_drawn, left, at)) {
+                    key = s_key[at];
+                    if (key == empty || key == tomb) {
+                        s_end[at] = 0;
+                        join |= kStInvalidKey;
+                        multi_write_status(a, base + uint64_t(at), kStInvalidKey);
+                    } else {
+                        has = true;
+                        Walk::start(a, key, s);
+                    }
+                }
+                if (!left && !__any_sync(kFull, has)) break;
+                uint32_t st = kStNone;
+                if (has && Walk::count_step(a, key, s, st)) {
+                    s_end[at] = s.num;
+                    join |= st;
+                    multi_write_status(a, base + uint64_t(at), st);
+                    has = false;
+                }
+            }
+        }
+        __syncthreads();
+
+        /* ---- offsets ---- */
+        constexpr int kPer = kMultiTile / kMultiThreads;
+        unsigned long long c[kPer], sum = 0, excl = 0;
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const int i = int(threadIdx.x) * kPer + j;
+            c[j] = i < m ? s_end[i] : 0ull;
+            sum += c[j];
+        }
+        const unsigned long long total = block_exclusive_scan(sum, excl);
+        if constexpr (!kOffsets) {
+            if (a.counts_out)
+                for (int i = threadIdx.x; i < m; i += kMultiThreads)
+                    a.counts_out[base + uint64_t(i)] = s_end[i];
+            if (threadIdx.x == 0 && total) atomicAdd(a.look + kLookTotal, total);
+        } else {
+            unsigned long long *const words = a.look + kLookTiles;
+            if (threadIdx.x == 0)
+                look_store(words + tile, tile == 0 ? (kLookEnd | total) : (kLookSum | total));
+            unsigned long long run = excl;
+#pragma unroll
+            for (int j = 0; j < kPer; ++j) {
+                run += c[j];
+                const int i = int(threadIdx.x) * kPer + j;
+                if (i < m) s_end[i] = run;
+            }
+            if (threadIdx.x < 32) {
+                const unsigned long long before = look_back(words, tile, lane);
+                if (lane == 0) {
+                    s_before = before;
+                    if (before == kLookBad) {
+                        look_store(words + tile, kLookBad);
+                        look_store(a.look + kLookFailed, 1ull);
+                    } else {
+                        if (tile) look_store(words + tile, kLookEnd | (before + total));
+                        if (tile + 1 == ntiles) look_store(a.look + kLookTotal, before + total);
+                    }
+                }
+            }
+            __syncthreads();
+            const unsigned long long before = s_before;
+            if (before == kLookBad) break; /* the host reports the timeout */
+            if (a.begin_first && tile == 0 && threadIdx.x == 0) *a.begin_first = 0;
+            for (int i = threadIdx.x; i < m; i += kMultiThreads) {
+                a.end_out[base + uint64_t(i)] = before + s_end[i];
+                if (a.begin_out)
+                    a.begin_out[base + uint64_t(i)] = before + (i ? s_end[i - 1] : 0ull);
+            }
+        }
+        __syncthreads(); /* the shared rows are rewritten by the next tile */
+    }
+    const uint32_t wj = __reduce_or_sync(kFull, join);
+    if (lane == 0) join_status(Walk::view(a).status, wj);
+}
+
+/* the second half of retrieve: every key's values, inside its own segment
+ * [begin, end) only.  A tile's keys without values are dropped first. */
+template <class Walk>
+__global__ void __launch_bounds__(kMultiThreads, WC_MULTI_VALUES_BLOCKS)
+    multi_values_kernel(const typename Walk::Args a)
+{
+    using K = typename Walk::key_t;
+    using V = typename Walk::val_t;
+    __shared__ K s_key[kMultiTile];
+    __shared__ unsigned long long s_begin[kMultiTile], s_room[kMultiTile];
+    __shared__ int s_drawn, s_found;
+    if (look_load(a.look + kLookFailed)) return;
+
+    const int lane = threadIdx.x & 31;
+    const K *const keys = reinterpret_cast<const K *>(a.keys);
+    for (uint64_t base = uint64_t(blockIdx.x) * a.tile; base < a.n;
+         base += uint64_t(gridDim.x) * a.tile) {
+        if (threadIdx.x == 0) {
+            s_drawn = 0;
+            s_found = 0;
+        }
+        __syncthreads();
+        const int m = int(a.n - base < a.tile ? a.n - base : a.tile);
+        for (int i0 = 0; i0 < m; i0 += kMultiThreads) {
+            const int i = i0 + int(threadIdx.x);
+            unsigned long long begin = 0, room = 0;
+            if (i < m) {
+                const unsigned long long end = a.end_out[base + uint64_t(i)];
+                begin = a.begin_out ? a.begin_out[base + uint64_t(i)]
+                                    : a.begin_first[base + uint64_t(i)];
+                room = end - begin;
+            }
+            const unsigned found = __ballot_sync(kFull, room != 0);
+            int p = 0;
+            if (lane == 0 && found) p = atomicAdd(&s_found, __popc(found));
+            p = __shfl_sync(kFull, p, 0) + __popc(found & ((1u << lane) - 1u));
+            if (room) {
+                s_key[p] = ld_stream(keys + base + uint64_t(i));
+                s_begin[p] = begin;
+                s_room[p] = room;
+            }
+        }
+        __syncthreads();
+        const int n = s_found;
+        bool has = false, left = n > 0;
+        int at = 0;
+        K key = 0;
+        V *out = nullptr;
+        uint64_t room = 0;
+        typename Walk::State s;
+        while (left || __any_sync(kFull, has)) {
+            if (draw_key(has, n, &s_drawn, left, at)) {
+                key = s_key[at];
+                out = reinterpret_cast<V *>(a.values_out) + s_begin[at];
+                room = s_room[at];
+                has = true;
+                Walk::start(a, key, s);
+            }
+            if (has && Walk::value_step(a, key, s, out, room)) has = false;
+        }
+        __syncthreads(); /* the shared rows are rewritten by the next tile */
+    }
+}
+
+/* dry run of retrieve: every key's status is dry_run */
+template <int kUnused = 0>
+__global__ void __launch_bounds__(256) multi_dry_status_kernel(void *status_out, uint64_t n,
+                                                               int handler, uint32_t bool_mask)
+{
+    const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
+    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
+        if (handler == kHandlerStatus)
+            reinterpret_cast<uint32_t *>(status_out)[i] = kStDryRun;
+        else if (handler == kHandlerBoolean)
+            reinterpret_cast<unsigned char *>(status_out)[i] =
+                (unsigned char)((kStDryRun & bool_mask) != 0);
+    }
+}
+
+} // namespace b200
+} // namespace warpcore
+
+#endif /* WC_MULTI_CUH */

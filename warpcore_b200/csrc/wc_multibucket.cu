@@ -29,7 +29,7 @@ struct wc_mbht {
     void *vals = nullptr;
     uint32_t *status = nullptr;           /* device Status word */
     unsigned long long *counters = nullptr; /* device: num_keys, num_occupied, scratch */
-    void *scan = nullptr;                 /* scan tile sums, grown on demand */
+    void *scan = nullptr;                 /* look-back words, grown on demand */
     uint64_t scan_bytes = 0;
     bool initialized = false;
 };
@@ -48,30 +48,9 @@ int mb_fail(int code, const char *msg) { return host_fail(code, msg); }
 
 uint64_t kmask(uint32_t bytes) { return bytes == 4 ? 0xffffffffull : ~0ull; }
 
-struct MbArgs {
+struct MbArgs : MultiArgs {
     MbView m;
-    const void *keys;
-    const void *values;              /* insert */
-    void *values_out;                /* retrieve */
-    const unsigned long long *begin; /* retrieve */
-    const unsigned long long *end;
-    unsigned long long *counts_out;  /* num_values: per key, or NULL */
-    unsigned long long *total;       /* num_values: sum */
-    void *status_out;
-    uint64_t n;
-    uint64_t max_windows;
-    uint32_t bool_mask;
-    int handler;
 };
-
-__device__ __forceinline__ void mb_write_status(const MbArgs &a, uint64_t i, uint32_t st)
-{
-    if (!a.status_out) return;
-    if (a.handler == kHandlerStatus)
-        reinterpret_cast<uint32_t *>(a.status_out)[i] = st;
-    else if (a.handler == kHandlerBoolean)
-        reinterpret_cast<unsigned char *>(a.status_out)[i] = (unsigned char)((st & a.bool_mask) != 0);
-}
 
 /* warp sums of two counters and the joined status, one atomic each per warp */
 __device__ __forceinline__ void mb_flush(const MbView &m, uint32_t join, unsigned claimed,
@@ -102,50 +81,102 @@ __global__ void __launch_bounds__(256, WC_MULTI_MIN_BLOCKS) mb_insert_kernel(con
         if (st != kStNone && st != kStDuplicateKey) join |= st;
         claimed += c;
         fresh += f;
-        mb_write_status(a, i, st);
+        multi_write_status(a, i, st);
     }
     mb_flush(a.m, join, claimed, fresh); /* every lane arrives (no early exit) */
 }
 
-/* num_values (kValues false) or retrieve of each key's values */
-template <class K, class V, int kW, int kB, bool kValues>
-__global__ void __launch_bounds__(256, WC_MULTI_MIN_BLOCKS) mb_find_kernel(const MbArgs a)
-{
-    uint32_t join = 0;
-    unsigned long long total = 0;
-    const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < a.n; i += stride) {
-        uint64_t num = 0;
-        const K key = reinterpret_cast<const K *>(a.keys)[i];
-        if constexpr (kValues) {
-            /* The counting pass walked every key to its end and wrote its
-             * status; this pass only reads values.  A key counted at 0
-             * needs no walk, and a walk ends once the counted values are
-             * read.  Values go inside the key's own segment only. */
-            const uint64_t room = a.end[i] - a.begin[i];
-            if (room == 0) continue;
-            V *const out = reinterpret_cast<V *>(a.values_out) + a.begin[i];
-            mb_for_each_one<K, V, kW, kB, true>(
-                a.m, key, a.max_windows, num, [&](V v, uint64_t j) {
-                    if (j < room) out[j] = v;
-                },
-                room);
+/* the key's slots window by window, as mb_for_each_one walks them: a window
+ * is one memory operation; then one bucket each: the last one of the window
+ * for the count (its free places are what the count needs), every one for
+ * the values */
+template <class K, class V, int kW, int kB>
+struct MbWalk {
+    using key_t = K;
+    using val_t = V;
+    using Args = MbArgs;
+    struct State {
+        uint64_t bucket, step, wins, num;
+        uint32_t hits; /* slots of the window whose buckets are still to be read */
+        bool free;     /* the window has a free slot */
+    };
+
+    static __device__ __forceinline__ const TableView &view(const Args &a) { return a.m.t; }
+
+    static __device__ __forceinline__ void start(const Args &a, K key, State &s)
+    {
+        s.bucket = probe_begin<K>(a.m.t, key);
+        s.step = 0;
+        s.wins = 0;
+        s.num = 0;
+        s.hits = 0;
+        s.free = false;
+    }
+
+    static __device__ __forceinline__ bool count_step(const Args &a, K key, State &s, uint32_t &st)
+    {
+        const uint32_t W = mb_w<kW>(a.m), B = mb_b<kB>(a.m);
+        if (!s.hits) {
+            window(a, key, s);
+            if (s.hits) return false;
         } else {
-            const uint32_t st = mb_for_each_one<K, V, kW, kB, false>(a.m, key, a.max_windows, num,
-                                                                     [](V, uint64_t) {});
-            join |= st;
-            if (a.counts_out) a.counts_out[i] = num;
-            total += num;
-            mb_write_status(a, i, st);
+            const int last = 31 - __clz(s.hits);
+            const uint32_t e = mb_bucket_empties<V, kB>(
+                reinterpret_cast<const V *>(a.m.vals) + (s.bucket * W + uint64_t(last)) * B, B,
+                V(a.m.empty_value), nullptr);
+            s.num += uint64_t(B) * uint64_t(__popc(s.hits)) - uint64_t(__popc(e));
+            s.hits = 0;
         }
+        return next(a, key, s, st, a.m.max_values);
     }
-    const uint32_t wj = __reduce_or_sync(0xffffffffu, join);
-    const unsigned long long sum = warp_sum_u64(total);
-    if ((threadIdx.x & 31) == 0) {
-        if (a.total && sum) atomicAdd(a.total, sum);
-        join_status(a.m.t.status, wj);
+
+    static __device__ __forceinline__ bool value_step(const Args &a, K key, State &s, V *out,
+                                                      uint64_t room)
+    {
+        const uint32_t W = mb_w<kW>(a.m), B = mb_b<kB>(a.m);
+        if (!s.hits) {
+            window(a, key, s);
+            if (s.hits) return false;
+        } else {
+            V v[kB ? kB : 32];
+            const uint64_t slot = s.bucket * W + uint64_t(__ffs(s.hits) - 1);
+            const uint32_t e =
+                mb_bucket_empties<V, kB>(reinterpret_cast<const V *>(a.m.vals) + slot * B, B,
+                                         V(a.m.empty_value), v);
+            for (uint32_t r = 0; r < (kB ? uint32_t(kB) : B); ++r)
+                if (!((e >> r) & 1u) && s.num + r < room) out[s.num + r] = v[r];
+            s.num += B;
+            s.hits &= s.hits - 1u;
+            if (s.hits) return false;
+            s.num -= uint64_t(__popc(e)); /* of the window's last bucket */
+        }
+        uint32_t st;
+        return next(a, key, s, st, room < a.m.max_values ? room : a.m.max_values);
     }
-}
+
+    static __device__ __forceinline__ void window(const Args &a, K key, State &s)
+    {
+        const uint32_t W = mb_w<kW>(a.m);
+        key_window<K, kW>(reinterpret_cast<const K *>(a.m.t.slots) + s.bucket * W, W, key,
+                          K(a.m.t.empty_key), s.hits, s.free);
+    }
+
+    static __device__ __forceinline__ bool next(const Args &a, K key, State &s, uint32_t &st,
+                                                uint64_t stop_at)
+    {
+        if (s.free || s.num >= stop_at) {
+            st = s.num ? kStNone : kStKeyNotFound;
+            return true;
+        }
+        if (++s.wins >= a.max_windows) {
+            st = kStProbingLengthExceeded;
+            return true;
+        }
+        if (s.wins == 1) s.step = probe_step<K>(a.m.t, key);
+        s.bucket = probe_next(a.m.t, s.bucket, s.step);
+        return false;
+    }
+};
 
 /* retrieve_all_keys (gpu_engine.cuh:51-93): slot `gid` emits its key when
  * it is the lowest slot of the first window holding the key; compacted by
@@ -196,15 +227,16 @@ __global__ void __launch_bounds__(256) mb_size_kernel(const MbView m, uint64_t c
 }
 
 struct MbKernels {
-    const void *insert, *count, *values, *unique, *size;
+    const void *insert, *count, *offsets, *values, *unique, *size;
 };
 
 template <class K, class V, int kW, int kB>
 MbKernels mb_kernels_of()
 {
     return {reinterpret_cast<const void *>(mb_insert_kernel<K, V, kW, kB>),
-            reinterpret_cast<const void *>(mb_find_kernel<K, V, kW, kB, false>),
-            reinterpret_cast<const void *>(mb_find_kernel<K, V, kW, kB, true>),
+            reinterpret_cast<const void *>(multi_find_kernel<MbWalk<K, V, kW, kB>, false>),
+            reinterpret_cast<const void *>(multi_find_kernel<MbWalk<K, V, kW, kB>, true>),
+            reinterpret_cast<const void *>(multi_values_kernel<MbWalk<K, V, kW, kB>>),
             reinterpret_cast<const void *>(mb_unique_keys_kernel<K>),
             reinterpret_cast<const void *>(mb_size_kernel<K, V>)};
 }
@@ -303,20 +335,8 @@ int read_counter(const unsigned long long *d, cudaStream_t s, uint64_t *out)
 int count(wc_mbht *t, const void *keys, uint64_t n, uint64_t *counts_dev, uint64_t *total,
           cudaStream_t s, uint64_t probing_length, void *status_out, int handler, uint32_t ignore)
 {
-    unsigned long long *tmp = t->counters + 2;
-    MB_CUDA(cudaMemsetAsync(tmp, 0, sizeof(unsigned long long), s));
     MbArgs a = args_of(t, keys, n, probing_length, true, status_out, handler, ignore);
-    a.counts_out = reinterpret_cast<unsigned long long *>(counts_dev);
-    a.total = tmp;
-    int rc = launch(mb_kernels(t).count, n, a, s);
-    if (rc) return rc;
-    return read_counter(tmp, s, total);
-}
-
-/* counts in end -> end = inclusive prefix sums, begin = exclusive ones */
-int scan(wc_mbht *t, uint64_t *begin, uint64_t *end, uint64_t n, cudaStream_t s)
-{
-    return host_offsets_scan(&t->scan, &t->scan_bytes, begin, end, n, s);
+    return host_multi_count(mb_kernels(t).count, &a, &a, t->counters + 8, counts_dev, total, s);
 }
 
 /* host join of status bits into the table's Status word */
@@ -476,26 +496,19 @@ int wc_mbht_retrieve(wc_mbht *t, const void *keys_in, uint64_t num_in,
     if (!keys_in || !end_offsets_out || (values_out && !begin_offsets_out))
         return mb_fail(WC_ERR_INVALID_ARGUMENT, "NULL buffer");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    /* pass 1: counts per key into end_offsets, and each key's status (the
-     * values pass reads values only) */
-    rc = count(t, keys_in, num_in, end_offsets_out, num_out, s, probing_length,
-               values_out ? status_out : nullptr, values_out ? status_handler : WC_HANDLER_NOTHING,
-               ignore);
-    if (rc) return rc;
     if (!values_out) {
         /* dry run: per-key counts, status dry_run for every key */
+        rc = count(t, keys_in, num_in, end_offsets_out, num_out, s, probing_length, nullptr,
+                   WC_HANDLER_NOTHING, ignore);
+        if (rc) return rc;
         rc = host_dry_run_status(status_out, num_in, status_handler, ignore, s);
         if (rc) return rc;
         return join_host(t, kStDryRun, s);
     }
-    /* pass 2: offsets; pass 3: values at each key's begin offset */
-    rc = scan(t, begin_offsets_out, end_offsets_out, num_in, s);
-    if (rc) return rc;
     MbArgs a = args_of(t, keys_in, num_in, probing_length, true, status_out, status_handler, ignore);
-    a.values_out = values_out;
-    a.begin = reinterpret_cast<const unsigned long long *>(begin_offsets_out);
-    a.end = reinterpret_cast<const unsigned long long *>(end_offsets_out);
-    return launch(mb_kernels(t).values, num_in, a, s);
+    const MbKernels k = mb_kernels(t);
+    return host_multi_retrieve(k.offsets, k.values, &a, &a, &t->scan, &t->scan_bytes,
+                               begin_offsets_out, end_offsets_out, values_out, num_out, s);
 }
 
 int wc_mbht_retrieve_all_keys(wc_mbht *t, void *keys_out, uint64_t *num_out, wc_stream_t stream)

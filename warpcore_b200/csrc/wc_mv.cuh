@@ -11,53 +11,23 @@
  * table kernels' bucket-aligned windows, so a key's values come out in the
  * order they were inserted, as in the reference.
  *
- * One lane owns one key and reads each bucket with 16-byte vector loads;
- * these tables are not on the headline path and keep the code close to the
- * reference's semantics, one bucket at a time.
+ * Lookups go through multi_find_kernel (wc_multi.cuh).
  */
 #ifndef WC_MV_CUH
 #define WC_MV_CUH
 
-#include "wc_kernels.cuh"
+#include "wc_lane_kernels.cuh"
+#include "wc_multi.cuh"
 #include <warpcore/detail/mv_ops.cuh>
 
 namespace warpcore {
 namespace b200 {
 
-/* resident 256-thread blocks per SM the multi-value kernels (multi-value,
- * multi-bucket, bucket-list) are built for: 4 measured best; 6 and 8
- * (42 and 32 registers) ran 0-10 % slower on the mv32 / mb32 / bl32
- * workloads, the register cap costing more than the extra warps bring */
-#ifndef WC_MULTI_MIN_BLOCKS
-#define WC_MULTI_MIN_BLOCKS 4
-#endif
-
-struct MvArgs {
+struct MvArgs : MultiArgs {
     TableView t;
-    const void *keys;
-    const void *values;               /* insert */
-    void *values_out;                 /* retrieve */
-    const unsigned long long *begin;  /* retrieve: begin offsets */
-    const unsigned long long *end;    /* retrieve: end offsets (overlap check) */
-    unsigned long long *counts_out;   /* num_values: per key, or NULL */
-    unsigned long long *total;        /* num_values: sum of the counts */
     unsigned long long *num_keys;     /* insert: keys that got their first value */
-    void *status_out;
-    uint64_t n;
-    uint64_t max_windows;
     uint64_t max_values;
-    uint32_t bool_mask;
-    int handler;
 };
-
-__device__ __forceinline__ void mv_write_status(const MvArgs &a, uint64_t i, uint32_t st)
-{
-    if (!a.status_out) return;
-    if (a.handler == kHandlerStatus)
-        reinterpret_cast<uint32_t *>(a.status_out)[i] = st;
-    else if (a.handler == kHandlerBoolean)
-        reinterpret_cast<unsigned char *>(a.status_out)[i] = (unsigned char)((st & a.bool_mask) != 0);
-}
 
 template <class L, int W>
 __global__ void __launch_bounds__(256, WC_MULTI_MIN_BLOCKS) mv_insert_kernel(const MvArgs a)
@@ -76,7 +46,7 @@ __global__ void __launch_bounds__(256, WC_MULTI_MIN_BLOCKS) mv_insert_kernel(con
          * a successful insert (:266-268) */
         if (st != kStNone && st != kStDuplicateKey) join |= st;
         new_keys += fresh;
-        mv_write_status(a, i, st);
+        multi_write_status(a, i, st);
     }
     /* every lane of the warp arrives here (no early exits) */
     const unsigned long long nk = __reduce_add_sync(kFull, unsigned(new_keys));
@@ -87,49 +57,89 @@ __global__ void __launch_bounds__(256, WC_MULTI_MIN_BLOCKS) mv_insert_kernel(con
     }
 }
 
-/* num_values (values_out == NULL) or retrieve of each key's values */
-template <class L, int W, bool kValues>
-__global__ void __launch_bounds__(256, WC_MULTI_MIN_BLOCKS) mv_find_kernel(const MvArgs a)
-{
-    using K = typename L::key_t;
-    using V = typename L::val_t;
-    uint32_t join = 0;
-    unsigned long long total = 0;
-    const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < a.n; i += stride) {
-        uint64_t num = 0;
-        if constexpr (kValues) {
-            /* The counting pass walked every key to its end and wrote its
-             * status; this pass only reads values.  A key counted at 0
-             * needs no walk, and a walk ends at the window where the
-             * counted values are read (its value limit).  Values are
-             * written inside the key's own segment only. */
-            const uint64_t room = a.end[i] - a.begin[i];
-            if (room == 0) continue;
-            V *const out = reinterpret_cast<V *>(a.values_out) + a.begin[i];
-            mv_for_each_one<L, W>(a.t, reinterpret_cast<const K *>(a.keys)[i], a.max_windows,
-                                  room < a.max_values ? room : a.max_values, num,
-                                  [&](V v, uint64_t j) {
-                                      if (j < room) out[j] = v;
-                                  });
+/* the key's slots window by window, as mv_for_each_one walks them */
+template <class L, int W>
+struct MvWalk {
+    using key_t = typename L::key_t;
+    using val_t = typename L::val_t;
+    using Args = MvArgs;
+    struct State {
+        uint64_t bucket, step, wins, num;
+    };
+
+    static __device__ __forceinline__ const TableView &view(const Args &a) { return a.t; }
+
+    static __device__ __forceinline__ void start(const Args &a, key_t key, State &s)
+    {
+        s.bucket = probe_begin<key_t>(a.t, key);
+        s.step = 0;
+        s.wins = 0;
+        s.num = 0;
+    }
+
+    /* one window; true where the walk ends */
+    static __device__ __forceinline__ bool count_step(const Args &a, key_t key, State &s,
+                                                      uint32_t &st)
+    {
+        return walk<false>(a, key, s, st, nullptr, 0, a.max_values);
+    }
+    static __device__ __forceinline__ bool value_step(const Args &a, key_t key, State &s,
+                                                      val_t *out, uint64_t room)
+    {
+        uint32_t st;
+        return walk<true>(a, key, s, st, out, room, room < a.max_values ? room : a.max_values);
+    }
+
+    template <bool kValues>
+    static __device__ __forceinline__ bool walk(const Args &a, key_t key, State &s, uint32_t &st,
+                                                val_t *out, uint64_t room, uint64_t stop_at)
+    {
+        const key_t empty = key_t(a.t.empty_key);
+        bool free = false;
+        constexpr int WB = W * L::kSlotBytes;
+        if constexpr (WB <= 128) {
+            uint32_t w[WB / 4];
+            load_window<WB>(reinterpret_cast<const unsigned char *>(a.t.slots) +
+                                s.bucket * uint64_t(WB), w);
+            bool any = false; /* one compare per slot; more only where the key is */
+#pragma unroll
+            for (int i = 0; i < W; ++i) {
+                any |= window_key<L>(w, i) == key;
+                free |= window_key<L>(w, i) == empty;
+            }
+            if (any) {
+#pragma unroll
+                for (int i = 0; i < W; ++i)
+                    if (window_key<L>(w, i) == key) {
+                        if constexpr (kValues) {
+                            if (s.num < room) out[s.num] = window_val<L>(w, i);
+                        }
+                        ++s.num;
+                    }
+            }
         } else {
-            const uint32_t st = mv_for_each_one<L, W>(a.t, reinterpret_cast<const K *>(a.keys)[i],
-                                                      a.max_windows, a.max_values, num,
-                                                      [](V, uint64_t) {});
-            join |= st;
-            if (a.counts_out) a.counts_out[i] = num;
-            total += num;
-            mv_write_status(a, i, st);
+            uint32_t hits, emp;
+            mv_bucket<L, W>(a.t, s.bucket, key, hits, emp, [&](int, const LaneWords &lw, int i) {
+                if constexpr (kValues) {
+                    if (s.num < room) out[s.num] = slot_val<L>(lw, i);
+                }
+                ++s.num;
+            });
+            free = emp != 0;
         }
+        if (free || s.num >= stop_at) {
+            st = s.num ? kStNone : kStKeyNotFound;
+            return true;
+        }
+        if (++s.wins >= a.max_windows) {
+            st = kStProbingLengthExceeded;
+            return true;
+        }
+        if (s.wins == 1) s.step = probe_step<key_t>(a.t, key);
+        s.bucket = probe_next(a.t, s.bucket, s.step);
+        return false;
     }
-    /* every lane of the warp arrives here (no early exits) */
-    const uint32_t wj = __reduce_or_sync(kFull, join);
-    const unsigned long long sum = warp_sum_u64(total);
-    if ((threadIdx.x & 31) == 0) {
-        if (a.total && sum) atomicAdd(a.total, sum);
-        join_status(a.t.status, wj);
-    }
-}
+};
 
 /* retrieve_all_keys: slot `gid` emits its key when it is the key's first
  * entry along its bucket sequence (lowest slot of the first bucket holding
@@ -158,126 +168,6 @@ __global__ void __launch_bounds__(256) mv_unique_keys_kernel(TableView t, uint64
                             }
                             return false;
                         });
-}
-
-/* ---- inclusive scan of per-key counts into end offsets, begin offsets
- * one behind (the reference uses cub::DeviceScan::InclusiveSum) ---- */
-constexpr int kScanThreads = 1024;
-constexpr int kScanItems = 4;
-constexpr uint64_t kScanTile = uint64_t(kScanThreads) * kScanItems;
-
-/* block-wide exclusive scan of one value per thread; returns the block total */
-__device__ __forceinline__ unsigned long long block_exclusive_scan(unsigned long long v,
-                                                                   unsigned long long &excl)
-{
-    __shared__ unsigned long long warp_sums[32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    unsigned long long x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long y = __shfl_up_sync(kFull, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_sums[wid] = x;
-    __syncthreads();
-    if (wid == 0) {
-        unsigned long long w = lane < int(blockDim.x >> 5) ? warp_sums[lane] : 0ull;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned long long y = __shfl_up_sync(kFull, w, o);
-            if (lane >= o) w += y;
-        }
-        warp_sums[lane] = w; /* inclusive over warps */
-    }
-    __syncthreads();
-    const unsigned long long warp_base = wid ? warp_sums[wid - 1] : 0ull;
-    excl = warp_base + x - v;
-    const unsigned long long total = warp_sums[(blockDim.x >> 5) - 1];
-    __syncthreads();
-    return total;
-}
-
-template <int kUnused = 0>
-__global__ void __launch_bounds__(kScanThreads) scan_tile_sums_kernel(
-    const unsigned long long *counts, uint64_t n, unsigned long long *tile_sums)
-{
-    const uint64_t t0 = uint64_t(blockIdx.x) * kScanTile;
-    unsigned long long s = 0;
-#pragma unroll
-    for (int j = 0; j < kScanItems; ++j) {
-        const uint64_t i = t0 + uint64_t(threadIdx.x) * kScanItems + j;
-        if (i < n) s += counts[i];
-    }
-    unsigned long long excl;
-    const unsigned long long total = block_exclusive_scan(s, excl);
-    if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
-}
-
-/* one block: exclusive scan of the tile sums, in place */
-template <int kUnused = 0>
-__global__ void __launch_bounds__(kScanThreads) scan_tile_offsets_kernel(unsigned long long *tile_sums,
-                                                                         uint64_t ntiles)
-{
-    const uint64_t per = (ntiles + kScanThreads - 1) / kScanThreads;
-    const uint64_t b = uint64_t(threadIdx.x) * per;
-    unsigned long long s = 0;
-    for (uint64_t k = 0; k < per && b + k < ntiles; ++k) s += tile_sums[b + k];
-    unsigned long long excl;
-    block_exclusive_scan(s, excl);
-    for (uint64_t k = 0; k < per && b + k < ntiles; ++k) {
-        const unsigned long long c = tile_sums[b + k];
-        tile_sums[b + k] = excl;
-        excl += c;
-    }
-}
-
-/* counts (in end) -> end = inclusive prefix sums, begin = end - count.
- * write_begin 0 leaves begin alone: the caller passed end == begin + 1 (the
- * reference's offsets_out, offsets_out + 1 idiom), where begin[i + 1] is
- * end[i] already and writing it would race with the block reading it. */
-template <int kUnused = 0>
-__global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(unsigned long long *end,
-                                                                  unsigned long long *begin,
-                                                                  uint64_t n,
-                                                                  const unsigned long long *tile_offsets,
-                                                                  int write_begin)
-{
-    const uint64_t t0 = uint64_t(blockIdx.x) * kScanTile;
-    unsigned long long c[kScanItems];
-    unsigned long long s = 0;
-#pragma unroll
-    for (int j = 0; j < kScanItems; ++j) {
-        const uint64_t i = t0 + uint64_t(threadIdx.x) * kScanItems + j;
-        c[j] = i < n ? end[i] : 0ull;
-        s += c[j];
-    }
-    unsigned long long excl;
-    block_exclusive_scan(s, excl);
-    unsigned long long run = tile_offsets[blockIdx.x] + excl;
-#pragma unroll
-    for (int j = 0; j < kScanItems; ++j) {
-        const uint64_t i = t0 + uint64_t(threadIdx.x) * kScanItems + j;
-        if (i < n) {
-            if (write_begin) begin[i] = run;
-            run += c[j];
-            end[i] = run;
-        }
-    }
-}
-
-/* dry run of retrieve: every key's status is dry_run */
-template <int kUnused = 0>
-__global__ void __launch_bounds__(256) mv_dry_status_kernel(void *status_out, uint64_t n,
-                                                            int handler, uint32_t bool_mask)
-{
-    const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
-        if (handler == kHandlerStatus)
-            reinterpret_cast<uint32_t *>(status_out)[i] = kStDryRun;
-        else if (handler == kHandlerBoolean)
-            reinterpret_cast<unsigned char *>(status_out)[i] =
-                (unsigned char)((kStDryRun & bool_mask) != 0);
-    }
 }
 
 } // namespace b200

@@ -16,8 +16,9 @@ MvKernels mv_pick()
 {
     MvKernels k;
     k.insert = reinterpret_cast<const void *>(mv_insert_kernel<L, W>);
-    k.count = reinterpret_cast<const void *>(mv_find_kernel<L, W, false>);
-    k.values = reinterpret_cast<const void *>(mv_find_kernel<L, W, true>);
+    k.count = reinterpret_cast<const void *>(multi_find_kernel<MvWalk<L, W>, false>);
+    k.offsets = reinterpret_cast<const void *>(multi_find_kernel<MvWalk<L, W>, true>);
+    k.values = reinterpret_cast<const void *>(multi_values_kernel<MvWalk<L, W>>);
     k.unique = reinterpret_cast<const void *>(mv_unique_keys_kernel<L, W>);
     return k;
 }

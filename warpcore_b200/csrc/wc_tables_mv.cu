@@ -12,14 +12,9 @@ MvKernels mv_kernels(int layout, int W)
     return MvKernels{};
 }
 
-MvScanKernels mv_scan_kernels()
+const void *multi_dry_status_kernel_ptr()
 {
-    MvScanKernels k;
-    k.tile_sums = reinterpret_cast<const void *>(scan_tile_sums_kernel<0>);
-    k.tile_offsets = reinterpret_cast<const void *>(scan_tile_offsets_kernel<0>);
-    k.apply = reinterpret_cast<const void *>(scan_apply_kernel<0>);
-    k.dry_status = reinterpret_cast<const void *>(mv_dry_status_kernel<0>);
-    return k;
+    return reinterpret_cast<const void *>(multi_dry_status_kernel<0>);
 }
 
 } // namespace b200
