@@ -96,3 +96,25 @@ def test_key_with_more_values_than_a_note_counts():
     assert np.array_equal(v[:extra], vals[:extra])
     assert np.array_equal(np.sort(v[extra:extra + n].view(np.uint32)), vals)
     assert np.array_equal(v[extra + n:], vals[:extra])
+
+
+@pytest.mark.parametrize("kb,vb", [(4, 4), (8, 8), (8, 4)])
+@pytest.mark.parametrize("cg", [1, 8, 16, 32])
+def test_insert_sizes_and_limits(kb, vb, cg):
+    # input counts around a warp, its two prefetch buffers and a full wave;
+    # every key three times with at most two values kept
+    keys = o.gen_unique_keys(kb, 148 * 4 * 256 + 1, 80)
+    for n in (1, 31, 32, 33, 63, 64, 65, 96, 97, len(keys)):
+        t = wc.MultiValueHashTable(4 * n, key_bytes=kb, value_bytes=vb, max_values_per_key=2,
+                                   cg_size=cg)
+        st = empty_dev(n, 4)
+        for round_, expect in enumerate((0, 1 << 4, (1 << 4) | (1 << 11))):
+            vals = (np.arange(n) + 1 + round_ * n).astype(DT[vb])
+            t.insert(dev(keys[:n]), dev(vals), status_out=st)
+            assert (host(st) == expect).all()
+        assert t.num_keys() == n and t.size() == 2 * n
+        num, b, e, v, _ = retrieve(t, keys[:n], 2 * n, vb)
+        assert num == 2 * n
+        got = v.view(DT[vb]).reshape(n, 2)
+        assert np.array_equal(got[:, 0], np.arange(n) + 1)
+        assert np.array_equal(got[:, 1], np.arange(n) + 1 + n)

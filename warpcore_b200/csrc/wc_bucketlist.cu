@@ -56,7 +56,7 @@ struct BlArgs : MultiArgs {
  * status of a key without a slot (invalid key, probing length exceeded)
  * unwritten, every key gets its status. */
 template <class K, class V, int kW>
-__global__ void __launch_bounds__(256, WC_MULTI_MIN_BLOCKS) bl_insert_kernel(const BlArgs a)
+__global__ void __launch_bounds__(256, WC_MULTI_INSERT_BLOCKS) bl_insert_kernel(const BlArgs a)
 {
     uint32_t join = 0;
     const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
@@ -168,10 +168,10 @@ struct BlWalk {
     {
         const TableView &t = a.v.t;
         const uint32_t W = kW ? uint32_t(kW) : t.cg_size;
-        uint32_t hits;
-        bool free;
-        key_window<K, kW>(reinterpret_cast<const K *>(t.slots) + s.bucket * W, W, key,
-                          K(t.empty_key), hits, free);
+        KeyWindow<K, kW> win;
+        win.load(reinterpret_cast<const K *>(t.slots) + s.bucket * W, W, key, K(t.empty_key));
+        const uint32_t hits = win.key_slots(key);
+        const bool free = win.any_free(K(t.empty_key));
         if (hits) {
             s.at = s.bucket * W + uint64_t(__ffs(hits) - 1);
             s.phase = 1;

@@ -67,7 +67,7 @@ __device__ __forceinline__ void mb_flush(const MbView &m, uint32_t join, unsigne
 }
 
 template <class K, class V, int kW, int kB>
-__global__ void __launch_bounds__(256, WC_MULTI_MIN_BLOCKS) mb_insert_kernel(const MbArgs a)
+__global__ void __launch_bounds__(256, WC_MULTI_INSERT_BLOCKS) mb_insert_kernel(const MbArgs a)
 {
     uint32_t join = 0;
     unsigned claimed = 0, fresh = 0;
@@ -113,17 +113,20 @@ struct MbWalk {
         s.free = false;
     }
 
+    /* the lanes' windows and buckets are loaded before any is looked at */
     static __device__ __forceinline__ bool count_step(const Args &a, K key, State &s, uint32_t &st)
     {
-        const uint32_t W = mb_w<kW>(a.m), B = mb_b<kB>(a.m);
-        if (!s.hits) {
-            window(a, key, s);
+        const uint32_t B = mb_b<kB>(a.m);
+        KeyWindow<K, kW> win;
+        uint32_t e = 0;
+        const bool at_window = s.hits == 0;
+        if (at_window) load(a, key, s, win);
+        else e = places(a, s, 31 - __clz(s.hits), nullptr);
+        if (at_window) {
+            s.free = win.any_free(K(a.m.t.empty_key));
+            s.hits = win.key_slots(key);
             if (s.hits) return false;
         } else {
-            const int last = 31 - __clz(s.hits);
-            const uint32_t e = mb_bucket_empties<V, kB>(
-                reinterpret_cast<const V *>(a.m.vals) + (s.bucket * W + uint64_t(last)) * B, B,
-                V(a.m.empty_value), nullptr);
             s.num += uint64_t(B) * uint64_t(__popc(s.hits)) - uint64_t(__popc(e));
             s.hits = 0;
         }
@@ -133,16 +136,18 @@ struct MbWalk {
     static __device__ __forceinline__ bool value_step(const Args &a, K key, State &s, V *out,
                                                       uint64_t room)
     {
-        const uint32_t W = mb_w<kW>(a.m), B = mb_b<kB>(a.m);
-        if (!s.hits) {
-            window(a, key, s);
+        const uint32_t B = mb_b<kB>(a.m);
+        KeyWindow<K, kW> win;
+        V v[kB ? kB : 32];
+        uint32_t e = 0;
+        const bool at_window = s.hits == 0;
+        if (at_window) load(a, key, s, win);
+        else e = places(a, s, __ffs(s.hits) - 1, v);
+        if (at_window) {
+            s.free = win.any_free(K(a.m.t.empty_key));
+            s.hits = win.key_slots(key);
             if (s.hits) return false;
         } else {
-            V v[kB ? kB : 32];
-            const uint64_t slot = s.bucket * W + uint64_t(__ffs(s.hits) - 1);
-            const uint32_t e =
-                mb_bucket_empties<V, kB>(reinterpret_cast<const V *>(a.m.vals) + slot * B, B,
-                                         V(a.m.empty_value), v);
             for (uint32_t r = 0; r < (kB ? uint32_t(kB) : B); ++r)
                 if (!((e >> r) & 1u) && s.num + r < room) out[s.num + r] = v[r];
             s.num += B;
@@ -154,11 +159,20 @@ struct MbWalk {
         return next(a, key, s, st, room < a.m.max_values ? room : a.m.max_values);
     }
 
-    static __device__ __forceinline__ void window(const Args &a, K key, State &s)
+    static __device__ __forceinline__ void load(const Args &a, K key, const State &s,
+                                                KeyWindow<K, kW> &win)
     {
         const uint32_t W = mb_w<kW>(a.m);
-        key_window<K, kW>(reinterpret_cast<const K *>(a.m.t.slots) + s.bucket * W, W, key,
-                          K(a.m.t.empty_key), s.hits, s.free);
+        win.load(reinterpret_cast<const K *>(a.m.t.slots) + s.bucket * W, W, key,
+                 K(a.m.t.empty_key));
+    }
+    /* the places of the bucket of window slot i: free ones, and all values */
+    static __device__ __forceinline__ uint32_t places(const Args &a, const State &s, int i, V *v)
+    {
+        const uint32_t W = mb_w<kW>(a.m), B = mb_b<kB>(a.m);
+        return mb_bucket_empties<V, kB>(
+            reinterpret_cast<const V *>(a.m.vals) + (s.bucket * W + uint64_t(i)) * B, B,
+            V(a.m.empty_value), v);
     }
 
     static __device__ __forceinline__ bool next(const Args &a, K key, State &s, uint32_t &st,

@@ -29,34 +29,6 @@ struct MvArgs : MultiArgs {
     uint64_t max_values;
 };
 
-template <class L, int W>
-__global__ void __launch_bounds__(256, WC_MULTI_MIN_BLOCKS) mv_insert_kernel(const MvArgs a)
-{
-    using K = typename L::key_t;
-    using V = typename L::val_t;
-    uint32_t join = 0;
-    unsigned long long new_keys = 0;
-    const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < a.n; i += stride) {
-        bool fresh = false;
-        const uint32_t st = mv_insert_one<L, W>(a.t, reinterpret_cast<const K *>(a.keys)[i],
-                                                reinterpret_cast<const V *>(a.values)[i],
-                                                a.max_windows, a.max_values, fresh);
-        /* the reference joins every status but the plain duplicate_key of
-         * a successful insert (:266-268) */
-        if (st != kStNone && st != kStDuplicateKey) join |= st;
-        new_keys += fresh;
-        multi_write_status(a, i, st);
-    }
-    /* every lane of the warp arrives here (no early exits) */
-    const unsigned long long nk = __reduce_add_sync(kFull, unsigned(new_keys));
-    const uint32_t wj = __reduce_or_sync(kFull, join);
-    if ((threadIdx.x & 31) == 0) {
-        if (nk) atomicAdd(a.num_keys, nk);
-        join_status(a.t.status, wj);
-    }
-}
-
 /* the key's slots window by window, as mv_for_each_one walks them */
 template <class L, int W>
 struct MvWalk {
@@ -90,13 +62,138 @@ struct MvWalk {
         return walk<true>(a, key, s, st, out, room, room < a.max_values ? room : a.max_values);
     }
 
+    /* ---- insert, as mv_insert_one: the key's values counted window by
+     * window, then a claim of the lowest free slot of the first window that
+     * has one; a claim that loses tries the next free slot it saw ---- */
+    static constexpr int WB = W * L::kSlotBytes;
+    static constexpr int kInsertBlocks = WB <= 64 ? WC_MULTI_INSERT_BLOCKS : 3;
+    struct InsertState {
+        uint64_t bucket, step, wins, num;
+        uint32_t free; /* free slots still to be tried; 0: the window is due */
+        val_t expect;  /* payload the slot is expected to hold */
+    };
+    struct InsertIo {
+        uint32_t w[WB <= 128 ? WB / 4 : 1];
+        uint32_t hits, free;
+        key_t old;
+        val_t old_payload;
+    };
+    struct Counts {
+        unsigned fresh; /* keys that got their first value */
+    };
+
+    static __device__ __forceinline__ uint32_t insert_start(const Args &a, key_t key, val_t,
+                                                            InsertState &s)
+    {
+        if (key == key_t(a.t.empty_key) || key == key_t(a.t.tombstone_key)) return kStInvalidKey;
+        s.bucket = probe_begin<key_t>(a.t, key);
+        s.step = 0;
+        s.wins = 0;
+        s.num = 0;
+        s.free = 0;
+        s.expect = 0;
+        return kStNone;
+    }
+
+    static __device__ __forceinline__ unsigned char *slot_of(const Args &a, const InsertState &s)
+    {
+        return reinterpret_cast<unsigned char *>(a.t.slots) + s.bucket * uint64_t(WB) +
+               (__ffs(s.free) - 1) * L::kSlotBytes;
+    }
+
+    static __device__ __forceinline__ void issue(const Args &a, key_t key, val_t val,
+                                                 const InsertState &s, InsertIo &io)
+    {
+        if (s.free) {
+            io.old = cas_slot<L>(slot_of(a, s), key_t(a.t.empty_key), s.expect, key, val,
+                                 &io.old_payload);
+        } else if constexpr (WB <= 128) {
+            load_window<WB>(reinterpret_cast<const unsigned char *>(a.t.slots) +
+                                s.bucket * uint64_t(WB), io.w);
+        } else {
+            mv_bucket<L, W>(a.t, s.bucket, key, io.hits, io.free,
+                            [](int, const LaneWords &, int) {});
+        }
+    }
+
+    static __device__ __forceinline__ bool look(const Args &a, key_t key, val_t val,
+                                                InsertState &s, const InsertIo &io, uint32_t &st,
+                                                uint32_t &join, Counts &counts)
+    {
+        const key_t empty = key_t(a.t.empty_key);
+        bool advance = false;
+        if (s.free) {
+            if (io.old == empty && io.old_payload == s.expect) {
+                counts.fresh += s.num == 0;
+                st = s.num ? kStDuplicateKey : kStNone;
+                return true;
+            }
+            if (io.old == empty) {
+                s.expect = io.old_payload; /* free slot, stale payload: again */
+                return false;
+            }
+            if (io.old == key && ++s.num >= a.max_values) {
+                st = kStDuplicateKey | kStMaxValuesReached;
+                join |= st;
+                return true;
+            }
+            s.free &= s.free - 1u;
+            s.expect = 0;
+            advance = s.free == 0;
+        } else {
+            uint32_t hits = io.hits, free = io.free;
+            if constexpr (WB <= 128) {
+                bool any_hit = false, any_free = false;
+#pragma unroll
+                for (int i = 0; i < W; ++i) {
+                    any_hit |= window_key<L>(io.w, i) == key;
+                    any_free |= window_key<L>(io.w, i) == empty;
+                }
+                hits = free = 0;
+                if (any_hit) {
+#pragma unroll
+                    for (int i = 0; i < W; ++i) hits += window_key<L>(io.w, i) == key;
+                    s.num += hits;
+                }
+                if (any_free) {
+#pragma unroll
+                    for (int i = 0; i < W; ++i)
+                        free |= uint32_t(window_key<L>(io.w, i) == empty) << i;
+                }
+            } else {
+                s.num += uint64_t(__popc(hits));
+            }
+            if (s.num >= a.max_values) {
+                st = kStDuplicateKey | kStMaxValuesReached;
+                join |= st;
+                return true;
+            }
+            s.free = free;
+            advance = free == 0;
+        }
+        if (!advance) return false;
+        if (++s.wins >= a.max_windows) {
+            st = kStProbingLengthExceeded | (s.num ? kStDuplicateKey : kStNone);
+            join |= st;
+            return true;
+        }
+        if (s.wins == 1) s.step = probe_step<key_t>(a.t, key);
+        s.bucket = probe_next(a.t, s.bucket, s.step);
+        return false;
+    }
+
+    static __device__ __forceinline__ void add_counts(const Args &a, const Counts &c)
+    {
+        const unsigned f = __reduce_add_sync(kFull, c.fresh);
+        if ((threadIdx.x & 31) == 0 && f) atomicAdd(a.num_keys, (unsigned long long)f);
+    }
+
     template <bool kValues>
     static __device__ __forceinline__ bool walk(const Args &a, key_t key, State &s, uint32_t &st,
                                                 val_t *out, uint64_t room, uint64_t stop_at)
     {
         const key_t empty = key_t(a.t.empty_key);
         bool free = false;
-        constexpr int WB = W * L::kSlotBytes;
         if constexpr (WB <= 128) {
             uint32_t w[WB / 4];
             load_window<WB>(reinterpret_cast<const unsigned char *>(a.t.slots) +

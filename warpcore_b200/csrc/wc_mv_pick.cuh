@@ -15,7 +15,7 @@ template <class L, int W>
 MvKernels mv_pick()
 {
     MvKernels k;
-    k.insert = reinterpret_cast<const void *>(mv_insert_kernel<L, W>);
+    k.insert = reinterpret_cast<const void *>(multi_insert_kernel<MvWalk<L, W>>);
     k.count = reinterpret_cast<const void *>(multi_find_kernel<MvWalk<L, W>, false>);
     k.offsets = reinterpret_cast<const void *>(multi_find_kernel<MvWalk<L, W>, true>);
     k.values = reinterpret_cast<const void *>(multi_values_kernel<MvWalk<L, W>>);
