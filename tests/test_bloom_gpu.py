@@ -82,3 +82,19 @@ def test_bloom_config4_shape_fpr():
     got = host(flags)
     assert got[: 1 << 20].all()
     assert got[1 << 20:].mean() < 1e-3
+
+
+@pytest.mark.parametrize("sb,cg", [(4, 4), (8, 2), (4, 8), (8, 4), (4, 16), (8, 8), (4, 32), (8, 16)])
+@pytest.mark.parametrize("ragged", [0, 1])
+def test_bloom_block_sizes_and_repeats(sb, cg, ragged):
+    # blocks of 16 to 128 bytes, whose inserts OR whole blocks at once: few
+    # and many keys, keys that repeat, an insert into a filled filter, and a
+    # last block that wraps to the front
+    num_bits = 8 * sb * (cg * 700 + ragged * (cg // 2))
+    f = wc.BloomFilter(num_bits, 6, key_bytes=8, slot_bytes=sb, cg_size=cg)
+    r = o.Bloom(num_bits, 6, key_bytes=8, slot_bytes=sb, cg=cg)
+    keys = o.gen_unique_keys(8, 9000, 79)
+    for part in (keys[:1], keys[:255], np.repeat(keys[300:330], 100), keys[400:9000]):
+        f.insert(dev(part))
+        r.insert(part)
+        assert np.array_equal(words_of(f, sb), r.words())
