@@ -272,17 +272,17 @@ void l2_window_release(L2Window &w)
 }
 
 cudaError_t launch_in_window(const void *kfn, unsigned grid, unsigned block, void **args,
-                             cudaStream_t s, const L2Window &w)
+                             cudaStream_t s, const L2Window &w, size_t smem = 0)
 {
     if (!w.bytes || !g_l2_mode.load(std::memory_order_relaxed)) {
-        const cudaError_t e = cudaLaunchKernel(kfn, dim3(grid), dim3(block), args, 0, s);
+        const cudaError_t e = cudaLaunchKernel(kfn, dim3(grid), dim3(block), args, smem, s);
         if (e == cudaSuccess) note_launches(1);
         return e;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeAccessPolicyWindow;
@@ -841,6 +841,87 @@ TableKernel pick_table_kernel(const wc_table *t, int op)
     }
 }
 
+/* The counting insert of wc_count.cuh (nullptr: table_op_kernel or the
+ * fingerprint kernel): no per-key statuses, and fewer keys than a 32-bit
+ * count holds.  On a table that L2 holds it is always the faster one.  On a
+ * larger one its lanes read windows sector by sector, so the line lies at
+ * what a window costs in DRAM: one sector (u32 pairs at CG 4) at any size,
+ * two sectors up to 512 MiB of slots, more never; and the batch has to be
+ * large enough for the fingerprints to be recomputed after it.  Measured
+ * against the fingerprint kernel: u32 pairs at CG 4, 2^28 Zipf(1.1) keys
+ * over 2^24 (159 MB) 7.13 -> 2.59 ms, 2^27 Zipf(0.5) over 2^25 (316 MB)
+ * 8.31 -> 4.93, over 2^26 (629 MB) 6.43 -> 5.98, but 2^22 keys into that
+ * 0.37 -> 0.39; 16-byte slots at CG 4, 2^26 Zipf(0.5) over 2^24 (316 MB)
+ * 4.06 -> 2.80 ms, Zipf(0.8) over 27 M (508 MB) 3.90 -> 3.72, 2^27 over
+ * 2^25 (629 MB) 7.94 -> 8.20, over 2^26 (1.26 GB) 6.65 -> 9.70. */
+CountInsertKernel pick_count_insert_kernel(const wc_table *t, int op, uint64_t n, int handler)
+{
+    if (op != kOpCount || handler != WC_HANDLER_NOTHING || (n >> 32)) return nullptr;
+    const uint64_t slots = t->capacity * t->slot_bytes;
+    const uint64_t window = uint64_t(t->cfg.cg_size) * t->slot_bytes;
+    if (slots > uint64_t(device_props().l2_bytes) &&
+        (window > 64 || (window > 32 && slots > (512ull << 20)) || n * 8 <= t->capacity))
+        return nullptr;
+    const int W = int(t->cfg.cg_size);
+    switch (t->layout) {
+    case kLayoutKV32: return count_insert_kv32(W);
+    case kLayoutKV64: return count_insert_kv64(W);
+    case kLayoutK32V64: return count_insert_k32v64(W);
+    case kLayoutK64V32: return count_insert_k64v32(W);
+    default: return nullptr;
+    }
+}
+
+/* every fingerprint recomputed from the slots (fp_rebuild_kernel) */
+int rebuild_fingerprints(wc_table *t, cudaStream_t s)
+{
+    const RebuildKernel rk = fp_rebuild_kernel_ptr(t->layout);
+    const void *rfn = reinterpret_cast<const void *>(rk);
+    const unsigned rgrid = grid_for(rfn, kBlock, t->capacity * t->slot_bytes / 64 + 1, kBlock);
+    const void *sl = t->slots;
+    uint64_t cap = t->capacity, em = t->cfg.empty_key, tb = t->cfg.tombstone_key;
+    unsigned char *fp = t->fps;
+    void *rargs[] = {&sl, &cap, &em, &tb, &fp};
+    WC_CUDA(cudaLaunchKernel(rfn, dim3(rgrid), dim3(kBlock), rargs, 0, s));
+    note_launches(1);
+    return WC_OK;
+}
+
+int count_insert(wc_table *t, CountInsertKernel k, const void *keys, uint64_t n, cudaStream_t s,
+                 uint64_t probing_length)
+{
+    CountArgs a;
+    a.t = view_of(t);
+    /* a batch of more than an eighth of the slots writes no fingerprints and
+     * has them recomputed after, as table_op's large inserts do */
+    const bool rebuild = t->fps && n * 8 > t->capacity &&
+                         (g_fp_ops.load(std::memory_order_relaxed) & 0x20u) == 0;
+    if (rebuild) a.t.fps = nullptr;
+    a.keys = keys;
+    a.n = n;
+    a.max_windows = max_windows(probing_length, t->cfg.cg_size, t->num_buckets);
+    const uint64_t sms = uint64_t(device_props().sms);
+    const uint64_t need = (n + kCountThreads - 1) / kCountThreads;
+    const unsigned grid = unsigned(need < sms ? need : sms);
+    /* as many entries as a block has keys, up to the largest cache */
+    const bool k4 = t->cfg.key_bytes == 4;
+    const uint32_t top = k4 ? count_cache_max_bits<uint32_t>() : count_cache_max_bits<uint64_t>();
+    a.cache_bits = 10;
+    while (a.cache_bits < top && (uint64_t(1) << a.cache_bits) * grid < n) ++a.cache_bits;
+    const size_t smem = k4 ? count_smem_bytes<uint32_t>(a.cache_bits)
+                           : count_smem_bytes<uint64_t>(a.cache_bits);
+    const void *kfn = reinterpret_cast<const void *>(k);
+    WC_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    void *args[] = {&a};
+    WC_CUDA(launch_in_window(kfn, grid, kCountThreads, args, s, t->l2, smem));
+    if (rebuild) {
+        const int rc = rebuild_fingerprints(t, s);
+        if (rc) return rc;
+    }
+    t->keys_inserted += n;
+    return WC_OK;
+}
+
 int table_op(wc_table *t, int op, const void *keys, const void *values, void *out,
              uint64_t n, wc_stream_t stream, uint64_t probing_length, void *status_out,
              int handler, uint32_t ignore)
@@ -852,6 +933,8 @@ int table_op(wc_table *t, int op, const void *keys, const void *values, void *ou
     if (op == kOpInsert && t->kind == 0 && !values)
         return fail(WC_ERR_INVALID_ARGUMENT, "values_in is NULL");
     if (op == kOpRetrieve && !out) return fail(WC_ERR_INVALID_ARGUMENT, "output is NULL");
+    if (const CountInsertKernel ck = pick_count_insert_kernel(t, op, n, handler))
+        return count_insert(t, ck, keys, n, reinterpret_cast<cudaStream_t>(stream), probing_length);
     /* A large insert into a table whose fingerprints exceed half of L2 runs
      * the whole-window kernel without fingerprint writes and then rebuilds
      * all fingerprints in one streaming pass (see fp_rebuild_kernel). */
@@ -889,16 +972,8 @@ int table_op(wc_table *t, int op, const void *keys, const void *values, void *ou
     WC_CUDA(launch_in_window(kfn, grid, unsigned(block), args,
                              reinterpret_cast<cudaStream_t>(stream), t->l2));
     if (rebuild) {
-        const RebuildKernel rk = fp_rebuild_kernel_ptr(t->layout);
-        const void *rfn = reinterpret_cast<const void *>(rk);
-        const unsigned rgrid = grid_for(rfn, kBlock, t->capacity * t->slot_bytes / 64 + 1, kBlock);
-        const void *sl = t->slots;
-        uint64_t cap = t->capacity, em = t->cfg.empty_key, tb = t->cfg.tombstone_key;
-        unsigned char *fp = t->fps;
-        void *rargs[] = {&sl, &cap, &em, &tb, &fp};
-        WC_CUDA(cudaLaunchKernel(rfn, dim3(rgrid), dim3(kBlock), rargs, 0,
-                                 reinterpret_cast<cudaStream_t>(stream)));
-        note_launches(1);
+        const int rc = rebuild_fingerprints(t, reinterpret_cast<cudaStream_t>(stream));
+        if (rc) return rc;
     }
     if (op == kOpInsert || op == kOpCount) t->keys_inserted += n;
     return WC_OK;

@@ -9,6 +9,7 @@
 
 #include "wc_bloom.cuh"
 #include "wc_batch.cuh"
+#include "wc_count.cuh"
 #include "wc_fp_kernels.cuh"
 #include "wc_lane_kernels.cuh"
 #include "wc_mv.cuh"
@@ -45,6 +46,13 @@ TableKernel lane_kernel_set32(int W, int op);
 TableKernel lane_kernel_set64(int W, int op);
 TableKernel lane_kernel_k32v64(int W, int op);
 TableKernel lane_kernel_k64v32(int W, int op);
+
+/* the counting insert of wc_count.cuh of window width W, nullptr if not built */
+using CountInsertKernel = void (*)(CountArgs);
+CountInsertKernel count_insert_kv32(int W);
+CountInsertKernel count_insert_kv64(int W);
+CountInsertKernel count_insert_k32v64(int W);
+CountInsertKernel count_insert_k64v32(int W);
 
 /* struct-of-arrays single-value tables (wc_tables_soa.cu): the window
  * kernel of (key width, value width, W, op) for insert, retrieve and erase,

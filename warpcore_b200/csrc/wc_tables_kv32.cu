@@ -6,6 +6,7 @@ namespace b200 {
 
 TableKernel table_kernel_kv32(int W, int op, bool fp) { return pick_table_kernel_for<LayoutKV32>(W, op, fp); }
 TableKernel lane_kernel_kv32(int W, int op) { return pick_lane_kernel_for<LayoutKV32>(W, op); }
+CountInsertKernel count_insert_kv32(int W) { return pick_count_insert<LayoutKV32>(W); }
 
 } // namespace b200
 } // namespace warpcore

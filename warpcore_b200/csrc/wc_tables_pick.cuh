@@ -69,6 +69,28 @@ TableKernel pick_lane_kernel_for(int W, int op)
     }
 }
 
+/* the counting insert of wc_count.cuh, where a window is at most 128 bytes;
+ * else nullptr */
+template <class L, int W>
+CountInsertKernel pick_count_insert_of()
+{
+    if constexpr (W * L::kSlotBytes > 128) return nullptr;
+    else return count_insert_kernel<L, W>;
+}
+
+template <class L>
+CountInsertKernel pick_count_insert(int W)
+{
+    switch (W) {
+    case 1: return pick_count_insert_of<L, 1>();
+    case 2: return pick_count_insert_of<L, 2>();
+    case 4: return pick_count_insert_of<L, 4>();
+    case 8: return pick_count_insert_of<L, 8>();
+    case 16: return pick_count_insert_of<L, 16>();
+    default: return nullptr;
+    }
+}
+
 } // namespace b200
 } // namespace warpcore
 
