@@ -118,3 +118,47 @@ def test_insert_sizes_and_limits(kb, vb, cg):
         got = v.view(DT[vb]).reshape(n, 2)
         assert np.array_equal(got[:, 0], np.arange(n) + 1)
         assert np.array_equal(got[:, 1], np.arange(n) + 1 + n)
+
+
+@pytest.mark.parametrize("kb,vb,cg", [(4, 4, 8), (8, 8, 8), (4, 8, 4), (8, 4, 16)])
+def test_bucket_list_insert_sizes(kb, vb, cg):
+    # one key per resident lane and one more (the line between the two
+    # kernels), full and ragged tiles; equal keys in one batch; a limit
+    # of values per key; a pool that runs out; keys without a slot
+    wave = 148 * 4 * 256
+    keys = o.gen_unique_keys(kb, wave + 1, 81)
+    for n, per in ((wave, 1), (wave + 1, 1), (wave // 5 + 7, 7), (2 * kb + 3, wave // 8)):
+        t = wc.BucketListHashTable(2 * n, 4 * n * per, key_bytes=kb, value_bytes=vb, cg_size=cg)
+        at = np.random.default_rng(9).permutation(np.repeat(np.arange(n), per))
+        vals = (np.arange(n * per) + 1).astype(DT[vb])
+        st = empty_dev(n * per, 4)
+        t.insert(dev(keys[at]), dev(vals), status_out=st)
+        assert t.num_keys() == n and t.num_values() == n * per
+        assert np.count_nonzero(host(st) == 0) == n  # one claim per key
+        assert np.count_nonzero(host(st) == 1 << 4) == n * (per - 1)
+        num, b, e, v, _ = retrieve(t, keys[:n], n * per, vb)
+        assert num == n * per
+        owner = np.repeat(np.arange(n), e - b)
+        order = np.argsort(v.view(DT[vb]), kind="stable")
+        assert np.array_equal(v.view(DT[vb])[order], vals)
+        assert np.array_equal(owner[order], at)
+    n = wave + 1
+    t = wc.BucketListHashTable(2 * n, 4 * n, key_bytes=kb, value_bytes=vb, cg_size=cg,
+                               max_values_per_key=1)
+    st = empty_dev(n, 4)
+    for expect in (0, (1 << 4) | (1 << 11)):
+        t.insert(dev(keys), dev((np.arange(n) + 1).astype(DT[vb])), status_out=st)
+        assert (host(st) == expect).all()
+    small = wc.BucketListHashTable(2 * n, n // 2, key_bytes=kb, value_bytes=vb, cg_size=cg)
+    small.insert(dev(keys), dev((np.arange(n) + 1).astype(DT[vb])), status_out=st)
+    got = host(st)
+    assert set(np.unique(got)) == {0, 1 << 7}
+    assert np.count_nonzero(got == 0) == small.num_values() <= n // 2
+    few = wc.BucketListHashTable(1000, 4 * n, key_bytes=kb, value_bytes=vb, cg_size=cg)
+    many = o.gen_unique_keys(kb, few.key_capacity + n, 82)
+    st = empty_dev(len(many), 4)
+    few.insert(dev(many), dev((np.arange(len(many)) + 1).astype(DT[vb])), status_out=st,
+               probing_length=cg)
+    got = host(st)
+    assert set(np.unique(got)) <= {0, 1 << 1, 1 << 7}
+    assert np.count_nonzero(got & 2) == len(many) - few.num_keys()

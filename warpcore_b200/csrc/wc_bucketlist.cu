@@ -72,6 +72,196 @@ __global__ void __launch_bounds__(256, WC_MULTI_INSERT_BLOCKS) bl_insert_kernel(
     if ((threadIdx.x & 31) == 0) join_status(a.v.t.status, wj);
 }
 
+/* Bulk insert (:235-326), as bl_insert_one, in two steps per block tile.  In
+ * the first the lanes draw keys and find or claim their slots, one window
+ * read or compare-and-swap per lane and step; a lane whose key is done takes
+ * the next one, so no lane waits for the longest walk of its warp.  In the
+ * second each thread appends to four lists at once: the handles, the newest
+ * buckets' headers and the swaps of all four are in flight together, and
+ * the lanes of a warp that grow their lists share one pool reservation
+ * (which a loop of single steps per lane breaks up: 3330 us).  An append
+ * that loses its swap goes on in bl_append.  24 M values, 8 per key, in
+ * eight rounds: 1993 us with bl_insert_kernel, 1763 now; 16 M u64 values in
+ * one batch, 8 per key: 1506 and 1010.  What is left is random reads and
+ * compare-and-swaps outside L2.  (The same two steps for the multi-bucket
+ * insert measured 2041 -> 1991 us at 2^25 values and 380 -> 468 at 8 M in
+ * one batch: its swaps into 168 MB of buckets already run at 16 G/s of the
+ * 20 that random atomics reach there.) */
+template <class K, class V, int kW>
+__global__ void __launch_bounds__(kMultiThreads, WC_MULTI_INSERT_BLOCKS)
+    bl_insert_tiles_kernel(const BlArgs a)
+{
+    constexpr int kPer = kMultiTile / kMultiThreads;
+    constexpr uint64_t kDone = ~0ull;      /* no slot: the status is written */
+    constexpr uint64_t kFound = 1ull << 63; /* the key was there */
+    __shared__ K s_key[kMultiTile];
+    __shared__ uint64_t s_slot[kMultiTile];
+    __shared__ int s_drawn;
+    const BlView &v = a.v;
+    const TableView &t = v.t;
+    const uint32_t W = kW ? uint32_t(kW) : t.cg_size;
+    const K empty = K(t.empty_key), tomb = K(t.tombstone_key);
+    K *const slots = reinterpret_cast<K *>(t.slots);
+    const K *const keys_in = reinterpret_cast<const K *>(a.keys);
+    const V *const vals_in = reinterpret_cast<const V *>(a.values);
+    const uint64_t head = bl_head(v.ib);
+    uint32_t join = 0;
+
+    for (uint64_t base = uint64_t(blockIdx.x) * a.tile; base < a.n;
+         base += uint64_t(gridDim.x) * a.tile) {
+        const int m = int(a.n - base < a.tile ? a.n - base : a.tile);
+        if (threadIdx.x == 0) s_drawn = 0;
+        for (int i = threadIdx.x; i < m; i += kMultiThreads)
+            s_key[i] = ld_stream(keys_in + base + uint64_t(i));
+        __syncthreads();
+
+        /* ---- the keys' slots ---- */
+        {
+            bool has = false, left = true;
+            int at = 0;
+            K key = K(0);
+            uint64_t bucket = 0, step = 0, wins = 0;
+            uint32_t free = 0; /* free slots still to be tried; 0: the window is due */
+            for (;;) {
+                if (draw_key(has, m, &s_drawn, left, at)) {
+                    key = s_key[at];
+                    if (key == empty || key == tomb) {
+                        s_slot[at] = kDone;
+                        join |= kStInvalidKey;
+                        multi_write_status(a, base + uint64_t(at), kStInvalidKey);
+                    } else {
+                        has = true;
+                        bucket = probe_begin<K>(t, key);
+                        step = 0;
+                        wins = 0;
+                        free = 0;
+                    }
+                }
+                if (!left && !__any_sync(0xffffffffu, has)) break;
+                KeyWindow<K, kW> win;
+                K old = empty;
+                const int i = __ffs(free) - 1;
+                if (has) {
+                    if (free) old = mb_cas<K>(slots + bucket * W + uint64_t(i), empty, key);
+                    else win.load(slots + bucket * W, W, key, empty);
+                }
+                if (!has) continue;
+                uint64_t slot = kDone;
+                if (free) {
+                    if (old == empty) slot = bucket * W + uint64_t(i);
+                    else if (old == key) slot = (bucket * W + uint64_t(i)) | kFound;
+                    free &= free - 1u;
+                } else {
+                    const uint32_t hits = win.key_slots(key);
+                    if (hits) slot = (bucket * W + uint64_t(__ffs(hits) - 1)) | kFound;
+                    else free = win.free_slots(empty);
+                }
+                if (slot == kDone) {
+                    if (free) continue;
+                    if (++wins < a.max_windows) {
+                        if (wins == 1) step = probe_step<K>(t, key);
+                        bucket = probe_next(t, bucket, step);
+                        continue;
+                    }
+                    join |= kStProbingLengthExceeded;
+                    multi_write_status(a, base + uint64_t(at), kStProbingLengthExceeded);
+                }
+                s_slot[at] = slot;
+                has = false;
+            }
+        }
+        __syncthreads();
+
+        /* ---- append, four lists per thread ---- */
+        uint64_t slot[kPer];
+        unsigned long long cur[kPer], want[kPer], old[kPer];
+        uint64_t size[kPer];
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const int i = int(threadIdx.x) + j * kMultiThreads;
+            slot[j] = i < m ? s_slot[i] : kDone;
+            /* a new key's list is as init left it, unless an equal key's
+             * append was faster (the swap finds out) */
+            cur[j] = bl_pack(v, kBlUninit, head, 0, 0);
+            if (slot[j] != kDone && (slot[j] & kFound))
+                cur[j] = bl_load(v.handles + (slot[j] & ~kFound));
+        }
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const BlHandle c = bl_unpack(v, cur[j]);
+            size[j] = v.min_bucket;
+            if (slot[j] != kDone && c.state == kBlInit && c.count > v.min_bucket &&
+                c.count < v.max_values)
+                size[j] = bl_header_size(v, bl_load(v.pool + c.index));
+        }
+        /* try[j]: the swap that takes a place or blocks the handle */
+        bool tried[kPer];
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const BlHandle c = bl_unpack(v, cur[j]);
+            tried[j] = slot[j] != kDone && c.count < v.max_values &&
+                       (c.state == kBlInit || c.state == kBlUninit);
+            want[j] = c.state == kBlUninit ? bl_pack(v, kBlBlocking, head, 0, 0)
+                      : c.tail == size[j]
+                          ? bl_pack(v, kBlBlocking, c.index, c.count, c.tail)
+                          : bl_pack(v, kBlInit, c.index, c.count + 1, c.tail + 1);
+            old[j] = ~cur[j];
+            if (tried[j]) old[j] = atomicCAS(v.handles + (slot[j] & ~kFound), cur[j], want[j]);
+        }
+        uint32_t ast[kPer];
+        /* what the swaps won is finished for all four before any append that
+         * lost one waits for another's list */
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            ast[j] = kStNone;
+            if (!tried[j] || old[j] != cur[j]) continue;
+            const int i = int(threadIdx.x) + j * kMultiThreads;
+            const unsigned long long value = (unsigned long long)vals_in[base + uint64_t(i)];
+            const BlHandle c = bl_unpack(v, cur[j]);
+            if ((want[j] & 3u) == kBlInit) {
+                v.pool[c.index + (c.count + 1 <= v.min_bucket ? c.tail : c.tail + 1)] = value;
+                continue;
+            }
+            unsigned long long *const h = v.handles + (slot[j] & ~kFound);
+            const bool first = c.state == kBlUninit; /* the first bucket has no header */
+            uint64_t grow = v.min_bucket;
+            if (!first) {
+                const float grown = ceilf(float(size[j]) * v.grow);
+                const float cap = float(v.max_bucket);
+                grow = uint64_t(cap < grown ? cap : grown);
+            }
+            const uint64_t need = grow + (first ? 0 : 1);
+            const unsigned long long alloc = bl_alloc(v, need);
+            if (alloc + need <= v.capacity) {
+                if (!first) v.pool[alloc] = bl_header(v, c.index, grow);
+                v.pool[alloc + (first ? 0 : 1)] = value;
+                __threadfence();
+                atomicExch(h, bl_pack(v, kBlInit, alloc, c.count + 1, 1));
+            } else {
+                atomicExch(h, bl_pack(v, kBlFull, first ? head : c.index, c.count, c.tail));
+                ast[j] = kStOutOfMemory;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            if (slot[j] == kDone) continue;
+            const int i = int(threadIdx.x) + j * kMultiThreads;
+            if (!tried[j] || old[j] != cur[j]) {
+                if (bl_unpack(v, cur[j]).count >= v.max_values) ast[j] = kStMaxValuesReached;
+                else ast[j] = bl_append<V>(v, v.handles + (slot[j] & ~kFound),
+                                           vals_in[base + uint64_t(i)],
+                                           tried[j] ? old[j] : cur[j]);
+            }
+            const uint32_t st = ((slot[j] & kFound) ? kStDuplicateKey : kStNone) | ast[j];
+            join |= st;
+            multi_write_status(a, base + uint64_t(i), st);
+        }
+        __syncthreads(); /* the shared rows are rewritten by the next tile */
+    }
+    const uint32_t wj = __reduce_or_sync(0xffffffffu, join); /* every lane arrives */
+    if ((threadIdx.x & 31) == 0) join_status(a.v.t.status, wj);
+}
+
 /* the key's slot (as bl_find looks for it), then its handle, which holds the
  * list's count, then for the values the list's buckets, newest first (as
  * bl_walk reads them): a bucket's header and its first four values are read
@@ -230,13 +420,14 @@ __global__ void __launch_bounds__(256) bl_scan_keys_kernel(const BlView v, uint6
 }
 
 struct BlKernels {
-    const void *insert, *count, *offsets, *values, *init, *scan;
+    const void *insert, *insert_tiles, *count, *offsets, *values, *init, *scan;
 };
 
 template <class K, class V, int kW>
 BlKernels bl_kernels_of()
 {
     return {reinterpret_cast<const void *>(bl_insert_kernel<K, V, kW>),
+            reinterpret_cast<const void *>(bl_insert_tiles_kernel<K, V, kW>),
             reinterpret_cast<const void *>(multi_find_kernel<BlWalk<K, V, kW>, false>),
             reinterpret_cast<const void *>(multi_find_kernel<BlWalk<K, V, kW>, true>),
             reinterpret_cast<const void *>(multi_values_kernel<BlWalk<K, V, kW>>),
@@ -478,7 +669,16 @@ int wc_blht_insert(wc_blht *t, const void *keys_in, const void *values_in, uint6
     if (!keys_in || !values_in) return bl_fail(WC_ERR_INVALID_ARGUMENT, "keys_in / values_in is NULL");
     BlArgs a = args_of(t, keys_in, num_in, probing_length, status_out, status_handler, ignore);
     a.values = values_in;
-    return launch(bl_kernels(t).insert, num_in, a, reinterpret_cast<cudaStream_t>(stream));
+    const BlKernels k = bl_kernels(t);
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    /* Where every resident lane gets at most one key, no lane has a second
+     * one to draw, and the kernel without tiles is the faster one; else the
+     * tiles (u32 pairs, per round of 50 000 / 100 000 / 200 000 / 1 M new
+     * values: 11.7 / 12.5 / 21.9 / 80.2 us without, 12.1 / 12.4 / 19.1 /
+     * 63.8 with them). */
+    if (num_in <= uint64_t(host_grid(k.insert, kBlock, num_in, kBlock)) * kBlock)
+        return launch(k.insert, num_in, a, s);
+    return host_multi_launch(k.insert_tiles, &a, &a, s);
 }
 
 int wc_blht_num_values(wc_blht *t, const void *keys_in, uint64_t num_in, uint64_t *num_out,

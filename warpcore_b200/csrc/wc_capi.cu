@@ -417,6 +417,13 @@ int multi_total(const MultiArgs *a, uint64_t *total, cudaStream_t s)
 
 } // namespace
 
+int warpcore::b200::host_multi_launch(const void *tile_kernel, MultiArgs *a, void *args,
+                                      cudaStream_t s)
+{
+    a->tile = multi_tile(tile_kernel, a->n);
+    return multi_launch(tile_kernel, a, args, s);
+}
+
 int warpcore::b200::host_multi_count(const void *count_kernel, MultiArgs *a, void *args,
                                      unsigned long long *look, uint64_t *counts, uint64_t *total,
                                      cudaStream_t s)

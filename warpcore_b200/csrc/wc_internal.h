@@ -103,9 +103,10 @@ unsigned host_grid(const void *kernel, int block, uint64_t items, uint64_t per_b
 uint64_t host_valid_capacity(uint64_t min_capacity, uint64_t cg);
 /* the multi-value tables' shared host steps: num_values / retrieve of the
  * keys in a (the kernels of wc_multi.cuh, whose argument is *args, which
- * starts with a), a host-side Status join, a dry run's statuses, one device
+ * starts with a), the launch of an insert by tiles, a host-side Status join, a dry run's statuses, one device
  * counter read back.  host_multi_count uses the kLookTiles words at `look`,
  * host_multi_retrieve a scratch array grown on demand; both synchronise. */
+int host_multi_launch(const void *tile_kernel, MultiArgs *a, void *args, cudaStream_t s);
 int host_multi_count(const void *count_kernel, MultiArgs *a, void *args, unsigned long long *look,
                      uint64_t *counts, uint64_t *total, cudaStream_t s);
 int host_multi_retrieve(const void *offsets_kernel, const void *values_kernel, MultiArgs *a,
