@@ -43,6 +43,7 @@ namespace {
     } while (0)
 
 constexpr int kBlock = 256;
+constexpr unsigned kBlAuxBytes = 256; /* Status word at 0, counters from 64 on */
 
 int bl_fail(int code, const char *msg) { return host_fail(code, msg); }
 
@@ -381,7 +382,8 @@ struct BlWalk {
     }
 };
 
-/* init: keys empty, handles uninitialized, pool headers {head, min}, next free 0 */
+/* init: keys empty, handles uninitialized, pool headers {head, min}, Status and
+ * counters 0 */
 template <class K>
 __global__ void __launch_bounds__(256) bl_init_kernel(const BlView v, uint64_t capacity)
 {
@@ -394,7 +396,8 @@ __global__ void __launch_bounds__(256) bl_init_kernel(const BlView v, uint64_t c
         v.handles[i] = u;
     }
     for (uint64_t i = tid; i < v.capacity; i += stride) v.pool[i] = hdr;
-    if (tid == 0) *v.next_free = 0;
+    /* the table's small device block: the Status word and the counters */
+    if (blockIdx.x == 0 && threadIdx.x < kBlAuxBytes / 4) v.t.status[threadIdx.x] = 0;
 }
 
 /* num_keys (valid keys), num_values (sum of list counts) and the keys,
@@ -606,7 +609,7 @@ int wc_blht_create(const wc_table_config *cfg, uint64_t key_capacity, uint64_t v
     const uint64_t pbytes = (value_capacity ? value_capacity : 1) * 8;
     void *mem = nullptr;
     cudaError_t e = cudaMalloc(&mem, kbytes + hbytes + pbytes);
-    if (e == cudaSuccess) e = cudaMalloc(&t->status, 256);
+    if (e == cudaSuccess) e = cudaMalloc(&t->status, kBlAuxBytes);
     if (e != cudaSuccess) {
         cudaGetLastError();
         if (mem) cudaFree(mem);
@@ -644,7 +647,6 @@ int wc_blht_init(wc_blht *t, uint64_t seed, wc_stream_t stream)
     if (!t) return bl_fail(WC_ERR_INVALID_ARGUMENT, "table is NULL");
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     t->seed = seed & kmask(t->cfg.key_bytes);
-    BL_CUDA(cudaMemsetAsync(t->status, 0, 256, s));
     BlView v = view_of(t);
     uint64_t cap = t->capacity;
     const void *k = bl_kernels(t).init;

@@ -630,7 +630,9 @@ int fill_slots(wc_table *t, cudaStream_t stream)
     uint32_t *p = reinterpret_cast<uint32_t *>(t->slots);
     uint64_t n = n_u32;
     uint4 pat = pattern;
-    void *args[] = {&p, &n, &pat};
+    uint32_t *zero = t->status; /* the whole device block: Status, counters */
+    uint32_t n_zero = uint32_t(kAuxBytes / 4);
+    void *args[] = {&p, &n, &pat, &zero, &n_zero};
     WC_CUDA(launch_in_window(kfn, grid, kBlock, args, stream, t->l2));
     return WC_OK;
 }
@@ -1155,9 +1157,6 @@ int wc_table_init(wc_table *t, uint64_t seed, wc_stream_t stream)
     if (rc) return rc;
     if (t->fps) WC_CUDA(cudaMemsetAsync(t->fps, kFpEmpty, t->capacity, s));
     if (t->values) WC_CUDA(cudaMemsetAsync(t->values, 0, t->capacity * t->cfg.value_bytes, s));
-    WC_CUDA(cudaMemsetAsync(t->status, 0, sizeof(uint32_t), s));
-    WC_CUDA(cudaMemsetAsync(t->live, 0, kLiveBytes, s));
-    if (t->kind == 3) WC_CUDA(cudaMemsetAsync(t->num_keys, 0, sizeof(unsigned long long), s));
     WC_CUDA(cudaStreamSynchronize(s));
     t->initialized = true;
     return WC_OK;
@@ -2035,7 +2034,9 @@ int host_op(wc_host_pipe *p, wc_table *t, bool insert, const void *h_keys, const
             uint32_t *fp = reinterpret_cast<uint32_t *>(dv);
             uint64_t fn = m * ob / 4;
             uint4 pat = make_uint4(w[0], w[1], w[2], w[3]);
-            void *fargs[] = {&fp, &fn, &pat};
+            uint32_t *zero = nullptr;
+            uint32_t n_zero = 0;
+            void *fargs[] = {&fp, &fn, &pat, &zero, &n_zero};
             const void *fk = reinterpret_cast<const void *>(fill_kernel<0>);
             WC_CUDA(cudaLaunchKernel(fk, dim3(grid_for(fk, kBlock, fn / 4, kBlock)), dim3(kBlock),
                                      fargs, 0, s));

@@ -359,8 +359,10 @@ int join_host(wc_mbht *t, uint32_t bits, cudaStream_t s)
     return host_join_status(t->status, bits, s);
 }
 
-/* fill `bytes` (a multiple of 4) with a repeated 4- or 8-byte word */
-int fill(void *p, uint64_t bytes, uint64_t word, uint32_t word_bytes, cudaStream_t s)
+/* fill `bytes` (a multiple of 4) with a repeated 4- or 8-byte word, and
+ * n_zero words at `zero` with zeros */
+int fill(void *p, uint64_t bytes, uint64_t word, uint32_t word_bytes, cudaStream_t s,
+         uint32_t *zero = nullptr, uint32_t n_zero = 0)
 {
     uint32_t w[4];
     if (word_bytes == 4) {
@@ -373,7 +375,7 @@ int fill(void *p, uint64_t bytes, uint64_t word, uint32_t word_bytes, cudaStream
     uint32_t *dst = reinterpret_cast<uint32_t *>(p);
     uint64_t n = bytes / 4;
     const void *kfn = reinterpret_cast<const void *>(fill_kernel<0>);
-    void *args[] = {&dst, &n, &pat};
+    void *args[] = {&dst, &n, &pat, &zero, &n_zero};
     MB_CUDA(cudaLaunchKernel(kfn, dim3(host_grid(kfn, kBlock, n / 4, kBlock)), dim3(kBlock), args, 0,
                              s));
     note_launches(1);
@@ -459,9 +461,8 @@ int wc_mbht_init(wc_mbht *t, wc_stream_t stream)
     int rc = fill(t->keys, t->capacity * t->cfg.key_bytes, t->cfg.empty_key, t->cfg.key_bytes, s);
     if (rc) return rc;
     rc = fill(t->vals, t->capacity * t->bucket * t->cfg.value_bytes, t->empty_value,
-              t->cfg.value_bytes, s);
+              t->cfg.value_bytes, s, t->status, 256 / 4);
     if (rc) return rc;
-    MB_CUDA(cudaMemsetAsync(t->status, 0, 256, s));
     MB_CUDA(cudaStreamSynchronize(s));
     t->initialized = true;
     return WC_OK;
