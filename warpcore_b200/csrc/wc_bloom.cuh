@@ -16,7 +16,7 @@
 #ifndef WC_BLOOM_CUH
 #define WC_BLOOM_CUH
 
-#include "wc_kernels.cuh"
+#include "wc_lane_kernels.cuh"
 
 #include <cstring>
 
@@ -141,56 +141,60 @@ struct BulkOr {
     }
 };
 
-/* word i of a block held in registers, by a select tree (no dynamic
- * register indexing) */
+/* a whole block into registers, by 32-byte loads where it has them: a load of
+ * 32 lanes at random addresses costs one pass per lane whatever its width */
 template <class S, int CG>
-__device__ __forceinline__ S pick_word(const S (&w)[CG], int i)
+__device__ __forceinline__ void load_block(const S *p, S (&w)[CG])
 {
-    if constexpr (CG == 1) {
-        return w[0];
-    } else if constexpr (CG == 2) {
-        return (i & 1) ? w[1] : w[0];
-    } else if constexpr (CG == 4) {
-        const S a = (i & 1) ? w[1] : w[0], b = (i & 1) ? w[3] : w[2];
-        return (i & 2) ? b : a;
-    } else if constexpr (CG == 8) {
-        const S a = (i & 1) ? w[1] : w[0], b = (i & 1) ? w[3] : w[2];
-        const S c = (i & 1) ? w[5] : w[4], d = (i & 1) ? w[7] : w[6];
-        const S e = (i & 2) ? b : a, f = (i & 2) ? d : c;
-        return (i & 4) ? f : e;
-    } else {
-        S v = 0;
+    constexpr int BB = CG * int(sizeof(S));
+    uint32_t x[BB / 4];
+    load_window<BB>(reinterpret_cast<const unsigned char *>(p), x);
 #pragma unroll
-        for (int s = 0; s < CG; ++s)
-            if (s == i) v = w[s];
-        return v;
+    for (int i = 0; i < CG; ++i) {
+        if constexpr (sizeof(S) == 4) w[i] = S(x[i]);
+        else w[i] = S(uint64_t(x[2 * i]) | (uint64_t(x[2 * i + 1]) << 32));
     }
 }
 
 /* Whether every one of the key's k bits is set in the block w, each bit
- * tested in the word it falls in (the query needs no masks).  Against
- * building the k masks (a compare and select per word and bit) and testing
- * them, 36.4 against 27.9 G queries/s on the 2^32-bit filter of 64-byte
- * blocks. */
+ * tested in the 32-bit word it falls in (the query needs no masks).  The
+ * block's words stand in this thread's column of shared memory, `col`, one
+ * of 256 columns, so that a word is picked by its address and no two lanes
+ * meet on a bank.  With the block in registers and each word picked by a
+ * tree of selects, queries were bound by instruction issue: 2^28 queries of
+ * the 2^32-bit filter of 64-byte blocks, k 8, 6.55 -> 5.52 ms (48.7 G/s; plain
+ * 64-byte reads at random measured 57), 12 M of a 16 MiB filter of 32-byte
+ * blocks, k 6, 129 -> 111 us.  (Those 6.55 ms were 7.40 with 16-byte loads of
+ * the blocks.) */
 template <class K, class S, int CG>
 __device__ __forceinline__ bool block_has_all(K key, K seed, uint32_t hasher, uint64_t k,
-                                              const S (&w)[CG])
+                                              const S (&w)[CG], uint32_t *col)
 {
-    constexpr uint64_t kSlotBits = sizeof(S) * 8;
-    constexpr uint64_t kBlockBits = kSlotBits * CG;
-    bool ok = true;
-    if (hasher == kHashMurmur) {
-        for (uint64_t j = 0; j < k; ++j) {
-            const uint64_t h = hash_key<K>(kHashMurmur, K(key + seed + K(j))) & (kBlockBits - 1);
-            ok &= ((pick_word<S, CG>(w, int(h / kSlotBits)) >> (h % kSlotBits)) & S(1)) != 0;
+    constexpr uint32_t kBlockBits = uint32_t(sizeof(S)) * 8 * CG;
+#pragma unroll
+    for (int i = 0; i < CG; ++i) {
+        if constexpr (sizeof(S) == 4) {
+            col[i * 256] = uint32_t(w[i]);
+        } else {
+            col[2 * i * 256] = uint32_t(w[i]);
+            col[(2 * i + 1) * 256] = uint32_t(uint64_t(w[i]) >> 32);
         }
-        return ok;
     }
-    for (uint64_t j = 0; j < k; ++j) {
-        const uint64_t h = hash_key<K>(hasher, K(key + seed + K(j))) & (kBlockBits - 1);
-        ok &= ((pick_word<S, CG>(w, int(h / kSlotBits)) >> (h % kSlotBits)) & S(1)) != 0;
+    uint32_t ok = 1;
+    const uint32_t n = uint32_t(k);
+    if (hasher == kHashMurmur) {
+        for (uint32_t j = 0; j < n; ++j) {
+            const uint32_t h = uint32_t(hash_key<K>(kHashMurmur, K(key + seed + K(j)))) &
+                               (kBlockBits - 1);
+            ok &= col[(h >> 5) * 256] >> (h & 31u);
+        }
+        return ok & 1u;
     }
-    return ok;
+    for (uint32_t j = 0; j < n; ++j) {
+        const uint32_t h = uint32_t(hash_key<K>(hasher, K(key + seed + K(j)))) & (kBlockBits - 1);
+        ok &= col[(h >> 5) * 256] >> (h & 31u);
+    }
+    return ok & 1u;
 }
 
 template <class K, class S, int CG, bool INSERT>
@@ -305,81 +309,96 @@ __global__ void __launch_bounds__(256) bloom_kernel(const BloomArgs a)
 }
 
 /* One key per lane, for blocks of at most 128 bytes: the lane computes its
- * key's masks, reads its own block with BB / 16 vector loads (all lanes'
- * loads independent, so a warp keeps 32 blocks in flight) and tests it.  An
- * insert of blocks of 16 bytes or more ORs the masks without a read
- * (BulkOr), of smaller ones only the words that miss bits.  Against the cooperative kernel above
- * it spends no shuffles on block indices and masks.  It serves the keys
- * whose block lies in [region_lo, region_hi) (one pass: the whole filter). */
+ * key's masks, reads its own block with 32-byte vector loads and tests it.
+ * An insert of blocks of 16 bytes or more ORs the masks without a read
+ * (BulkOr), of smaller ones only the words that miss bits.  Against the
+ * cooperative kernel above it spends no shuffles on block indices and masks.
+ * It serves the keys whose block lies in [region_lo, region_hi) (one pass:
+ * the whole filter).
+ *
+ * Two keys per lane at a time pay for inserts of up to 32 bytes, which wait
+ * for their keys (6 M into a 16 MiB filter of 32-byte blocks 174 -> 165 us);
+ * for queries, bound by instruction issue, more than one costs registers
+ * (12 M: 129 / 135 / 134 us with one / two / four). */
+template <class S, int CG, bool INSERT>
+constexpr int bloom_keys_per_lane()
+{
+    return INSERT && BulkOr<S, CG>::kUsed && CG * int(sizeof(S)) <= 32 ? 2 : 1;
+}
+
 template <class K, class S, int CG, bool INSERT>
 __global__ void __launch_bounds__(256) bloom_lane_kernel(const BloomArgs a)
 {
-    constexpr int SB = sizeof(S);
-    constexpr int BB = CG * SB;               /* block bytes, <= 128 */
-    constexpr int VB = BB < 16 ? BB : 16;     /* bytes per load */
-    constexpr int NV = BB / VB;               /* loads per block */
-    constexpr int WPV = VB / SB;              /* words per load */
-    static_assert(BB <= 128 && NV * VB == BB && WPV * SB == VB, "block split");
+    constexpr int U = bloom_keys_per_lane<S, CG, INSERT>();
+    static_assert(CG * sizeof(S) <= 128, "block of one lane");
+    using Bulk = BulkOr<S, CG>;
+    constexpr bool kBulk = INSERT && Bulk::kUsed;
+    constexpr bool kRead = (!INSERT || WC_BLOOM_INSERT_READS_BLOCK) && !kBulk;
+    constexpr uint64_t kNone = ~0ull;
 
     S *const words = reinterpret_cast<S *>(a.words);
     const K *const keys = reinterpret_cast<const K *>(a.keys);
     const K seed = K(a.seed);
-    using Bulk = BulkOr<S, CG>;
-    constexpr bool kBulk = INSERT && Bulk::kUsed;
     __shared__ alignas(16) unsigned char s_rows[kBulk ? 256 * Bulk::kRow : 16];
+    __shared__ uint32_t s_words[INSERT ? 1 : CG * sizeof(S) / 4 * 256];
     const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < a.n; i += stride) {
-        const K key = ld_stream(keys + i);
-        const uint64_t blk =
-            fast_mod(hash_key<K>(a.hasher, K(key + seed)), a.num_blocks, a.magic_blocks) -
-            a.block_base;
-        if (blk >= a.local_blocks) {
+    for (uint64_t i0 = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i0 < a.n;
+         i0 += stride * U) {
+        K key[U];
+        uint64_t w0[U]; /* first word of the key's block, kNone: not served */
+        S w[U][CG];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint64_t i = i0 + uint64_t(u) * stride;
+            key[u] = i < a.n ? ld_stream(keys + i) : K(0);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint64_t i = i0 + uint64_t(u) * stride;
+            const uint64_t blk = mod_hash<K>(hash_key<K>(a.hasher, K(key[u] + seed)),
+                                             a.num_blocks, a.magic_blocks) - a.block_base;
+            w0[u] = i < a.n && blk < a.local_blocks && blk >= a.region_lo && blk < a.region_hi
+                        ? blk * CG : kNone;
             if constexpr (!INSERT) {
-                if (a.region_lo == 0) a.flags_out[i] = 0;
+                if (i < a.n && blk >= a.local_blocks && a.region_lo == 0) a.flags_out[i] = 0;
             }
-            continue;
-        }
-        if (blk < a.region_lo || blk >= a.region_hi) continue;
-        const uint64_t w0 = blk * CG;
-        if constexpr (kBulk) {
-            if (w0 + CG <= a.num_slots) {
-                S m[CG];
-                block_masks<K, S, CG>(key, seed, a.hasher, a.k, m);
-                Bulk::reduce(words + w0, s_rows + threadIdx.x * Bulk::kRow, m);
-                continue;
-            }
-        }
-        S w[CG];
-        constexpr bool kRead = !INSERT || WC_BLOOM_INSERT_READS_BLOCK;
-        if (kRead) {
-            if (w0 + CG <= a.num_slots) {
 #pragma unroll
-                for (int v = 0; v < NV; ++v) {
-                    const LaneWords lw = load_lane<VB>(words + w0 + uint64_t(v) * WPV);
+            for (int s = 0; s < CG; ++s) w[u][s] = 0;
+            if (kRead && w0[u] != kNone) {
+                if (w0[u] + CG <= a.num_slots) {
+                    load_block<S, CG>(words + w0[u], w[u]);
+                } else {
+                    /* ragged last block: words wrap to the front */
 #pragma unroll
-                    for (int s = 0; s < WPV; ++s) w[v * WPV + s] = lane_word<S>(lw, s);
+                    for (int s = 0; s < CG; ++s)
+                        w[u][s] = __ldcg(words + (w0[u] + s) % a.num_slots);
                 }
-            } else {
-                /* ragged last block: words wrap to the front */
-#pragma unroll
-                for (int s = 0; s < CG; ++s) w[s] = __ldcg(words + (w0 + s) % a.num_slots);
             }
-        } else {
-#pragma unroll
-            for (int s = 0; s < CG; ++s) w[s] = 0;
         }
-        if constexpr (!INSERT) {
-            a.flags_out[i] = (unsigned char)block_has_all<K, S, CG>(key, seed, a.hasher, a.k, w);
-        } else {
-            S m[CG];
-            block_masks<K, S, CG>(key, seed, a.hasher, a.k, m);
 #pragma unroll
-            for (int s = 0; s < CG; ++s) {
-                const bool missing = (w[s] & m[s]) != m[s];
-                if (m[s] && (!kRead || missing)) {
-                    uint64_t wi = w0 + uint64_t(s);
-                    if (wi >= a.num_slots) wi -= a.num_slots;
-                    atomic_or_any(words + wi, m[s]);
+        for (int u = 0; u < U; ++u) {
+            if (w0[u] == kNone) continue;
+            if constexpr (!INSERT) {
+                a.flags_out[i0 + uint64_t(u) * stride] =
+                    (unsigned char)block_has_all<K, S, CG>(key[u], seed, a.hasher, a.k, w[u],
+                                                           s_words + threadIdx.x);
+            } else {
+                S m[CG];
+                block_masks<K, S, CG>(key[u], seed, a.hasher, a.k, m);
+                if constexpr (kBulk) {
+                    if (w0[u] + CG <= a.num_slots) {
+                        Bulk::reduce(words + w0[u], s_rows + threadIdx.x * Bulk::kRow, m);
+                        continue;
+                    }
+                }
+#pragma unroll
+                for (int s = 0; s < CG; ++s) {
+                    const bool missing = (w[u][s] & m[s]) != m[s];
+                    if (m[s] && (!kRead || missing)) {
+                        uint64_t wi = w0[u] + uint64_t(s);
+                        if (wi >= a.num_slots) wi -= a.num_slots;
+                        atomic_or_any(words + wi, m[s]);
+                    }
                 }
             }
         }
@@ -398,7 +417,7 @@ __global__ void __launch_bounds__(256) bloom_lane_kernel(const BloomArgs a)
  *
  * A pass must keep many block reads in flight although only a fraction of
  * the keys it streams belongs to its region.  So a warp takes a tile of
- * kRegionKpl x 32 keys (kRegionKpl coalesced loads per lane in flight),
+ * region_kpl x 32 keys (region_kpl coalesced loads per lane in flight),
  * computes their blocks, and compacts the keys of its region into a list
  * in shared memory (ballot + prefix count, input order kept).  The lanes
  * then take the list densely, kRegionU entries per lane at a time, issue
@@ -408,10 +427,14 @@ __global__ void __launch_bounds__(256) bloom_lane_kernel(const BloomArgs a)
  * twice the registers) keeps more warps issuing than four entries per lane
  * with two blocks: on the 2^32-bit filter of 64-byte blocks, 2^28 keys,
  * 20.3 / 27.2 G keys/s (insert / query) against 16.9 / 21.3; two entries
- * with three blocks 19.7 / 25.5.  Each key is served by exactly one
+ * with three blocks 19.7 / 25.5 (masks in registers then; with the query's
+ * columns in shared memory 5.52 ms, with three or five blocks 6.22 / 7.44).
+ * Each key is served by exactly one
  * pass; a query's flag is written there (a key of another shard's block
  * gets 0 in the first pass). */
-constexpr int kRegionKpl = 8;   /* keys per lane per warp tile */
+/* keys per lane per warp tile (the rows of 128-byte blocks leave shared
+ * memory for half as many) */
+constexpr int region_kpl(int block_bytes) { return block_bytes <= 64 ? 8 : 4; }
 constexpr int kRegionU = 1;     /* compacted keys per lane in flight */
 constexpr int kRegionWarps = 8; /* 256 threads */
 
@@ -420,11 +443,9 @@ __global__ void __launch_bounds__(256, CG * sizeof(S) <= 64 ? 4 : 2) bloom_regio
 {
     constexpr int SB = sizeof(S);
     constexpr int BB = CG * SB;
-    constexpr int VB = BB < 16 ? BB : 16;
-    constexpr int NV = BB / VB;
-    constexpr int WPV = VB / SB;
+    constexpr int kRegionKpl = region_kpl(BB);
     constexpr int WT = 32 * kRegionKpl; /* keys per warp tile */
-    static_assert(BB <= 128 && NV * VB == BB && WPV * SB == VB, "block split");
+    static_assert(BB <= 128, "block of one lane");
     static_assert(WT <= 256, "tile offsets are one byte");
     constexpr bool kRead = !INSERT || WC_BLOOM_INSERT_READS_BLOCK;
 
@@ -434,6 +455,7 @@ __global__ void __launch_bounds__(256, CG * sizeof(S) <= 64 ? 4 : 2) bloom_regio
     using Bulk = BulkOr<S, CG>;
     constexpr bool kBulk = INSERT && Bulk::kUsed && BB <= 64; /* 48 KiB in all */
     __shared__ alignas(16) unsigned char s_rows[kBulk ? 256 * Bulk::kRow : 16];
+    __shared__ uint32_t s_words[INSERT ? 1 : BB / 4 * 256];
 
     S *const words = reinterpret_cast<S *>(a.words);
     const K *const keys = reinterpret_cast<const K *>(a.keys);
@@ -456,7 +478,7 @@ __global__ void __launch_bounds__(256, CG * sizeof(S) <= 64 ? 4 : 2) bloom_regio
         for (int j = 0; j < kRegionKpl; ++j) {
             const uint64_t i = base + uint64_t(j) * 32 + lane;
             const uint64_t blk =
-                fast_mod(hash_key<K>(a.hasher, K(kk[j] + seed)), a.num_blocks, a.magic_blocks) -
+                mod_hash<K>(hash_key<K>(a.hasher, K(kk[j] + seed)), a.num_blocks, a.magic_blocks) -
                 a.block_base;
             if constexpr (!INSERT) {
                 if (i < a.n && a.region_lo == 0 && blk >= a.local_blocks) a.flags_out[i] = 0;
@@ -481,12 +503,7 @@ __global__ void __launch_bounds__(256, CG * sizeof(S) <= 64 ? 4 : 2) bloom_regio
                 if (kRead && !kBulk && e < cnt) {
                     const uint64_t w0 = (a.region_lo + s_rel[wib][e]) * CG;
                     if (w0 + CG <= a.num_slots) {
-#pragma unroll
-                        for (int v = 0; v < NV; ++v) {
-                            const LaneWords lw = load_lane<VB>(words + w0 + uint64_t(v) * WPV);
-#pragma unroll
-                            for (int s = 0; s < WPV; ++s) w[u][v * WPV + s] = lane_word<S>(lw, s);
-                        }
+                        load_block<S, CG>(words + w0, w[u]);
                     } else {
 #pragma unroll
                         for (int s = 0; s < CG; ++s) w[u][s] = __ldcg(words + (w0 + s) % a.num_slots);
@@ -504,7 +521,8 @@ __global__ void __launch_bounds__(256, CG * sizeof(S) <= 64 ? 4 : 2) bloom_regio
                 const uint64_t w0 = (a.region_lo + s_rel[wib][e]) * CG;
                 if constexpr (!INSERT) {
                     a.flags_out[base + s_off[wib][e]] =
-                        (unsigned char)block_has_all<K, S, CG>(key, seed, a.hasher, a.k, w[u]);
+                        (unsigned char)block_has_all<K, S, CG>(key, seed, a.hasher, a.k, w[u],
+                                                               s_words + threadIdx.x);
                 } else {
                     S m[CG];
                     block_masks<K, S, CG>(key, seed, a.hasher, a.k, m);
