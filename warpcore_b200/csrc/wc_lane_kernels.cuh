@@ -13,7 +13,12 @@
  * own compare-and-swap: no ballots, no shuffles, no shared memory.
  *
  * Each lane issues one memory operation per wave, a window read or a
- * claim's compare-and-swap, so a warp keeps 32 of them in flight.  Keys are
+ * claim's compare-and-swap, so a warp keeps 32 of them in flight.  A window
+ * is looked at with one compare and at most two selects per slot, in four
+ * chains for lookups, and places in the warp's range are 32 bits wide; with
+ * masks of all slots and 64-bit places, u32 pairs took 137 / 144 us (insert
+ * of 4 M / lookup of 8 M, load 0.76) against 131 / 121 now, a u32 set 213
+ * against 187 (lookup of 16 M), mixed 4- and 8-byte pairs 66 against 68.  Keys are
  * refilled in input order from a double-buffered prefetch of the warp's
  * contiguous key range, as in table_op_kernel.  Equal keys need no merging
  * before the atomics: every claim goes to the lowest free slot of the
@@ -135,91 +140,106 @@ __global__ void __launch_bounds__(256, lane_min_blocks<L, W>()) lane_op_kernel(c
     uint64_t per = (a.n + nwarps - 1) / nwarps;
     per = (per + 31) & ~uint64_t(31);
     const uint64_t wb = warp * per < a.n ? warp * per : a.n;
-    const uint64_t we = wb + per < a.n ? wb + per : a.n;
+    const uint32_t m = uint32_t(wb + per < a.n ? per : a.n - wb);
 
     const K empty = K(t.empty_key);
     const K tomb = K(t.tombstone_key);
     unsigned char *const slots = reinterpret_cast<unsigned char *>(t.slots);
-    const K *const keys = reinterpret_cast<const K *>(a.keys);
-    const V *const vals_in = reinterpret_cast<const V *>(a.values);
+    const K *const keys = reinterpret_cast<const K *>(a.keys) + wb;
+    const V *const vals_in = reinterpret_cast<const V *>(a.values) + (kValueIn ? wb : 0);
 
-    uint64_t pf_base = wb;
-    K pfA = (wb + lane < we) ? ld_stream(keys + wb + lane) : empty;
-    K pfB = (wb + 32 + lane < we) ? ld_stream(keys + wb + 32 + lane) : empty;
+    uint32_t pf_base = 0, cursor = 0;
+    K pfA = uint32_t(lane) < m ? ld_stream(keys + lane) : empty;
+    K pfB = 32 + uint32_t(lane) < m ? ld_stream(keys + 32 + lane) : empty;
     V pvA = 0, pvB = 0;
     if constexpr (kValueIn) {
-        if (wb + lane < we) pvA = ld_stream(vals_in + wb + lane);
-        if (wb + 32 + lane < we) pvB = ld_stream(vals_in + wb + 32 + lane);
+        if (uint32_t(lane) < m) pvA = ld_stream(vals_in + lane);
+        if (32 + uint32_t(lane) < m) pvB = ld_stream(vals_in + 32 + lane);
     }
-    uint64_t cursor = wb;
 
-    /* the key this lane owns: waiting for its window (claiming == false) or
-     * for the compare-and-swap on slot claim_slot, expected to hold the
-     * empty key with payload claim_expect */
-    bool has = false, pending = false, flag = false, claiming = false;
-    int claim_slot = 0;
+    /* the key this lane owns: waiting for its window (claim < 0) or for the
+     * compare-and-swap on slot `claim` of it, expected to hold the empty key
+     * with payload claim_expect */
+    bool has = false;
+    int claim = -1;
     V claim_expect = 0;
-    uint64_t i = 0, bucket = 0, step = 0, wins = 0;
+    uint32_t at = 0; /* the key's place in the warp's range */
+    uint64_t bucket = 0, step = 0, wins = 0;
     K key = empty;
     V val = 0;
-    uint32_t st = kStNone, join = 0;
+    uint32_t join = 0;
     int live_delta = 0;
+
+    /* a key is done: its flag (sets) and its status */
+    auto finish = [&](uint32_t st, bool flag) {
+        if constexpr (OP == kOpRetrieve) {
+            if (a.is_set && st == kStNone)
+                reinterpret_cast<unsigned char *>(a.out)[wb + at] = (unsigned char)flag;
+        }
+        if (a.status_out) {
+            if (a.handler == kHandlerStatus)
+                st_stream(reinterpret_cast<uint32_t *>(a.status_out) + wb + at, st);
+            else if (a.handler == kHandlerBoolean)
+                reinterpret_cast<unsigned char *>(a.status_out)[wb + at] =
+                    (unsigned char)((st & a.bool_mask) != 0);
+        }
+        has = false;
+    };
 
     for (;;) {
         /* ---- refill lanes whose key is done, in input order ---- */
         const unsigned need = __ballot_sync(kFull, !has);
-        const uint64_t avail = we - cursor;
-        const int take = int(uint64_t(__popc(need)) < avail ? uint64_t(__popc(need)) : avail);
+        const uint32_t idle = uint32_t(__popc(need)), avail = m - cursor;
+        const uint32_t take = idle < avail ? idle : avail;
         if (take == 0 && need == kFull) break;
-        const int r = __popc(need & lanemask_lt);
-        const bool refill = !has && r < take;
-        const int off = int(cursor - pf_base) + r; /* < 64 for refilling lanes */
-        const K ka = shfl_any(pfA, off & 31);
-        const K kb = shfl_any(pfB, off & 31);
-        V va = 0, vb = 0;
-        if constexpr (kValueIn) {
-            va = shfl_any(pvA, off & 31);
-            vb = shfl_any(pvB, off & 31);
-        }
-        if (refill) {
-            key = off < 32 ? ka : kb;
-            if constexpr (kValueIn) val = off < 32 ? va : vb;
-            i = cursor + r;
-            has = true;
-            pending = true;
-            flag = false;
-            claiming = false;
-            st = kStNone;
-            wins = 0;
-            step = 0;
-            if (key == empty || key == tomb) {
-                st = kStInvalidKey;
-                join |= kStInvalidKey;
-                pending = false;
-            } else {
-                bucket = probe_begin<K>(t, key);
+        if (take) {
+            const uint32_t r = uint32_t(__popc(need & lanemask_lt));
+            const uint32_t off = cursor - pf_base + r; /* < 64 for refilling lanes */
+            const K ka = shfl_any(pfA, int(off & 31u));
+            const K kb = shfl_any(pfB, int(off & 31u));
+            V va = 0, vb = 0;
+            if constexpr (kValueIn) {
+                va = shfl_any(pvA, int(off & 31u));
+                vb = shfl_any(pvB, int(off & 31u));
+            }
+            if (!has && r < take) {
+                key = off < 32 ? ka : kb;
+                if constexpr (kValueIn) val = off < 32 ? va : vb;
+                at = cursor + r;
+                has = true;
+                claim = -1;
+                wins = 0;
+                step = 0;
+                if (key == empty || key == tomb) {
+                    join |= kStInvalidKey;
+                    finish(kStInvalidKey, false);
+                } else {
+                    bucket = probe_begin<K>(t, key);
+                }
+            }
+            cursor += take;
+            if (cursor - pf_base >= 32) {
+                pf_base += 32;
+                pfA = pfB;
+                pvA = pvB;
+                const uint32_t nx = pf_base + 32 + uint32_t(lane);
+                if (nx < m) {
+                    pfB = ld_stream(keys + nx);
+                    if constexpr (kValueIn) pvB = ld_stream(vals_in + nx);
+                }
             }
         }
-        cursor += uint64_t(take);
-        if (cursor - pf_base >= 32) {
-            pf_base += 32;
-            pfA = pfB;
-            pvA = pvB;
-            const uint64_t nx = pf_base + 32 + lane;
-            pfB = nx < we ? ld_stream(keys + nx) : empty;
-            if constexpr (kValueIn) pvB = nx < we ? ld_stream(vals_in + nx) : V(0);
-        }
 
-        /* ---- one memory operation per pending lane: its window, or its
+        /* ---- one memory operation per lane with a key: its window, or its
          * claim; all lanes' operations are in flight together ---- */
-        unsigned char *const bptr = slots + bucket * uint64_t(W) * SB;
+        unsigned char *const bptr = slots + bucket * uint64_t(WB);
         uint32_t w[WB / 4];
         K cas_old = empty;
         V cas_old_payload = 0;
-        if (pending) {
+        if (has) {
             if constexpr (OP == kOpInsert) {
-                if (claiming)
-                    cas_old = cas_slot<L>(bptr + claim_slot * SB, empty, claim_expect, key, val,
+                if (claim >= 0)
+                    cas_old = cas_slot<L>(bptr + claim * SB, empty, claim_expect, key, val,
                                           &cas_old_payload);
                 else
                     load_window<WB>(bptr, w);
@@ -227,111 +247,105 @@ __global__ void __launch_bounds__(256, lane_min_blocks<L, W>()) lane_op_kernel(c
                 load_window<WB>(bptr, w);
             }
         }
+        if (!has) continue;
 
-        bool advance = false;
-        if (pending && !claiming) {
-            uint32_t hit = 0, emp = 0;
-#pragma unroll
-            for (int s = 0; s < W; ++s) {
-                const K sk = window_key<L>(w, s);
-                hit |= uint32_t(sk == key) << s;
-                emp |= uint32_t(sk == empty) << s;
-            }
-            if (hit) {
-                const int s = __ffs(hit) - 1;
-                unsigned char *const sp = bptr + s * SB;
-                if constexpr (OP == kOpRetrieve) {
-                    st = kStNone;
-                    flag = true;
-                    if constexpr (L::kHasValue) {
-                        if (!a.is_set) {
-                            V v = window_val_at<L, W>(w, s);
-                            if (uint64_t(v) > t.max_count) v = V(t.max_count);
-                            st_stream(reinterpret_cast<V *>(a.out) + i, v);
-                        }
-                    }
-                } else if constexpr (OP == kOpInsert) {
-                    st = kStDuplicateKey;
-                    join |= kStDuplicateKey;
-                    store_value<L>(sp, val);
-                } else {
-                    if (erase_slot<L>(sp, key, tomb)) {
-                        fp_store(t, bucket * W + uint64_t(s), kFpTomb);
-                        --live_delta;
-                    }
-                    st = kStNone;
-                }
-                pending = false;
-            } else if (emp) {
-                if constexpr (OP == kOpRetrieve) {
-                    if (a.is_set) {
-                        st = kStNone;
-                        flag = false;
-                    } else {
-                        st = kStKeyNotFound;
-                        join |= kStKeyNotFound;
-                    }
-                    pending = false;
-                } else if constexpr (OP == kOpErase) {
-                    st = a.is_set ? kStNone : kStKeyNotFound;
-                    pending = false;
-                } else {
-                    /* claim the lowest free slot in the next wave */
-                    claiming = true;
-                    claim_slot = __ffs(emp) - 1;
-                    claim_expect = window_val_at<L, W>(w, claim_slot);
-                }
-            } else {
-                advance = true;
-            }
-        } else if (pending) {
-            if constexpr (OP == kOpInsert) {
+        if constexpr (OP == kOpInsert) {
+            if (claim >= 0) {
                 if (cas_old == empty && cas_old_payload == claim_expect) {
-                    fp_store(t, bucket * W + uint64_t(claim_slot), fingerprint(key));
+                    fp_store(t, bucket * W + uint64_t(claim), fingerprint(key));
                     ++live_delta;
-                    st = kStNone;
-                    pending = false;
+                    finish(kStNone, false);
                 } else if (cas_old == key) {
-                    st = kStDuplicateKey;
                     join |= kStDuplicateKey;
-                    store_value<L>(bptr + claim_slot * SB, val);
-                    pending = false;
+                    store_value<L>(bptr + claim * SB, val);
+                    finish(kStDuplicateKey, false);
                 } else if (cas_old == empty) {
                     claim_expect = cas_old_payload; /* free slot, stale payload: again */
                 } else {
-                    claiming = false; /* taken by another key: read the window again */
+                    claim = -1; /* taken by another key: read the window again */
                 }
-            }
-        }
-        if (pending && advance) {
-            if (++wins >= a.max_windows) {
-                pending = false;
-                if (OP == kOpErase) {
-                    st = a.is_set ? kStNone : kStProbingLengthExceeded;
-                } else {
-                    st = kStProbingLengthExceeded;
-                    join |= kStProbingLengthExceeded;
-                }
-            } else {
-                if (wins == 1) step = probe_step<K>(t, key);
-                bucket = probe_next(t, bucket, step);
+                continue;
             }
         }
 
-        /* ---- keys that finished this wave write their results ---- */
-        if (has && !pending) {
-            if constexpr (OP == kOpRetrieve) {
-                if (a.is_set && st == kStNone)
-                    reinterpret_cast<unsigned char *>(a.out)[i] = (unsigned char)flag;
+        /* the slot that holds the key, a free slot: one compare and one or
+         * two selects per slot, no masks */
+        bool hit = false, any_free = false;
+        if constexpr (OP == kOpRetrieve) {
+            /* four chains of compares side by side */
+            bool h[4] = {false, false, false, false}, f[4] = {false, false, false, false};
+            V x[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int s = 0; s < W; ++s) {
+                const K sk = window_key<L>(w, s);
+                f[s & 3] |= sk == empty;
+                h[s & 3] |= sk == key;
+                if constexpr (L::kHasValue) x[s & 3] = sk == key ? window_val<L>(w, s) : x[s & 3];
             }
-            if (a.status_out) {
-                if (a.handler == kHandlerStatus)
-                    st_stream(reinterpret_cast<uint32_t *>(a.status_out) + i, st);
-                else if (a.handler == kHandlerBoolean)
-                    reinterpret_cast<unsigned char *>(a.status_out)[i] =
-                        (unsigned char)((st & a.bool_mask) != 0);
+            hit = h[0] | h[1] | h[2] | h[3];
+            any_free = f[0] | f[1] | f[2] | f[3];
+            V v = x[0] | x[1] | x[2] | x[3]; /* a key has one slot */
+            if (hit || any_free) {
+                if constexpr (L::kHasValue) {
+                    if (hit && !a.is_set) {
+                        if (uint64_t(v) > t.max_count) v = V(t.max_count);
+                        st_stream(reinterpret_cast<V *>(a.out) + wb + at, v);
+                    }
+                }
+                const uint32_t st = hit || a.is_set ? kStNone : kStKeyNotFound;
+                join |= st;
+                finish(st, hit);
+                continue;
             }
-            has = false;
+        } else {
+            int hs = 0;
+#pragma unroll
+            for (int s = W - 1; s >= 0; --s) {
+                const K sk = window_key<L>(w, s);
+                if (sk == key) {
+                    hit = true;
+                    hs = s;
+                }
+                if constexpr (OP == kOpInsert) {
+                    if (sk == empty) { /* the lowest free slot is left over */
+                        any_free = true;
+                        claim = s;
+                        claim_expect = window_val<L>(w, s);
+                    }
+                } else {
+                    any_free |= sk == empty;
+                }
+            }
+            if (hit) {
+                unsigned char *const sp = bptr + hs * SB;
+                if constexpr (OP == kOpInsert) {
+                    join |= kStDuplicateKey;
+                    store_value<L>(sp, val);
+                    finish(kStDuplicateKey, false);
+                } else {
+                    if (erase_slot<L>(sp, key, tomb)) {
+                        fp_store(t, bucket * W + uint64_t(hs), kFpTomb);
+                        --live_delta;
+                    }
+                    finish(kStNone, false);
+                }
+                continue;
+            }
+        }
+        if (any_free) {
+            if constexpr (OP == kOpErase) finish(a.is_set ? kStNone : kStKeyNotFound, false);
+            continue; /* insert: the claim follows in the next wave */
+        }
+        if (++wins >= a.max_windows) {
+            if constexpr (OP == kOpErase) {
+                finish(a.is_set ? kStNone : kStProbingLengthExceeded, false);
+            } else {
+                join |= kStProbingLengthExceeded;
+                finish(kStProbingLengthExceeded, false);
+            }
+        } else {
+            if (wins == 1) step = probe_step<K>(t, key);
+            bucket = probe_next(t, bucket, step);
         }
     }
     const uint32_t wjoin = __reduce_or_sync(kFull, join);
