@@ -18,6 +18,8 @@
  *     erase: its compare-and-swap on the slot follows, with the words read
  *     as the expected value).
  *
+ * Inserts run fp_op_kernel, retrieve and erase fp_find_kernel.
+ *
  * Each lane owns one key and issues one memory operation per wave: a
  * fingerprint load, a candidate slot load, or a compare-and-swap claim.
  * The 32 lanes' operations are independent, so a warp keeps 32 requests in
@@ -176,10 +178,9 @@ __device__ __forceinline__ LaneWords load_slot_once(const unsigned char *sp)
 }
 
 template <class L, int W, int OP>
-__global__ void __launch_bounds__(256, (OP == kOpRetrieve || OP == kOpErase) ? WC_FP_MIN_BLOCKS_READ
-                                                                            : WC_FP_MIN_BLOCKS)
-    fp_op_kernel(const TableOpArgs a)
+__global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_op_kernel(const TableOpArgs a)
 {
+    static_assert(OP == kOpInsert || OP == kOpCount, "operation");
     using K = typename L::key_t;
     using V = typename L::val_t;
     constexpr int SB = L::kSlotBytes;
@@ -216,7 +217,7 @@ __global__ void __launch_bounds__(256, (OP == kOpRetrieve || OP == kOpErase) ? W
     }
     uint64_t cursor = wb;
 
-    bool has = false, pending = false, flag = false;
+    bool has = false, pending = false;
     int phase = kPhaseFps;
     uint32_t cand = 0, emp = 0, fp = 0;
     V claim_expect = 0;
@@ -260,7 +261,6 @@ __global__ void __launch_bounds__(256, (OP == kOpRetrieve || OP == kOpErase) ? W
             i = cursor + r;
             has = true;
             pending = true;
-            flag = false;
             st = kStNone;
             cnt_add = 1;
             wins = 0;
@@ -347,41 +347,20 @@ __global__ void __launch_bounds__(256, (OP == kOpRetrieve || OP == kOpErase) ? W
             } else if (phase == kPhaseCheck) {
                 const int s = __ffs(cand) - 1;
                 unsigned char *const sp = slots + (base_slot + uint64_t(s)) * SB;
-                /* inserts read the slot where the claims' atomics land (L2):
-                 * an L1 copy may predate the claim of an equal key by
-                 * another lane, which would then be inserted twice.  Erase
-                 * reads it the same way, since its compare-and-swap follows
-                 * on the same line: with the evict-first read and a second
-                 * read before the compare-and-swap, erasing 2^27 keys of a
-                 * 2.4 GB table ran at 7.0 G keys/s, against 9.2 now */
-                const LaneWords sw = (OP != kOpRetrieve) ? load_lane<SB>(sp)
-                                                         : load_slot_once<L>(sp);
+                /* read where the claims' atomics land (L2): an L1 copy may
+                 * predate the claim of an equal key by another lane, which
+                 * would then be inserted twice */
+                const LaneWords sw = load_lane<SB>(sp);
                 const K sk = slot_key<L>(sw, 0);
                 if (sk == key) {
-                    if constexpr (OP == kOpRetrieve) {
-                        st = kStNone;
-                        flag = true;
-                        if constexpr (L::kHasValue) {
-                            if (!a.is_set) {
-                                V v = slot_val<L>(sw, 0);
-                                if (uint64_t(v) > t.max_count) v = V(t.max_count);
-                                st_stream(reinterpret_cast<V *>(a.out) + i, v);
-                            }
-                        }
-                    } else if constexpr (OP == kOpInsert) {
+                    if constexpr (OP == kOpInsert) {
                         st = kStDuplicateKey;
                         join |= kStDuplicateKey;
                         store_value<L>(sp, val);
-                    } else if constexpr (OP == kOpCount) {
+                    } else {
                         st = kStDuplicateKey;
                         join |= kStDuplicateKey;
                         count_add<L>(sp, cnt_add, t.max_count, st, join);
-                    } else {
-                        if (erase_slot_seen<L>(sp, key, tomb, sw)) {
-                            fp_store(t, base_slot + uint64_t(s), kFpTomb);
-                            --live_delta;
-                        }
-                        st = kStNone;
                     }
                     pending = false;
                 } else {
@@ -453,22 +432,8 @@ __global__ void __launch_bounds__(256, (OP == kOpRetrieve || OP == kOpErase) ? W
                 if (cand) {
                     phase = kPhaseCheck;
                 } else if (emp) {
-                    if constexpr (OP == kOpRetrieve) {
-                        if (a.is_set) {
-                            st = kStNone;
-                            flag = false;
-                        } else {
-                            st = kStKeyNotFound;
-                            join |= kStKeyNotFound;
-                        }
-                        pending = false;
-                    } else if constexpr (OP == kOpErase) {
-                        st = a.is_set ? kStNone : kStKeyNotFound;
-                        pending = false;
-                    } else {
-                        phase = preload ? kPhasePreload : kPhaseClaim;
-                        claim_expect = 0;
-                    }
+                    phase = preload ? kPhasePreload : kPhaseClaim;
+                    claim_expect = 0;
                 } else {
                     advance = true;
                 }
@@ -480,12 +445,8 @@ __global__ void __launch_bounds__(256, (OP == kOpRetrieve || OP == kOpErase) ? W
                 claim_expect = 0;
                 if (++wins >= a.max_windows) {
                     pending = false;
-                    if (OP == kOpErase) {
-                        st = a.is_set ? kStNone : kStProbingLengthExceeded;
-                    } else {
-                        st = kStProbingLengthExceeded;
-                        join |= kStProbingLengthExceeded;
-                    }
+                    st = kStProbingLengthExceeded;
+                    join |= kStProbingLengthExceeded;
                 } else {
                     if (wins == 1) step = probe_step<K>(t, key);
                     bucket = probe_next(t, bucket, step);
@@ -495,10 +456,6 @@ __global__ void __launch_bounds__(256, (OP == kOpRetrieve || OP == kOpErase) ? W
 
         /* ---- keys that finished this wave write their results ---- */
         if (has && !pending) {
-            if constexpr (OP == kOpRetrieve) {
-                if (a.is_set && st == kStNone)
-                    reinterpret_cast<unsigned char *>(a.out)[i] = (unsigned char)flag;
-            }
             if (a.status_out) {
                 if (a.handler == kHandlerStatus)
                     st_stream(reinterpret_cast<uint32_t *>(a.status_out) + i, st);
@@ -517,6 +474,225 @@ __global__ void __launch_bounds__(256, (OP == kOpRetrieve || OP == kOpErase) ? W
                 if (ck != empty)
                     count_one<L, W>(t, ck, uint32_t(sc_cnt[c]), a.max_windows, join, live_delta);
             }
+        }
+    }
+    const uint32_t wjoin = __reduce_or_sync(kFull, join);
+    const int wlive = int(__reduce_add_sync(kFull, unsigned(live_delta)));
+    if (lane == 0) {
+        join_status(t.status, wjoin);
+        live_add(t, wlive);
+    }
+}
+
+/* The W fingerprint bytes of a bucket as 32-bit words */
+template <int W>
+struct FpWords {
+    static constexpr int NW = W >= 4 ? W / 4 : 1;
+    uint32_t w[NW];
+
+    __device__ __forceinline__ void load(const unsigned char *p, uint64_t pol)
+    {
+        if constexpr (W == 1) {
+            w[0] = ld_hint_u8(p, pol);
+        } else if constexpr (W == 2) {
+            w[0] = ld_hint_u16(p, pol);
+        } else if constexpr (W == 4) {
+            w[0] = ld_hint_u32(p, pol);
+        } else if constexpr (W == 8) {
+            const uint2 v = ld_hint_v2(p, pol);
+            w[0] = v.x;
+            w[1] = v.y;
+        } else {
+#pragma unroll
+            for (int h = 0; h < W / 16; ++h) {
+                const uint4 v = ld_hint_v4(p + 16 * h, pol);
+                w[4 * h + 0] = v.x;
+                w[4 * h + 1] = v.y;
+                w[4 * h + 2] = v.z;
+                w[4 * h + 3] = v.w;
+            }
+        }
+    }
+    /* the top bit of each byte of x that is zero; a byte of 1 above a zero
+     * byte may be marked too (the borrow), so "any" is exact and a marked
+     * byte is a candidate */
+    static __device__ __forceinline__ uint32_t zero_bytes(uint32_t x)
+    {
+        constexpr uint32_t kBytes = W >= 4 ? 0x80808080u : W == 2 ? 0x8080u : 0x80u;
+        return (x - 0x01010101u) & ~x & kBytes;
+    }
+    __device__ __forceinline__ bool any_empty() const
+    {
+        uint32_t m = 0;
+#pragma unroll
+        for (int k = 0; k < NW; ++k) m |= zero_bytes(w[k]);
+        return m != 0;
+    }
+    /* candidates for the pattern of four equal bytes: bit 8 b + k stands for
+     * byte b of word k (slot_of) */
+    __device__ __forceinline__ uint32_t candidates(uint32_t pat) const
+    {
+        uint32_t c = 0;
+#pragma unroll
+        for (int k = 0; k < NW; ++k) c |= (zero_bytes(w[k] ^ pat) >> 7) << k;
+        return c;
+    }
+    static __device__ __forceinline__ int slot_of(int bit) { return (bit >> 3) + 4 * (bit & 7); }
+};
+
+/* Retrieve and erase on tables with fingerprints.  What fp_op_kernel was
+ * bound by here is instruction issue (28 warp instructions per query, 77 %
+ * issue-active): a wave ran the fingerprint and the slot step one after the
+ * other, each waiting for its own load, built masks byte by byte and carried
+ * 64-bit places.  Here the lanes' fingerprint and slot loads are in flight
+ * together before any is looked at, a zero-byte test finds the empty and
+ * the matching fingerprints of a word (a match is checked against the slot
+ * anyway), and places in the warp's range are 32 bits wide.  Against it, u64 set of
+ * 134 MB at load 0.9: 15 M lookups 584 -> 483 us, 3.75 M erases 171 -> 158; u64
+ * pairs of 2.4 GB, 2^27 lookups 5.54 -> 5.34 ms (25.1 G/s; plain 8-byte reads
+ * at random measured 38 there, and a hit needs two); u32 pairs of 269 MB 30 M
+ * 991 -> 863 us; u32 set at CG 32 50 M 1611 -> 1126. */
+template <class L, int W, int OP>
+__global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS_READ) fp_find_kernel(const TableOpArgs a)
+{
+    using K = typename L::key_t;
+    using V = typename L::val_t;
+    static_assert(OP == kOpRetrieve || OP == kOpErase, "operation");
+    constexpr int SB = L::kSlotBytes;
+    const uint64_t pol_keep = l2_policy_evict_last(); /* fingerprint lines */
+
+    const TableView &t = a.t;
+    const int lane = threadIdx.x & 31;
+    const unsigned lanemask_lt = (1u << lane) - 1u;
+    const uint64_t warp = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nwarps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
+
+    /* this warp's contiguous range of keys */
+    uint64_t per = (a.n + nwarps - 1) / nwarps;
+    per = (per + 31) & ~uint64_t(31);
+    const uint64_t wb = warp * per < a.n ? warp * per : a.n;
+    const uint32_t m = uint32_t(wb + per < a.n ? per : a.n - wb);
+    const K empty = K(t.empty_key);
+    const K tomb = K(t.tombstone_key);
+    unsigned char *const slots = reinterpret_cast<unsigned char *>(t.slots);
+    const K *const keys = reinterpret_cast<const K *>(a.keys) + wb;
+
+    uint32_t pf_base = 0, cursor = 0;
+    K pfA = uint32_t(lane) < m ? ld_stream(keys + lane) : empty;
+    K pfB = 32 + uint32_t(lane) < m ? ld_stream(keys + 32 + lane) : empty;
+
+    /* the key this lane owns; cand: slots of its bucket still to be read (0:
+     * the bucket's fingerprints are due), any_empty: the bucket has a free one */
+    bool has = false, any_empty = false;
+    uint32_t cand = 0, at = 0;
+    uint64_t bucket = 0, step = 0, wins = 0;
+    K key = empty;
+    uint32_t join = 0;
+    int live_delta = 0;
+
+    auto finish = [&](uint32_t st, bool flag) {
+        if constexpr (OP == kOpRetrieve) {
+            if (a.is_set && st == kStNone)
+                reinterpret_cast<unsigned char *>(a.out)[wb + at] = (unsigned char)flag;
+        }
+        if (a.status_out) {
+            if (a.handler == kHandlerStatus)
+                st_stream(reinterpret_cast<uint32_t *>(a.status_out) + wb + at, st);
+            else if (a.handler == kHandlerBoolean)
+                reinterpret_cast<unsigned char *>(a.status_out)[wb + at] =
+                    (unsigned char)((st & a.bool_mask) != 0);
+        }
+        has = false;
+    };
+
+    for (;;) {
+        /* ---- refill lanes whose key is done, in input order ---- */
+        const unsigned need = __ballot_sync(kFull, !has);
+        const uint32_t idle = uint32_t(__popc(need)), avail = m - cursor;
+        const uint32_t take = idle < avail ? idle : avail;
+        if (take == 0 && need == kFull) break;
+        if (take) {
+            const uint32_t r = uint32_t(__popc(need & lanemask_lt));
+            const uint32_t off = cursor - pf_base + r; /* < 64 for refilling lanes */
+            const K ka = shfl_any(pfA, int(off & 31u));
+            const K kb = shfl_any(pfB, int(off & 31u));
+            if (!has && r < take) {
+                key = off < 32 ? ka : kb;
+                at = cursor + r;
+                has = true;
+                cand = 0;
+                wins = 0;
+                step = 0;
+                if (key == empty || key == tomb) {
+                    join |= kStInvalidKey;
+                    finish(kStInvalidKey, false);
+                } else {
+                    bucket = probe_begin<K>(t, key);
+                }
+            }
+            cursor += take;
+            if (cursor - pf_base >= 32) {
+                pf_base += 32;
+                pfA = pfB;
+                const uint32_t nx = pf_base + 32 + uint32_t(lane);
+                if (nx < m) pfB = ld_stream(keys + nx);
+            }
+        }
+
+        /* ---- one load per lane with a key: the bucket's fingerprints or a
+         * candidate's slot ---- */
+        const uint64_t base_slot = bucket * uint64_t(W);
+        FpWords<W> f;
+        LaneWords sw;
+        unsigned char *const sp =
+            slots + (base_slot + uint64_t(FpWords<W>::slot_of(__ffs(cand) - 1))) * SB;
+        if (has) {
+            if (cand == 0) f.load(t.fps + base_slot, pol_keep);
+            /* (erase reads from L2, where its compare-and-swap follows) */
+            else if constexpr (OP == kOpRetrieve) sw = load_slot_once<L>(sp);
+            else sw = load_lane<SB>(sp);
+        }
+        if (!has) continue;
+
+        if (cand == 0) {
+            cand = f.candidates(fingerprint(key) * 0x01010101u);
+            any_empty = f.any_empty();
+            if (cand) continue; /* the slot follows in the next wave */
+        } else {
+            if (slot_key<L>(sw, 0) == key) {
+                if constexpr (OP == kOpRetrieve) {
+                    if constexpr (L::kHasValue) {
+                        if (!a.is_set) {
+                            V v = slot_val<L>(sw, 0);
+                            if (uint64_t(v) > t.max_count) v = V(t.max_count);
+                            st_stream(reinterpret_cast<V *>(a.out) + wb + at, v);
+                        }
+                    }
+                } else if (erase_slot_seen<L>(sp, key, tomb, sw)) {
+                    fp_store(t, base_slot + uint64_t(FpWords<W>::slot_of(__ffs(cand) - 1)), kFpTomb);
+                    --live_delta;
+                }
+                finish(kStNone, true);
+                continue;
+            }
+            cand &= cand - 1u;
+            if (cand) continue;
+        }
+        /* no candidate left: absent if the bucket has a free slot */
+        if (any_empty) {
+            const uint32_t st = a.is_set ? kStNone : kStKeyNotFound;
+            if constexpr (OP == kOpRetrieve) join |= st;
+            finish(st, false);
+        } else if (++wins >= a.max_windows) {
+            if constexpr (OP == kOpErase) {
+                finish(a.is_set ? kStNone : kStProbingLengthExceeded, false);
+            } else {
+                join |= kStProbingLengthExceeded;
+                finish(kStProbingLengthExceeded, false);
+            }
+        } else {
+            if (wins == 1) step = probe_step<K>(t, key);
+            bucket = probe_next(t, bucket, step);
         }
     }
     const uint32_t wjoin = __reduce_or_sync(kFull, join);
