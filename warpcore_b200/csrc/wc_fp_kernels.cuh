@@ -18,7 +18,8 @@
  *     erase: its compare-and-swap on the slot follows, with the words read
  *     as the expected value).
  *
- * Inserts run fp_op_kernel, retrieve and erase fp_find_kernel.
+ * Counting inserts run fp_op_kernel, inserts fp_insert_kernel, retrieve and
+ * erase fp_find_kernel.
  *
  * Each lane owns one key and issues one memory operation per wave: a
  * fingerprint load, a candidate slot load, or a compare-and-swap claim.
@@ -180,11 +181,10 @@ __device__ __forceinline__ LaneWords load_slot_once(const unsigned char *sp)
 template <class L, int W, int OP>
 __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_op_kernel(const TableOpArgs a)
 {
-    static_assert(OP == kOpInsert || OP == kOpCount, "operation");
+    static_assert(OP == kOpCount, "operation");
     using K = typename L::key_t;
     using V = typename L::val_t;
     constexpr int SB = L::kSlotBytes;
-    constexpr bool kValueIn = OP == kOpInsert && L::kHasValue;
     enum : int { kPhaseFps = 0, kPhaseCheck = 1, kPhaseClaim = 2, kPhasePreload = 3 };
     const bool preload = (a.flags & kFlagPreloadClaim) != 0;
     const uint64_t pol_keep = l2_policy_evict_last(); /* fingerprint lines */
@@ -205,16 +205,10 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_op_kernel(const Tabl
     const K tomb = K(t.tombstone_key);
     unsigned char *const slots = reinterpret_cast<unsigned char *>(t.slots);
     const K *const keys = reinterpret_cast<const K *>(a.keys);
-    const V *const vals_in = reinterpret_cast<const V *>(a.values);
 
     uint64_t pf_base = wb;
     K pfA = (wb + lane < we) ? ld_stream(keys + wb + lane) : empty;
     K pfB = (wb + 32 + lane < we) ? ld_stream(keys + wb + 32 + lane) : empty;
-    V pvA = 0, pvB = 0;
-    if constexpr (kValueIn) {
-        if (wb + lane < we) pvA = ld_stream(vals_in + wb + lane);
-        if (wb + 32 + lane < we) pvB = ld_stream(vals_in + wb + 32 + lane);
-    }
     uint64_t cursor = wb;
 
     bool has = false, pending = false;
@@ -223,7 +217,6 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_op_kernel(const Tabl
     V claim_expect = 0;
     uint64_t i = 0, bucket = 0, step = 0, wins = 0;
     K key = empty;
-    V val = 0;
     uint32_t st = kStNone, join = 0, cnt_add = 1;
     int live_delta = 0; /* claims minus erases of this lane */
 
@@ -250,14 +243,8 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_op_kernel(const Tabl
         const int off = int(cursor - pf_base) + r;
         const K ka = shfl_any(pfA, off & 31);
         const K kb = shfl_any(pfB, off & 31);
-        V va = 0, vb = 0;
-        if constexpr (kValueIn) {
-            va = shfl_any(pvA, off & 31);
-            vb = shfl_any(pvB, off & 31);
-        }
         if (refill) {
             key = off < 32 ? ka : kb;
-            if constexpr (kValueIn) val = off < 32 ? va : vb;
             i = cursor + r;
             has = true;
             pending = true;
@@ -279,30 +266,22 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_op_kernel(const Tabl
         if (cursor - pf_base >= 32) {
             pf_base += 32;
             pfA = pfB;
-            pvA = pvB;
             const uint64_t nx = pf_base + 32 + lane;
             pfB = nx < we ? ld_stream(keys + nx) : empty;
-            if constexpr (kValueIn) pvB = nx < we ? ld_stream(vals_in + nx) : V(0);
         }
 
-        if constexpr (OP == kOpInsert || OP == kOpCount) {
+        {
             const bool fresh = refill && pending;
             const unsigned fmask = __ballot_sync(kFull, fresh);
             const unsigned peers = __match_any_sync(kFull, fresh ? key : empty) & fmask;
-            int last = lane;
             if (fresh) {
                 const int leader = __ffs(peers) - 1;
-                last = 31 - __clz(peers);
                 cnt_add = __popc(peers);
                 if (lane != leader) {
                     st = kStDuplicateKey;
                     join |= kStDuplicateKey;
                     pending = false;
                 }
-            }
-            if constexpr (kValueIn) {
-                const V lv = shfl_any(val, last);
-                if (fresh) val = lv;
             }
         }
         if constexpr (OP == kOpCount) {
@@ -353,20 +332,14 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_op_kernel(const Tabl
                 const LaneWords sw = load_lane<SB>(sp);
                 const K sk = slot_key<L>(sw, 0);
                 if (sk == key) {
-                    if constexpr (OP == kOpInsert) {
-                        st = kStDuplicateKey;
-                        join |= kStDuplicateKey;
-                        store_value<L>(sp, val);
-                    } else {
-                        st = kStDuplicateKey;
-                        join |= kStDuplicateKey;
-                        count_add<L>(sp, cnt_add, t.max_count, st, join);
-                    }
+                    st = kStDuplicateKey;
+                    join |= kStDuplicateKey;
+                    count_add<L>(sp, cnt_add, t.max_count, st, join);
                     pending = false;
                 } else {
                     /* a set fingerprint over a key that reads empty is
                      * left to the compare-and-swap, which sees the key */
-                    if ((OP == kOpInsert || OP == kOpCount) && sk == empty) emp |= 1u << s;
+                    if (sk == empty) emp |= 1u << s;
                     cand &= cand - 1u;
                 }
             } else if (phase == kPhasePreload) {
@@ -374,7 +347,7 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_op_kernel(const Tabl
                  * slot that is no longer empty is skipped (its key is
                  * another one: equal keys show up as fingerprint matches,
                  * or as the CAS's old key) */
-                if constexpr (OP == kOpInsert || OP == kOpCount) {
+                {
                     int s = __ffs(emp) - 1;
                     const LaneWords sw = load_lane<SB>(slots + (base_slot + uint64_t(s)) * SB);
                     const K sk = slot_key<L>(sw, 0);
@@ -382,8 +355,7 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_op_kernel(const Tabl
                         st = kStDuplicateKey;
                         join |= kStDuplicateKey;
                         unsigned char *const sp = slots + (base_slot + uint64_t(s)) * SB;
-                        if constexpr (OP == kOpInsert) store_value<L>(sp, val);
-                        else count_add<L>(sp, cnt_add, t.max_count, st, join);
+                        count_add<L>(sp, cnt_add, t.max_count, st, join);
                         pending = false;
                     } else if (sk != empty) {
                         emp &= emp - 1u;
@@ -394,10 +366,10 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_op_kernel(const Tabl
                     }
                 }
             } else {
-                if constexpr (OP == kOpInsert || OP == kOpCount) {
+                {
                     const int s = __ffs(emp) - 1;
                     unsigned char *const sp = slots + (base_slot + uint64_t(s)) * SB;
-                    const V payload = OP == kOpCount ? V(cnt_add) : val;
+                    const V payload = V(cnt_add);
                     V old_payload = 0;
                     /* (atom.cas takes no L2 cache hint) */
                     const K old = cas_slot<L>(sp, empty, claim_expect, key, payload, &old_payload);
@@ -413,8 +385,7 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_op_kernel(const Tabl
                     } else if (old == key) {
                         st = kStDuplicateKey;
                         join |= kStDuplicateKey;
-                        if constexpr (OP == kOpInsert) store_value<L>(sp, val);
-                        else count_add<L>(sp, cnt_add, t.max_count, st, join);
+                        count_add<L>(sp, cnt_add, t.max_count, st, join);
                         pending = false;
                     } else if (old == empty) {
                         claim_expect = old_payload; /* free slot, stale payload: again */
@@ -538,6 +509,15 @@ struct FpWords {
         return c;
     }
     static __device__ __forceinline__ int slot_of(int bit) { return (bit >> 3) + 4 * (bit & 7); }
+    /* the empty slots, bit s for slot s (a tombstone above an empty slot may
+     * be marked too: its claim fails) */
+    __device__ __forceinline__ uint32_t empty_slots() const
+    {
+        uint32_t e = 0;
+#pragma unroll
+        for (int k = 0; k < NW; ++k) e |= pack_bytes4(zero_bytes(w[k])) << (4 * k);
+        return e;
+    }
 };
 
 /* Retrieve and erase on tables with fingerprints.  What fp_op_kernel was
@@ -693,6 +673,179 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS_READ) fp_find_kernel(con
         } else {
             if (wins == 1) step = probe_step<K>(t, key);
             bucket = probe_next(t, bucket, step);
+        }
+    }
+    const uint32_t wjoin = __reduce_or_sync(kFull, join);
+    const int wlive = int(__reduce_add_sync(kFull, unsigned(live_delta)));
+    if (lane == 0) {
+        join_status(t.status, wjoin);
+        live_add(t, wlive);
+    }
+}
+
+/* Insert on tables with fingerprints, in the form of fp_find_kernel: the
+ * lanes' fingerprint loads, slot reads and claims are in flight together.
+ * Claims take the lowest slot with an empty fingerprint first, as in
+ * fp_op_kernel; equal keys in one wave meet on that slot, so they need no
+ * merging.  Against fp_op_kernel, which ran the
+ * three steps one after the other: u64 set of 134 MB at load 0.9, 15 M keys
+ * 727 -> 597 us; u64 pairs of 161 MB, 9 M 491 -> 444; u32 pairs of 269 MB, 30 M
+ * 1612 -> 1423; 65 536 updates of 575 MB of u64 pairs 41 -> 33. */
+template <class L, int W>
+__global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_insert_kernel(const TableOpArgs a)
+{
+    using K = typename L::key_t;
+    using V = typename L::val_t;
+    constexpr int SB = L::kSlotBytes;
+    constexpr bool kValueIn = L::kHasValue;
+    const uint64_t pol_keep = l2_policy_evict_last(); /* fingerprint lines */
+
+    const TableView &t = a.t;
+    const int lane = threadIdx.x & 31;
+    const unsigned lanemask_lt = (1u << lane) - 1u;
+    const uint64_t warp = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nwarps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
+
+    /* this warp's contiguous range of keys */
+    uint64_t per = (a.n + nwarps - 1) / nwarps;
+    per = (per + 31) & ~uint64_t(31);
+    const uint64_t wb = warp * per < a.n ? warp * per : a.n;
+    const uint32_t m = uint32_t(wb + per < a.n ? per : a.n - wb);
+    const K empty = K(t.empty_key);
+    const K tomb = K(t.tombstone_key);
+    unsigned char *const slots = reinterpret_cast<unsigned char *>(t.slots);
+    const K *const keys = reinterpret_cast<const K *>(a.keys) + wb;
+    const V *const vals_in = reinterpret_cast<const V *>(a.values) + (kValueIn ? wb : 0);
+
+    uint32_t pf_base = 0, cursor = 0;
+    K pfA = uint32_t(lane) < m ? ld_stream(keys + lane) : empty;
+    K pfB = 32 + uint32_t(lane) < m ? ld_stream(keys + 32 + lane) : empty;
+    V pvA = 0, pvB = 0;
+    if constexpr (kValueIn) {
+        if (uint32_t(lane) < m) pvA = ld_stream(vals_in + lane);
+        if (32 + uint32_t(lane) < m) pvB = ld_stream(vals_in + 32 + lane);
+    }
+
+    /* the key this lane owns: with cand its candidates are to be read, else
+     * with `free` the lowest slot of it is to be claimed, else the bucket's
+     * fingerprints are due */
+    bool has = false;
+    uint32_t cand = 0, free = 0, at = 0;
+    uint64_t bucket = 0, step = 0, wins = 0;
+    K key = empty;
+    V val = 0, expect = 0;
+    uint32_t join = 0;
+    int live_delta = 0;
+
+    auto finish = [&](uint32_t st) {
+        join |= st;
+        if (a.status_out) {
+            if (a.handler == kHandlerStatus)
+                st_stream(reinterpret_cast<uint32_t *>(a.status_out) + wb + at, st);
+            else if (a.handler == kHandlerBoolean)
+                reinterpret_cast<unsigned char *>(a.status_out)[wb + at] =
+                    (unsigned char)((st & a.bool_mask) != 0);
+        }
+        has = false;
+    };
+
+    for (;;) {
+        /* ---- refill lanes whose key is done, in input order ---- */
+        const unsigned need = __ballot_sync(kFull, !has);
+        const uint32_t idle = uint32_t(__popc(need)), avail = m - cursor;
+        const uint32_t take = idle < avail ? idle : avail;
+        if (take == 0 && need == kFull) break;
+        if (take) {
+            const uint32_t r = uint32_t(__popc(need & lanemask_lt));
+            const uint32_t off = cursor - pf_base + r; /* < 64 for refilling lanes */
+            const K ka = shfl_any(pfA, int(off & 31u));
+            const K kb = shfl_any(pfB, int(off & 31u));
+            V va = 0, vb = 0;
+            if constexpr (kValueIn) {
+                va = shfl_any(pvA, int(off & 31u));
+                vb = shfl_any(pvB, int(off & 31u));
+            }
+            if (!has && r < take) {
+                key = off < 32 ? ka : kb;
+                if constexpr (kValueIn) val = off < 32 ? va : vb;
+                at = cursor + r;
+                has = true;
+                cand = 0;
+                free = 0;
+                wins = 0;
+                step = 0;
+                if (key == empty || key == tomb) finish(kStInvalidKey);
+                else bucket = probe_begin<K>(t, key);
+            }
+            cursor += take;
+            if (cursor - pf_base >= 32) {
+                pf_base += 32;
+                pfA = pfB;
+                pvA = pvB;
+                const uint32_t nx = pf_base + 32 + uint32_t(lane);
+                if (nx < m) {
+                    pfB = ld_stream(keys + nx);
+                    if constexpr (kValueIn) pvB = ld_stream(vals_in + nx);
+                }
+            }
+        }
+
+        /* ---- one memory operation per lane with a key ---- */
+        const uint64_t base_slot = bucket * uint64_t(W);
+        FpWords<W> f;
+        LaneWords sw;
+        K old = empty;
+        V old_payload = 0;
+        const uint64_t s = cand ? base_slot + uint64_t(FpWords<W>::slot_of(__ffs(cand) - 1))
+                                : base_slot + uint64_t(free ? __ffs(free) - 1 : 0);
+        unsigned char *const sp = slots + s * SB;
+        const bool checking = cand != 0, claiming = !checking && free != 0;
+        if (has) {
+            /* slots are read where the claims' atomics land (L2): an L1 copy
+             * may predate the claim of an equal key by another lane */
+            if (checking) sw = load_lane<SB>(sp);
+            else if (claiming) old = cas_slot<L>(sp, empty, expect, key, val, &old_payload);
+            else f.load(t.fps + base_slot, pol_keep);
+        }
+        if (!has) continue;
+
+        bool advance = false;
+        if (checking) {
+            if (slot_key<L>(sw, 0) == key) {
+                store_value<L>(sp, val);
+                finish(kStDuplicateKey);
+                continue;
+            }
+            cand &= cand - 1u;
+            advance = cand == 0 && free == 0;
+        } else if (claiming) {
+            if (old == empty && old_payload == expect) {
+                st_hint_u8(t.fps + s, fingerprint(key), pol_keep);
+                ++live_delta;
+                finish(kStNone);
+            } else if (old == key) {
+                store_value<L>(sp, val);
+                finish(kStDuplicateKey);
+            } else if (old == empty) {
+                expect = old_payload; /* free slot, stale payload: again */
+            } else {
+                free &= free - 1u;
+                expect = 0;
+                advance = free == 0;
+            }
+        } else {
+            cand = f.candidates(fingerprint(key) * 0x01010101u);
+            free = f.any_empty() ? f.empty_slots() : 0u;
+            expect = 0;
+            advance = cand == 0 && free == 0;
+        }
+        if (advance) {
+            if (++wins >= a.max_windows) {
+                finish(kStProbingLengthExceeded);
+            } else {
+                if (wins == 1) step = probe_step<K>(t, key);
+                bucket = probe_next(t, bucket, step);
+            }
         }
     }
     const uint32_t wjoin = __reduce_or_sync(kFull, join);
