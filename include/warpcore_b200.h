@@ -602,7 +602,7 @@ int wc_fingerprint_ops(uint32_t op_mask, uint32_t *previous);
  * 3 erase, default all three) instead of with groups of lanes per window
  * and ballots.  Applies to tables whose slot array fits in L2 and whose
  * window is at most 128 bytes (64 bytes for inserts); counting inserts
- * (bit 1) always use the group kernel.  Results are the same either way. */
+ * (bit 1) have kernels of their own.  Results are the same either way. */
 int wc_lane_ops(uint32_t op_mask, uint32_t *previous);
 
 /* ------------------------------------------------------------------ */

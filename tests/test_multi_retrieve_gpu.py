@@ -162,3 +162,44 @@ def test_bucket_list_insert_sizes(kb, vb, cg):
     got = host(st)
     assert set(np.unique(got)) <= {0, 1 << 1, 1 << 7}
     assert np.count_nonzero(got & 2) == len(many) - few.num_keys()
+
+
+@pytest.mark.parametrize("kb,vb,cg", [(4, 4, 8), (8, 8, 8), (4, 8, 16), (8, 4, 4)])
+@pytest.mark.parametrize("bucket", [1, 2, 3, 4])
+def test_multi_bucket_insert_sizes(kb, vb, cg, bucket):
+    # input counts around a warp, its queue of 64 and a full wave; equal keys
+    # in one batch; a limit of values per key; the empty value; full windows
+    keys = o.gen_unique_keys(kb, 148 * 4 * 256 + 1, 83)
+    for n, per in ((1, 1), (31, 1), (33, 2), (64, 3), (97, 2), (len(keys), 1), (30011, 5)):
+        t = wc.MultiBucketHashTable(2 * n * per, key_bytes=kb, value_bytes=vb, bucket_size=bucket,
+                                    cg_size=cg)
+        at = np.random.default_rng(9).permutation(np.repeat(np.arange(n), per))
+        vals = (np.arange(n * per) + 1).astype(DT[vb])
+        st = empty_dev(n * per, 4)
+        t.insert(dev(keys[at]), dev(vals), status_out=st)
+        assert t.num_keys() == n and t.size() == n * per
+        assert np.count_nonzero(host(st) == 0) == n  # one first value per key
+        assert np.count_nonzero(host(st) == 1 << 4) == n * (per - 1)
+        num, b, e, v, _ = retrieve(t, keys[:n], n * per, vb)
+        assert num == n * per
+        owner = np.repeat(np.arange(n), e - b)
+        order = np.argsort(v.view(DT[vb]), kind="stable")
+        assert np.array_equal(v.view(DT[vb])[order], vals)
+        assert np.array_equal(owner[order], at)
+    n = 5003
+    t = wc.MultiBucketHashTable(4 * n, key_bytes=kb, value_bytes=vb, bucket_size=bucket,
+                                cg_size=cg, max_values_per_key=2)
+    st = empty_dev(n, 4)
+    for expect in (0, 1 << 4, (1 << 4) | (1 << 11)):
+        t.insert(dev(keys[:n]), dev((np.arange(n) + 1).astype(DT[vb])), status_out=st)
+        assert (host(st) == expect).all()
+    t.insert(dev(keys[:n]), dev(np.zeros(n, dtype=DT[vb])), status_out=st)
+    assert (host(st) == 1 << 12).all()  # invalid_value
+    few = wc.MultiBucketHashTable(1000, key_bytes=kb, value_bytes=vb, bucket_size=bucket, cg_size=cg)
+    many = o.gen_unique_keys(kb, few.capacity + n, 84)
+    st = empty_dev(len(many), 4)
+    few.insert(dev(many), dev((np.arange(len(many)) + 1).astype(DT[vb])), status_out=st,
+               probing_length=cg)
+    got = host(st)
+    assert set(np.unique(got)) == {0, 1 << 1}
+    assert np.count_nonzero(got == 0) == few.num_keys() == few.num_occupied()

@@ -84,10 +84,7 @@ __global__ void __launch_bounds__(256, WC_MULTI_INSERT_BLOCKS) bl_insert_kernel(
  * that loses its swap goes on in bl_append.  24 M values, 8 per key, in
  * eight rounds: 1993 us with bl_insert_kernel, 1763 now; 16 M u64 values in
  * one batch, 8 per key: 1506 and 1010.  What is left is random reads and
- * compare-and-swaps outside L2.  (The same two steps for the multi-bucket
- * insert measured 2041 -> 1991 us at 2^25 values and 380 -> 468 at 8 M in
- * one batch: its swaps into 168 MB of buckets already run at 16 G/s of the
- * 20 that random atomics reach there.) */
+ * compare-and-swaps outside L2. */
 template <class K, class V, int kW>
 __global__ void __launch_bounds__(kMultiThreads, WC_MULTI_INSERT_BLOCKS)
     bl_insert_tiles_kernel(const BlArgs a)

@@ -424,9 +424,8 @@ __global__ void __launch_bounds__(kMultiThreads, WC_MULTI_VALUES_BLOCKS)
  * multi-value table (u32 pairs, 2^24 into 168 MB, four values per key): 981
  * us with one pair per lane until the warp was done, 679 now.  Used where a
  * step has two kinds: with the four or five kinds of a multi-bucket or
- * bucket-list insert, a warp runs most kinds in every step and the bucket
- * lists' growing lanes no longer share one pool reservation (2048 to 2230
- * us and 1990 to 3330 us). */
+ * bucket-list insert, a warp runs most kinds in every step, so those tables
+ * have kernels of their own. */
 template <class Walk>
 __global__ void __launch_bounds__(256, Walk::kInsertBlocks)
     multi_insert_kernel(const typename Walk::Args a)

@@ -86,6 +86,222 @@ __global__ void __launch_bounds__(256, WC_MULTI_INSERT_BLOCKS) mb_insert_kernel(
     mb_flush(a.m, join, claimed, fresh); /* every lane arrives (no early exit) */
 }
 
+/* Bulk insert, as mb_insert_one, with buckets of two values or more.  A
+ * warp's lanes walk the windows of its range of keys, one window per lane
+ * and step, up to the first with a free slot, and put what they found into
+ * a queue of the warp; a lane whose key is walked takes the next one, so no
+ * lane waits for the longest walk.  Whenever 32 keys are queued, the warp
+ * does for all of them what is left: read the key's last bucket, then swap
+ * the value into a free place of it or claim the free slot.  A key that
+ * loses its swap is inserted from the start by mb_insert_one.
+ *
+ * With one key per lane for the whole insert (mb_insert_kernel), the warp
+ * waited for the longest of 32 walks and then for every other step.  2^25 u32
+ * values, 8 per key in buckets of 4, in eight rounds 2036 -> 1836 us; 16 M u32
+ * values of u64 keys in buckets of 8 865 -> 719; 10 M u64 in buckets of 2 758
+ * -> 730, in one batch 886 -> 733.  Buckets of one value have no last bucket to
+ * read and keep mb_insert_kernel (6 M u64 values of u32 keys 272 us, 313 here).
+ * Tried as well: the two steps per block tile, four keys per thread in the
+ * second (1991 us, in one batch slower), and every step of an insert in one
+ * loop (2230). */
+constexpr int kMbQueue = 64; /* keys a warp's queue holds */
+
+template <class K, class V, int kW, int kB>
+__global__ void __launch_bounds__(256, WC_MULTI_INSERT_BLOCKS)
+    mb_insert_queue_kernel(const MbArgs a)
+{
+    /* slots that stand for: values up to max_values_per_key already (by
+     * slots); windows used up; and for no last slot */
+    constexpr uint64_t kCapped = ~0ull, kLength = ~1ull, kNone = ~0ull;
+    __shared__ uint64_t s_last[8][kMbQueue], s_slot[8][kMbQueue];
+    __shared__ uint32_t s_num[8][kMbQueue], s_at[8][kMbQueue];
+    const MbView &mv = a.m;
+    const TableView &t = mv.t;
+    const uint32_t W = mb_w<kW>(mv), B = mb_b<kB>(mv);
+    const K empty = K(t.empty_key), tomb = K(t.tombstone_key);
+    const V ev = V(mv.empty_value);
+    K *const slots = reinterpret_cast<K *>(t.slots);
+    V *const places = reinterpret_cast<V *>(mv.vals);
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const unsigned lanemask_lt = (1u << lane) - 1u;
+    const uint64_t warp = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nwarps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
+    uint64_t per = (a.n + nwarps - 1) / nwarps;
+    per = (per + 31) & ~uint64_t(31);
+    const uint64_t wb = warp * per < a.n ? warp * per : a.n;
+    const uint32_t m = uint32_t(wb + per < a.n ? per : a.n - wb);
+    const K *const keys = reinterpret_cast<const K *>(a.keys) + wb;
+    const V *const vals = reinterpret_cast<const V *>(a.values) + wb;
+
+    uint32_t join = 0;
+    unsigned claimed = 0, fresh = 0;
+    int queued = 0;
+
+    /* every status but a stored value's none / duplicate_key is joined */
+    auto finish = [&](uint32_t i, uint32_t st) {
+        if (st != kStNone && st != kStDuplicateKey) join |= st;
+        multi_write_status(a, wb + i, st);
+    };
+
+    /* the last `take` queued keys, one per lane */
+    auto place = [&](int take) {
+        queued -= take;
+        const bool in = lane < take;
+        const int q = queued + lane;
+        enum : int { kOver, kPlace, kClaim, kAgain };
+        int todo = kOver;
+        uint64_t slot = 0, last = kNone;
+        uint32_t num = 0, at = 0, e = 0, st = kStNone;
+        K key = K(0), old_key = K(0);
+        V value = V(0), old_value = V(0);
+        if (in) {
+            slot = s_slot[wib][q];
+            last = s_last[wib][q];
+            num = s_num[wib][q];
+            at = s_at[wib][q];
+            key = keys[at];
+            value = vals[at];
+            if (B > 1 && last != kNone)
+                e = mb_bucket_empties<V, kB>(places + last * B, B, ev, nullptr) & ~1u;
+        }
+        __syncwarp();
+        if (in) {
+            todo = kClaim;
+            if (num == 0xffffffffu) {
+                todo = kAgain; /* not counted exactly */
+            } else if (B > 1 && last != kNone) {
+                /* insert_into_bucket (:262-330): place 0 counts as full */
+                const uint64_t before = uint64_t(num) - uint64_t(__popc(e));
+                if (before >= mv.max_values) {
+                    st = kStDuplicateKey | kStMaxValuesReached;
+                    todo = kOver;
+                } else if (e) {
+                    st = before > 0 ? kStDuplicateKey : kStNone;
+                    todo = kPlace;
+                } else if (slot == kCapped) {
+                    st = kStUnknownError;
+                    todo = kOver;
+                } else if (slot == kLength) {
+                    st = kStProbingLengthExceeded | (num > 0 ? kStDuplicateKey : kStNone);
+                    todo = kOver;
+                }
+            }
+            if (todo == kPlace)
+                old_value = mb_cas<V>(places + last * B + (__ffs(e) - 1), ev, value);
+            else if (todo == kClaim)
+                old_key = mb_cas<K>(slots + slot, empty, key);
+        }
+        if (todo == kPlace && old_value != ev) todo = kAgain;
+        if (todo == kClaim) {
+            if (old_key == empty) {
+                /* the bucket's first place, after the key (:446-449) */
+                places[slot * B] = value;
+                ++claimed;
+                fresh += num == 0;
+                st = num == 0 ? kStNone : kStDuplicateKey;
+            } else {
+                todo = kAgain;
+            }
+        }
+        if (todo == kAgain) {
+            bool c = false, f = false;
+            st = mb_insert_one<K, V, kW, kB>(mv, key, value, a.max_windows, c, f);
+            claimed += c;
+            fresh += f;
+        }
+        if (in) finish(at, st);
+        __syncwarp();
+    };
+
+    uint32_t pf_base = 0, cursor = 0;
+    K pfA = uint32_t(lane) < m ? ld_stream(keys + lane) : empty;
+    K pfB = 32 + uint32_t(lane) < m ? ld_stream(keys + 32 + lane) : empty;
+    bool has = false;
+    uint32_t at = 0;
+    K key = K(0);
+    uint64_t bucket = 0, step = 0, wins = 0, num = 0, last = kNone;
+    for (;;) {
+        /* ---- lanes without a key take the next ones, in input order ---- */
+        const unsigned need = __ballot_sync(0xffffffffu, !has);
+        const uint32_t idle = uint32_t(__popc(need)), avail = m - cursor;
+        const uint32_t take = idle < avail ? idle : avail;
+        if (take == 0 && need == 0xffffffffu) break;
+        if (take) {
+            const uint32_t r = uint32_t(__popc(need & lanemask_lt));
+            const uint32_t off = cursor - pf_base + r;
+            const K ka = shfl_any(pfA, int(off & 31u)), kb = shfl_any(pfB, int(off & 31u));
+            if (!has && r < take) {
+                key = off < 32 ? ka : kb;
+                at = cursor + r;
+                const uint32_t st = key == empty || key == tomb ? kStInvalidKey
+                                    : ld_stream(vals + at) == ev ? kStInvalidValue : kStNone;
+                if (st != kStNone) {
+                    finish(at, st);
+                } else {
+                    has = true;
+                    bucket = probe_begin<K>(t, key);
+                    step = 0;
+                    wins = 0;
+                    num = 0;
+                    last = kNone;
+                }
+            }
+            cursor += take;
+            if (cursor - pf_base >= 32) {
+                pf_base += 32;
+                pfA = pfB;
+                const uint32_t nx = pf_base + 32 + uint32_t(lane);
+                if (nx < m) pfB = ld_stream(keys + nx);
+            }
+        }
+
+        /* ---- one window per lane ---- */
+        uint64_t slot = 0;
+        bool walked = false;
+        if (has) {
+            KeyWindow<K, kW> win;
+            win.load(slots + bucket * W, W, key, empty);
+            const uint32_t hits = win.key_slots(key), free = win.free_slots(empty);
+            if (hits) {
+                last = bucket * W + uint64_t(31 - __clz(hits));
+                num += uint64_t(B) * uint64_t(__popc(hits));
+            }
+            if (num >= mv.max_values) {
+                has = false;
+                walked = B > 1 && last != kNone;
+                slot = kCapped;
+                if (!walked) finish(at, kStDuplicateKey | kStMaxValuesReached);
+            } else if (free) {
+                has = false;
+                walked = true;
+                slot = bucket * W + uint64_t(__ffs(free) - 1);
+            } else if (++wins >= a.max_windows) {
+                has = false;
+                walked = B > 1 && last != kNone;
+                slot = kLength;
+                if (!walked)
+                    finish(at, kStProbingLengthExceeded | (num > 0 ? kStDuplicateKey : kStNone));
+            } else {
+                if (wins == 1) step = probe_step<K>(t, key);
+                bucket = probe_next(t, bucket, step);
+            }
+        }
+        const unsigned done = __ballot_sync(0xffffffffu, walked);
+        if (walked) {
+            const int q = queued + __popc(done & lanemask_lt);
+            s_slot[wib][q] = slot;
+            s_last[wib][q] = last;
+            s_num[wib][q] = num < 0xffffffffull ? uint32_t(num) : 0xffffffffu;
+            s_at[wib][q] = at;
+        }
+        queued += __popc(done);
+        __syncwarp();
+        if (queued >= 32) place(32);
+    }
+    if (queued) place(queued);
+    mb_flush(a.m, join, claimed, fresh);
+}
+
 /* the key's slots window by window, as mb_for_each_one walks them: a window
  * is one memory operation; then one bucket each: the last one of the window
  * for the count (its free places are what the count needs), every one for
@@ -241,13 +457,18 @@ __global__ void __launch_bounds__(256) mb_size_kernel(const MbView m, uint64_t c
 }
 
 struct MbKernels {
-    const void *insert, *count, *offsets, *values, *unique, *size;
+    const void *insert_one, *insert_more, *count, *offsets, *values, *unique, *size;
 };
 
 template <class K, class V, int kW, int kB>
 MbKernels mb_kernels_of()
 {
-    return {reinterpret_cast<const void *>(mb_insert_kernel<K, V, kW, kB>),
+    /* buckets of one value, and of more */
+    const void *one = nullptr, *more = nullptr;
+    if constexpr (kB <= 1) one = reinterpret_cast<const void *>(mb_insert_kernel<K, V, kW, kB>);
+    if constexpr (kB != 1)
+        more = reinterpret_cast<const void *>(mb_insert_queue_kernel<K, V, kW, kB>);
+    return {one, more,
             reinterpret_cast<const void *>(multi_find_kernel<MbWalk<K, V, kW, kB>, false>),
             reinterpret_cast<const void *>(multi_find_kernel<MbWalk<K, V, kW, kB>, true>),
             reinterpret_cast<const void *>(multi_values_kernel<MbWalk<K, V, kW, kB>>),
@@ -480,7 +701,9 @@ int wc_mbht_insert(wc_mbht *t, const void *keys_in, const void *values_in, uint6
     if (!keys_in || !values_in) return mb_fail(WC_ERR_INVALID_ARGUMENT, "keys_in / values_in is NULL");
     MbArgs a = args_of(t, keys_in, num_in, probing_length, false, status_out, status_handler, ignore);
     a.values = values_in;
-    return launch(mb_kernels(t).insert, num_in, a, reinterpret_cast<cudaStream_t>(stream));
+    const MbKernels k = mb_kernels(t);
+    return launch(t->bucket == 1 ? k.insert_one : k.insert_more, num_in, a,
+                  reinterpret_cast<cudaStream_t>(stream));
 }
 
 int wc_mbht_num_values(wc_mbht *t, const void *keys_in, uint64_t num_in, uint64_t *num_out,
