@@ -101,3 +101,32 @@ def test_wrapped_count_is_reported():
     for _ in range(2):
         t.insert(one)
     assert int(t.pop_status()) & int(wc.Status.index_overflow())
+
+
+def test_two_threads_with_calls_of_other_sizes():
+    # each call asks for shared memory by its number of keys; threads must
+    # not lower each other's limit
+    import threading
+    keys = o.gen_unique_keys(4, 400000, 85)
+    tables = [wc.CountingHashTable(800000, key_bytes=4) for _ in range(2)]
+    inputs = [dev(keys[:1000]), dev(keys)]
+    torch.cuda.synchronize()
+    errors = []
+
+    def work(t, x):
+        try:
+            s = torch.cuda.Stream()
+            for _ in range(200):
+                t.insert(x, stream=s)
+            s.synchronize()
+        except Exception as e:  # noqa: BLE001 (reported below)
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=a) for a in zip(tables, inputs)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not errors
+    assert (counts_of(tables[0], keys[:1000], 4) == 200).all()
+    assert (counts_of(tables[1], keys, 4) == 200).all()

@@ -922,7 +922,10 @@ int count_insert(wc_table *t, CountInsertKernel k, const void *keys, uint64_t n,
     const size_t smem = k4 ? count_smem_bytes<uint32_t>(a.cache_bits)
                            : count_smem_bytes<uint64_t>(a.cache_bits);
     const void *kfn = reinterpret_cast<const void *>(k);
-    WC_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    /* always the largest size, so that calls of other threads, with other
+     * sizes, never find a smaller limit than they need */
+    const uint32_t most = k4 ? count_smem_bytes<uint32_t>(top) : count_smem_bytes<uint64_t>(top);
+    WC_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most)));
     void *args[] = {&a};
     WC_CUDA(launch_in_window(kfn, grid, kCountThreads, args, s, t->l2, smem));
     if (rebuild) {
