@@ -601,7 +601,7 @@ int wc_fingerprint_ops(uint32_t op_mask, uint32_t *previous);
  * lane reads its key's window with 32-byte loads; bit 0 insert, 2 retrieve,
  * 3 erase, default all three) instead of with groups of lanes per window
  * and ballots.  Applies to tables whose slot array fits in L2 and whose
- * window is at most 128 bytes (64 bytes for inserts); counting inserts
+ * window is at most 128 bytes; counting inserts
  * (bit 1) have kernels of their own.  Results are the same either way. */
 int wc_lane_ops(uint32_t op_mask, uint32_t *previous);
 

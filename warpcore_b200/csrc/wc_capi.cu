@@ -800,17 +800,17 @@ int check_table(const wc_table *t, int kind_mask)
 
 /* The one-key-per-lane window kernel reads a window with one 32-byte load
  * per sector.  On a table that L2 holds, that beats groups of lanes per
- * window and their ballots (B200, CUDA events: u32 pairs, 16 MB table:
- * retrieve 60.2 vs 38.0 G keys/s, insert 21.1 vs 18.0; u64 pairs, 48 MB:
- * retrieve 29.5 vs 16.8, insert 13.2 vs 14.8).  On a table in DRAM its
- * sector requests cost more than one request per window (u64 pairs,
- * 2.4 GB: insert 5.9 vs 14.5), so larger tables keep the group kernel.
- * Inserts take the lane kernel for windows of at most 64 bytes. */
+ * window and their ballots, for every window of at most 128 bytes (B200,
+ * group / lane kernel: u32 pairs, 16 MB, lookups 38.0 / 60.2 G keys/s; u64
+ * pairs at load 0.72, 67 MB, 3 M inserts 175 / 136 us; u64 keys with u32
+ * values, 50 MB, 2 M inserts 121 / 93; u64 set at CG 16, 4 M inserts 244 /
+ * 142).  On a table in DRAM its sector requests cost more than one request
+ * per window (u64 pairs, 2.4 GB: insert 5.9 vs 14.5), so larger tables keep
+ * the group kernel. */
 TableKernel pick_lane_kernel(const wc_table *t, int op)
 {
     if (!((g_lane_ops.load(std::memory_order_relaxed) >> op) & 1u)) return nullptr;
     if (t->capacity * t->slot_bytes > uint64_t(device_props().l2_bytes)) return nullptr;
-    if (op == kOpInsert && uint64_t(t->cfg.cg_size) * t->slot_bytes > 64) return nullptr;
     const int W = int(t->cfg.cg_size);
     switch (t->layout) {
     case kLayoutKV32: return lane_kernel_kv32(W, op);
