@@ -49,7 +49,8 @@ def test_tile_edges(kind, kb, vb):
         t.insert(dev(keys), dev(np.ascontiguousarray(values[:, j])))
     # a bucket list is read newest bucket first: buckets of 1, 2, 3 values
     order = [3, 4, 1, 2, 0] if kind == "bl" else range(per)
-    for n in (1, 31, 255, 256, 257, 1024, 1025, 148 * 4 * 256 + 1, 148 * 4 * 1024 + 1025):
+    for n in (1, 31, 255, 256, 257, 1024, 1025, 2048, 2049, 148 * 6 * 256 + 1,
+              148 * 6 * 1024 + 1025, 148 * 6 * 2048 + 2049):
         at = rng.integers(0, 2 * nkeys, size=n)
         hit = at < nkeys
         cnt = np.where(hit, per, 0)

@@ -269,6 +269,7 @@ struct BlWalk {
     using key_t = K;
     using val_t = V;
     using Args = BlArgs;
+    static constexpr int kFindTile = multi_find_tile(sizeof(K), kW * int(sizeof(K)));
     struct State {
         uint64_t bucket, step, wins, num;
         uint64_t at;    /* the key's slot, then the list bucket's pool index */
@@ -420,13 +421,15 @@ __global__ void __launch_bounds__(256) bl_scan_keys_kernel(const BlView v, uint6
 }
 
 struct BlKernels {
+    uint32_t find_tile;
     const void *insert, *insert_tiles, *count, *offsets, *values, *init, *scan;
 };
 
 template <class K, class V, int kW>
 BlKernels bl_kernels_of()
 {
-    return {reinterpret_cast<const void *>(bl_insert_kernel<K, V, kW>),
+    return {BlWalk<K, V, kW>::kFindTile,
+            reinterpret_cast<const void *>(bl_insert_kernel<K, V, kW>),
             reinterpret_cast<const void *>(bl_insert_tiles_kernel<K, V, kW>),
             reinterpret_cast<const void *>(multi_find_kernel<BlWalk<K, V, kW>, false>),
             reinterpret_cast<const void *>(multi_find_kernel<BlWalk<K, V, kW>, true>),
@@ -521,7 +524,8 @@ int count(wc_blht *t, const void *keys, uint64_t n, uint64_t *counts_dev, uint64
           cudaStream_t s, uint64_t probing_length, void *status_out, int handler, uint32_t ignore)
 {
     BlArgs a = args_of(t, keys, n, probing_length, status_out, handler, ignore);
-    return host_multi_count(bl_kernels(t).count, &a, &a, t->counters + 8, counts_dev, total, s);
+    const BlKernels k = bl_kernels(t);
+    return host_multi_count(k.count, k.find_tile, &a, &a, t->counters + 8, counts_dev, total, s);
 }
 
 int join_host(wc_blht *t, uint32_t bits, cudaStream_t s)
@@ -718,7 +722,7 @@ int wc_blht_retrieve(wc_blht *t, const void *keys_in, uint64_t num_in,
     }
     BlArgs a = args_of(t, keys_in, num_in, probing_length, status_out, status_handler, ignore);
     const BlKernels k = bl_kernels(t);
-    return host_multi_retrieve(k.offsets, k.values, &a, &a, &t->scan, &t->scan_bytes,
+    return host_multi_retrieve(k.offsets, k.find_tile, k.values, &a, &a, &t->scan, &t->scan_bytes,
                                begin_offsets_out, end_offsets_out, values_out, num_out, s);
 }
 

@@ -383,9 +383,9 @@ uint64_t warpcore::b200::host_valid_capacity(uint64_t min_capacity, uint64_t cg)
 
 namespace {
 
-/* A tile is at most kMultiTile keys and small enough that every resident
+/* A tile is at most `most` keys and small enough that every resident
  * block gets one, in steps of a block's threads: a small call then walks one
- * key per lane on all SMs, and a large one draws four keys per lane. */
+ * key per lane on all SMs, and a large one draws four or eight keys per lane. */
 int multi_launch(const void *kernel, MultiArgs *a, void *args, cudaStream_t s)
 {
     void *kargs[] = {args};
@@ -397,12 +397,12 @@ int multi_launch(const void *kernel, MultiArgs *a, void *args, cudaStream_t s)
     return WC_OK;
 }
 
-uint32_t multi_tile(const void *kernel, uint64_t n)
+uint32_t multi_tile(const void *kernel, uint64_t n, uint32_t most = kMultiTile)
 {
     const uint64_t wave = uint64_t(device_props().sms) * blocks_per_sm(kernel, kMultiThreads);
     uint64_t tile = (n + wave - 1) / wave;
     tile = (tile + kMultiThreads - 1) / kMultiThreads * kMultiThreads;
-    return uint32_t(tile < kMultiTile ? tile : kMultiTile);
+    return uint32_t(tile < most ? tile : most);
 }
 
 /* the sum of the counts, read back */
@@ -426,11 +426,11 @@ int warpcore::b200::host_multi_launch(const void *tile_kernel, MultiArgs *a, voi
     return multi_launch(tile_kernel, a, args, s);
 }
 
-int warpcore::b200::host_multi_count(const void *count_kernel, MultiArgs *a, void *args,
-                                     unsigned long long *look, uint64_t *counts, uint64_t *total,
+int warpcore::b200::host_multi_count(const void *count_kernel, uint32_t find_tile, MultiArgs *a,
+                                     void *args, unsigned long long *look, uint64_t *counts, uint64_t *total,
                                      cudaStream_t s)
 {
-    a->tile = multi_tile(count_kernel, a->n);
+    a->tile = multi_tile(count_kernel, a->n, find_tile);
     a->look = look;
     a->counts_out = reinterpret_cast<unsigned long long *>(counts);
     WC_CUDA(cudaMemsetAsync(look, 0, kLookTiles * sizeof(unsigned long long), s));
@@ -438,12 +438,12 @@ int warpcore::b200::host_multi_count(const void *count_kernel, MultiArgs *a, voi
     return rc ? rc : multi_total(a, total, s);
 }
 
-int warpcore::b200::host_multi_retrieve(const void *offsets_kernel, const void *values_kernel,
-                                        MultiArgs *a, void *args, void **scratch,
+int warpcore::b200::host_multi_retrieve(const void *offsets_kernel, uint32_t find_tile,
+                                        const void *values_kernel, MultiArgs *a, void *args, void **scratch,
                                         uint64_t *scratch_bytes, uint64_t *begin, uint64_t *end,
                                         void *values_out, uint64_t *total, cudaStream_t s)
 {
-    a->tile = multi_tile(offsets_kernel, a->n);
+    a->tile = multi_tile(offsets_kernel, a->n, find_tile);
     const uint64_t ntiles = (a->n + a->tile - 1) / a->tile;
     const uint64_t need = (kLookTiles + ntiles) * sizeof(unsigned long long);
     if (need > *scratch_bytes) {
@@ -1434,7 +1434,7 @@ int mv_count(wc_table *t, const void *keys, uint64_t n, uint64_t *counts_dev, ui
     const MvKernels k = mv_kernels(t->layout, int(t->cfg.cg_size));
     if (!k.count) return fail(WC_ERR_UNSUPPORTED, "no kernel for this configuration");
     MvArgs a = mv_args(t, keys, n, probing_length, true, status_out, handler, ignore);
-    return host_multi_count(k.count, &a, &a, t->counter, counts_dev, total, s);
+    return host_multi_count(k.count, k.find_tile, &a, &a, t->counter, counts_dev, total, s);
 }
 
 int mv_join(wc_table *t, uint32_t bits, cudaStream_t s)
@@ -1502,7 +1502,7 @@ int wc_mvht_retrieve(wc_table *t, const void *keys_in, uint64_t num_in,
     if (!k.values) return fail(WC_ERR_UNSUPPORTED, "no kernel for this configuration");
     MvArgs a = mv_args(t, keys_in, num_in, probing_length, true, status_out, status_handler,
                        ignore);
-    return host_multi_retrieve(k.offsets, k.values, &a, &a, &t->scratch, &t->scratch_bytes,
+    return host_multi_retrieve(k.offsets, k.find_tile, k.values, &a, &a, &t->scratch, &t->scratch_bytes,
                                begin_offsets_out, end_offsets_out, values_out, num_out, s);
 }
 

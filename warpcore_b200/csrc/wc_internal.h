@@ -86,6 +86,7 @@ const void *batch_kernel_ptr(int layout, int W, bool inline_desc);
 struct MvKernels {
     const void *insert = nullptr, *count = nullptr, *offsets = nullptr, *values = nullptr,
                *unique = nullptr;
+    uint32_t find_tile = 0; /* keys per tile of count and offsets */
 };
 MvKernels mv_kernels(int layout, int W);
 MvKernels mv_kernels_mixed(int layout, int W); /* u32/u64 and u64/u32 */
@@ -107,10 +108,10 @@ uint64_t host_valid_capacity(uint64_t min_capacity, uint64_t cg);
  * counter read back.  host_multi_count uses the kLookTiles words at `look`,
  * host_multi_retrieve a scratch array grown on demand; both synchronise. */
 int host_multi_launch(const void *tile_kernel, MultiArgs *a, void *args, cudaStream_t s);
-int host_multi_count(const void *count_kernel, MultiArgs *a, void *args, unsigned long long *look,
-                     uint64_t *counts, uint64_t *total, cudaStream_t s);
-int host_multi_retrieve(const void *offsets_kernel, const void *values_kernel, MultiArgs *a,
-                        void *args, void **scratch, uint64_t *scratch_bytes, uint64_t *begin,
+int host_multi_count(const void *count_kernel, uint32_t find_tile, MultiArgs *a, void *args,
+                     unsigned long long *look, uint64_t *counts, uint64_t *total, cudaStream_t s);
+int host_multi_retrieve(const void *offsets_kernel, uint32_t find_tile, const void *values_kernel,
+                        MultiArgs *a, void *args, void **scratch, uint64_t *scratch_bytes, uint64_t *begin,
                         uint64_t *end, void *values_out, uint64_t *total, cudaStream_t s);
 int host_join_status(uint32_t *status, uint32_t bits, cudaStream_t s);
 int host_dry_run_status(void *status_out, uint64_t n, int handler, uint32_t ignore, cudaStream_t s);

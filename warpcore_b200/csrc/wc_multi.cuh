@@ -68,7 +68,7 @@ struct MultiArgs {
     void *status_out;
     uint64_t n;
     uint64_t max_windows;
-    uint32_t tile;                  /* keys per tile, at most kMultiTile */
+    uint32_t tile;                  /* keys per tile */
     uint32_t bool_mask;
     int handler;
 };
@@ -76,6 +76,15 @@ struct MultiArgs {
 /* keys per tile: four per thread, so that a lane draws a few times before
  * the tile's last walks leave lanes idle */
 constexpr int kMultiTile = 1024;
+/* keys per tile of multi_find_kernel, whose last walks leave lanes idle at a
+ * barrier (a quarter of its stalls at 1024 keys).  2048 where keys take 4
+ * bytes and windows at most 64; with more, the shared memory of six blocks
+ * leaves L1 too small for the windows in flight (1024 / 2048: u32 pairs 380 /
+ * 357 us, multi-bucket of u32 keys 586 / 550, u64 pairs 280 / 436). */
+constexpr int multi_find_tile(int key_bytes, int window_bytes)
+{
+    return key_bytes == 4 && window_bytes <= 64 ? 2 * kMultiTile : kMultiTile;
+}
 constexpr int kMultiThreads = 256;
 
 /* look-back words: ticket, total, timeout flag, then one word per tile */
@@ -241,8 +250,9 @@ __global__ void __launch_bounds__(kMultiThreads, WC_MULTI_COUNT_BLOCKS)
     multi_find_kernel(const typename Walk::Args a)
 {
     using K = typename Walk::key_t;
-    __shared__ K s_key[kMultiTile];
-    __shared__ unsigned long long s_end[kMultiTile]; /* counts, then end offsets in the tile */
+    constexpr int kTile = Walk::kFindTile;
+    __shared__ K s_key[kTile];
+    __shared__ unsigned long long s_end[kTile]; /* counts, then end offsets in the tile */
     __shared__ int s_drawn;
     __shared__ unsigned long long s_before;
     __shared__ uint64_t s_tile;
@@ -297,7 +307,7 @@ __global__ void __launch_bounds__(kMultiThreads, WC_MULTI_COUNT_BLOCKS)
         __syncthreads();
 
         /* ---- offsets ---- */
-        constexpr int kPer = kMultiTile / kMultiThreads;
+        constexpr int kPer = kTile / kMultiThreads;
         unsigned long long c[kPer], sum = 0, excl = 0;
 #pragma unroll
         for (int j = 0; j < kPer; ++j) {

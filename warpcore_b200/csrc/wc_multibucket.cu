@@ -311,6 +311,7 @@ struct MbWalk {
     using key_t = K;
     using val_t = V;
     using Args = MbArgs;
+    static constexpr int kFindTile = multi_find_tile(sizeof(K), kW * int(sizeof(K)));
     struct State {
         uint64_t bucket, step, wins, num;
         uint32_t hits; /* slots of the window whose buckets are still to be read */
@@ -457,6 +458,7 @@ __global__ void __launch_bounds__(256) mb_size_kernel(const MbView m, uint64_t c
 }
 
 struct MbKernels {
+    uint32_t find_tile;
     const void *insert_one, *insert_more, *count, *offsets, *values, *unique, *size;
 };
 
@@ -468,7 +470,7 @@ MbKernels mb_kernels_of()
     if constexpr (kB <= 1) one = reinterpret_cast<const void *>(mb_insert_kernel<K, V, kW, kB>);
     if constexpr (kB != 1)
         more = reinterpret_cast<const void *>(mb_insert_queue_kernel<K, V, kW, kB>);
-    return {one, more,
+    return {MbWalk<K, V, kW, kB>::kFindTile, one, more,
             reinterpret_cast<const void *>(multi_find_kernel<MbWalk<K, V, kW, kB>, false>),
             reinterpret_cast<const void *>(multi_find_kernel<MbWalk<K, V, kW, kB>, true>),
             reinterpret_cast<const void *>(multi_values_kernel<MbWalk<K, V, kW, kB>>),
@@ -571,7 +573,8 @@ int count(wc_mbht *t, const void *keys, uint64_t n, uint64_t *counts_dev, uint64
           cudaStream_t s, uint64_t probing_length, void *status_out, int handler, uint32_t ignore)
 {
     MbArgs a = args_of(t, keys, n, probing_length, true, status_out, handler, ignore);
-    return host_multi_count(mb_kernels(t).count, &a, &a, t->counters + 8, counts_dev, total, s);
+    const MbKernels k = mb_kernels(t);
+    return host_multi_count(k.count, k.find_tile, &a, &a, t->counters + 8, counts_dev, total, s);
 }
 
 /* host join of status bits into the table's Status word */
@@ -745,7 +748,7 @@ int wc_mbht_retrieve(wc_mbht *t, const void *keys_in, uint64_t num_in,
     }
     MbArgs a = args_of(t, keys_in, num_in, probing_length, true, status_out, status_handler, ignore);
     const MbKernels k = mb_kernels(t);
-    return host_multi_retrieve(k.offsets, k.values, &a, &a, &t->scan, &t->scan_bytes,
+    return host_multi_retrieve(k.offsets, k.find_tile, k.values, &a, &a, &t->scan, &t->scan_bytes,
                                begin_offsets_out, end_offsets_out, values_out, num_out, s);
 }
 

@@ -35,6 +35,7 @@ struct MvWalk {
     using key_t = typename L::key_t;
     using val_t = typename L::val_t;
     using Args = MvArgs;
+    static constexpr int kFindTile = multi_find_tile(sizeof(key_t), W * L::kSlotBytes);
     struct State {
         uint64_t bucket, step, wins, num;
     };

@@ -20,6 +20,7 @@ MvKernels mv_pick()
     k.offsets = reinterpret_cast<const void *>(multi_find_kernel<MvWalk<L, W>, true>);
     k.values = reinterpret_cast<const void *>(multi_values_kernel<MvWalk<L, W>>);
     k.unique = reinterpret_cast<const void *>(mv_unique_keys_kernel<L, W>);
+    k.find_tile = MvWalk<L, W>::kFindTile;
     return k;
 }
 
