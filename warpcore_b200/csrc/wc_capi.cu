@@ -383,9 +383,7 @@ uint64_t warpcore::b200::host_valid_capacity(uint64_t min_capacity, uint64_t cg)
 
 namespace {
 
-/* A tile is at most `most` keys and small enough that every resident
- * block gets one, in steps of a block's threads: a small call then walks one
- * key per lane on all SMs, and a large one draws four or eight keys per lane. */
+/* one block per tile of a->tile keys, at most one wave */
 int multi_launch(const void *kernel, MultiArgs *a, void *args, cudaStream_t s)
 {
     void *kargs[] = {args};
@@ -397,6 +395,9 @@ int multi_launch(const void *kernel, MultiArgs *a, void *args, cudaStream_t s)
     return WC_OK;
 }
 
+/* A tile is at most `most` keys and small enough that every resident
+ * block gets one, in steps of a block's threads: a small call then walks one
+ * key per lane on all SMs, and a large one draws four or eight keys per lane. */
 uint32_t multi_tile(const void *kernel, uint64_t n, uint32_t most = kMultiTile)
 {
     const uint64_t wave = uint64_t(device_props().sms) * blocks_per_sm(kernel, kMultiThreads);
@@ -408,12 +409,10 @@ uint32_t multi_tile(const void *kernel, uint64_t n, uint32_t most = kMultiTile)
 /* the sum of the counts, read back */
 int multi_total(const MultiArgs *a, uint64_t *total, cudaStream_t s)
 {
-    unsigned long long h[kLookFailed + 1] = {0};
-    WC_CUDA(cudaMemcpyAsync(h, a->look, sizeof(h), cudaMemcpyDeviceToHost, s));
+    unsigned long long h = 0;
+    WC_CUDA(cudaMemcpyAsync(&h, a->look + kLookTotal, sizeof(h), cudaMemcpyDeviceToHost, s));
     WC_CUDA(cudaStreamSynchronize(s));
-    if (h[kLookFailed])
-        return fail(WC_ERR_TIMEOUT, "retrieve: the wait for an earlier tile's offsets ran out");
-    *total = h[kLookTotal];
+    *total = h;
     return WC_OK;
 }
 
@@ -465,10 +464,9 @@ int warpcore::b200::host_multi_retrieve(const void *offsets_kernel, uint32_t fin
         a->begin_out = nullptr;
     }
     a->values_out = values_out;
-    WC_CUDA(cudaMemsetAsync(*scratch, 0, need, s));
+    WC_CUDA(cudaMemsetAsync(*scratch, 0, kLookTiles * sizeof(unsigned long long), s));
     int rc = multi_launch(offsets_kernel, a, args, s);
     if (rc) return rc;
-    a->tile = multi_tile(values_kernel, a->n);
     rc = multi_launch(values_kernel, a, args, s);
     return rc ? rc : multi_total(a, total, s);
 }

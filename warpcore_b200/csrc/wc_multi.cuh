@@ -9,15 +9,15 @@
  * The reference counts the values of every key, scans the counts into
  * offsets and walks every key again to copy its values.  Here two kernels
  * do it:
- *   multi_find_kernel counts and makes the offsets.  A block takes a tile
- *     of keys and walks them; the tile's counts are scanned in the block,
- *     and the values of all earlier tiles are summed by looking back over
- *     the tiles' published sums (one 64-bit word each: a tile's own sum,
- *     then the sum up to its end).  Tiles are handed out in order by a
- *     ticket, so a tile waits only for tiles that already run; the wait has
- *     a limit all the same, after which the call reports a timeout.
- *   multi_values_kernel walks the keys that have values, up to the window
- *     where the last of them is, and copies the values as it meets them.
+ *   multi_find_kernel counts.  A block takes a tile of keys, walks them and
+ *     scans the counts in the block: every key gets its end offset within
+ *     its tile, every tile its sum.  The block that finishes last turns the
+ *     tiles' sums into the tiles' offsets.
+ *   multi_values_kernel adds each tile's offset to its keys' offsets, walks
+ *     the keys that have values, up to the window where the last of them is,
+ *     and copies the values as it meets them.
+ * No block waits for another: one walk may be as long as the whole table
+ * (an absent key in a full one), and a slow tile then delays only the call.
  *
  * Both are bound by the latency of the walks' dependent reads.  A walk ends
  * at the first window with a free slot: at load 0.8 its mean is 2 to 3
@@ -64,7 +64,7 @@ struct MultiArgs {
     unsigned long long *end_out;
     unsigned long long *begin_first;
     unsigned long long *counts_out; /* num_values: per key, or NULL */
-    unsigned long long *look;       /* look-back words, see kLook* */
+    unsigned long long *look;       /* scratch words, see kLook* */
     void *status_out;
     uint64_t n;
     uint64_t max_windows;
@@ -87,13 +87,10 @@ constexpr int multi_find_tile(int key_bytes, int window_bytes)
 }
 constexpr int kMultiThreads = 256;
 
-/* look-back words: ticket, total, timeout flag, then one word per tile */
-constexpr int kLookTicket = 0, kLookTotal = 1, kLookFailed = 2, kLookTiles = 4;
-constexpr unsigned long long kLookSum = 1ull << 62;  /* the tile's own sum */
-constexpr unsigned long long kLookEnd = 2ull << 62;  /* the sum up to its end */
-constexpr unsigned long long kLookBad = 3ull << 62;  /* a wait ran out */
-constexpr unsigned long long kLookMask = (1ull << 62) - 1;
-constexpr uint32_t kLookPolls = 1u << 21; /* of at least 64 ns each */
+/* scratch words: the next tile, the blocks that are done, the sum of all
+ * counts, then (retrieve) one word per tile: its sum, later its offset.  The
+ * first kLookTiles are zeroed before a call. */
+constexpr int kLookTicket = 0, kLookDone = 1, kLookTotal = 2, kLookTiles = 4;
 
 __device__ __forceinline__ void multi_write_status(const MultiArgs &a, uint64_t i, uint32_t st)
 {
@@ -103,15 +100,6 @@ __device__ __forceinline__ void multi_write_status(const MultiArgs &a, uint64_t 
     else if (a.handler == kHandlerBoolean)
         reinterpret_cast<unsigned char *>(a.status_out)[i] =
             (unsigned char)((st & a.bool_mask) != 0);
-}
-
-__device__ __forceinline__ unsigned long long look_load(const unsigned long long *p)
-{
-    return *reinterpret_cast<const volatile unsigned long long *>(p);
-}
-__device__ __forceinline__ void look_store(unsigned long long *p, unsigned long long v)
-{
-    *reinterpret_cast<volatile unsigned long long *>(p) = v;
 }
 
 /* exclusive scan over the block of one value per thread; returns the total */
@@ -145,34 +133,32 @@ __device__ __forceinline__ unsigned long long block_exclusive_scan(unsigned long
     return total;
 }
 
-/* The sum of all tiles before `tile`, by one warp (every lane returns it):
- * 32 tiles' words at a time, nearest first, until one holds the sum up to
- * its end.  kLookBad if a word is not written within kLookPolls polls. */
-__device__ __forceinline__ unsigned long long look_back(const unsigned long long *words,
-                                                        uint64_t tile, int lane)
+/* By the block that is done last: the tiles' sums to their offsets, in
+ * place, and the sum of all.  The sums were written by other blocks of this
+ * launch, each followed by a fence and the block's count in kLookDone. */
+__device__ __forceinline__ void scan_tile_sums(unsigned long long *look, uint64_t ntiles)
 {
-    unsigned long long sum = 0;
-    uint64_t upto = tile; /* words [.., upto) are still to be added */
-    uint32_t polls = 0;
-    while (upto > 0) {
-        const bool in = uint64_t(lane) < upto;
-        const unsigned long long w = in ? look_load(words + (upto - 1 - uint64_t(lane))) : kLookEnd;
-        const unsigned long long kind = w & ~kLookMask;
-        if (__any_sync(kFull, kind == kLookBad)) return kLookBad;
-        const unsigned ends = __ballot_sync(kFull, kind == kLookEnd);
-        const unsigned none = __ballot_sync(kFull, kind == 0);
-        const int last = ends ? __ffs(ends) - 1 : 31; /* the nearest tile whose end is known */
-        const unsigned used = last == 31 ? kFull : ((1u << (last + 1)) - 1u);
-        if (none & used) {
-            if (++polls > kLookPolls) return kLookBad;
-            __nanosleep(64);
-            continue;
+    constexpr int kPer = 4;
+    unsigned long long *const words = look + kLookTiles;
+    unsigned long long before = 0;
+    for (uint64_t at = 0; at < ntiles; at += uint64_t(blockDim.x) * kPer) {
+        const uint64_t i0 = at + uint64_t(threadIdx.x) * kPer;
+        unsigned long long c[kPer], sum = 0, excl = 0;
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            c[j] = i0 + j < ntiles ? __ldcg(words + i0 + j) : 0ull;
+            sum += c[j];
         }
-        sum += warp_sum_u64(lane <= last ? (w & kLookMask) : 0ull);
-        if (ends) break;
-        upto -= 32;
+        const unsigned long long total = block_exclusive_scan(sum, excl);
+        excl += before;
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            if (i0 + j < ntiles) words[i0 + j] = excl;
+            excl += c[j];
+        }
+        before += total;
     }
-    return sum;
+    if (threadIdx.x == 0) look[kLookTotal] = before;
 }
 
 /* A window of W keys read by one lane, loaded first and looked at later, so
@@ -244,7 +230,8 @@ __device__ __forceinline__ bool draw_key(bool has, int m, int *drawn, bool &left
 }
 
 /* num_values (kOffsets false): per-key counts and their sum; the first half
- * of retrieve (kOffsets): begin / end offsets and the sum */
+ * of retrieve (kOffsets): end offsets within the tiles, the tiles' offsets
+ * and the sum */
 template <class Walk, bool kOffsets>
 __global__ void __launch_bounds__(kMultiThreads, WC_MULTI_COUNT_BLOCKS)
     multi_find_kernel(const typename Walk::Args a)
@@ -254,7 +241,6 @@ __global__ void __launch_bounds__(kMultiThreads, WC_MULTI_COUNT_BLOCKS)
     __shared__ K s_key[kTile];
     __shared__ unsigned long long s_end[kTile]; /* counts, then end offsets in the tile */
     __shared__ int s_drawn;
-    __shared__ unsigned long long s_before;
     __shared__ uint64_t s_tile;
 
     const int lane = threadIdx.x & 31;
@@ -322,9 +308,10 @@ __global__ void __launch_bounds__(kMultiThreads, WC_MULTI_COUNT_BLOCKS)
                     a.counts_out[base + uint64_t(i)] = s_end[i];
             if (threadIdx.x == 0 && total) atomicAdd(a.look + kLookTotal, total);
         } else {
-            unsigned long long *const words = a.look + kLookTiles;
-            if (threadIdx.x == 0)
-                look_store(words + tile, tile == 0 ? (kLookEnd | total) : (kLookSum | total));
+            if (threadIdx.x == 0) {
+                a.look[kLookTiles + tile] = total;
+                __threadfence();
+            }
             unsigned long long run = excl;
 #pragma unroll
             for (int j = 0; j < kPer; ++j) {
@@ -332,37 +319,29 @@ __global__ void __launch_bounds__(kMultiThreads, WC_MULTI_COUNT_BLOCKS)
                 const int i = int(threadIdx.x) * kPer + j;
                 if (i < m) s_end[i] = run;
             }
-            if (threadIdx.x < 32) {
-                const unsigned long long before = look_back(words, tile, lane);
-                if (lane == 0) {
-                    s_before = before;
-                    if (before == kLookBad) {
-                        look_store(words + tile, kLookBad);
-                        look_store(a.look + kLookFailed, 1ull);
-                    } else {
-                        if (tile) look_store(words + tile, kLookEnd | (before + total));
-                        if (tile + 1 == ntiles) look_store(a.look + kLookTotal, before + total);
-                    }
-                }
-            }
             __syncthreads();
-            const unsigned long long before = s_before;
-            if (before == kLookBad) break; /* the host reports the timeout */
-            if (a.begin_first && tile == 0 && threadIdx.x == 0) *a.begin_first = 0;
-            for (int i = threadIdx.x; i < m; i += kMultiThreads) {
-                a.end_out[base + uint64_t(i)] = before + s_end[i];
-                if (a.begin_out)
-                    a.begin_out[base + uint64_t(i)] = before + (i ? s_end[i - 1] : 0ull);
-            }
+            for (int i = threadIdx.x; i < m; i += kMultiThreads)
+                a.end_out[base + uint64_t(i)] = s_end[i];
         }
         __syncthreads(); /* the shared rows are rewritten by the next tile */
     }
     const uint32_t wj = __reduce_or_sync(kFull, join);
     if (lane == 0) join_status(Walk::view(a).status, wj);
+    if constexpr (kOffsets) {
+        if (threadIdx.x == 0) {
+            const bool last = atomicAdd(a.look + kLookDone, 1ull) + 1 == gridDim.x;
+            __threadfence();
+            s_drawn = int(last);
+        }
+        __syncthreads();
+        if (s_drawn) scan_tile_sums(a.look, ntiles);
+    }
 }
 
-/* the second half of retrieve: every key's values, inside its own segment
- * [begin, end) only.  A tile's keys without values are dropped first. */
+/* the second half of retrieve, with the tiles of the first: the keys'
+ * offsets, and every key's values, inside its own segment [begin, end) only.
+ * A tile is taken kMultiTile keys at a time; those without values are dropped
+ * first. */
 template <class Walk>
 __global__ void __launch_bounds__(kMultiThreads, WC_MULTI_VALUES_BLOCKS)
     multi_values_kernel(const typename Walk::Args a)
@@ -372,56 +351,73 @@ __global__ void __launch_bounds__(kMultiThreads, WC_MULTI_VALUES_BLOCKS)
     __shared__ K s_key[kMultiTile];
     __shared__ unsigned long long s_begin[kMultiTile], s_room[kMultiTile];
     __shared__ int s_drawn, s_found;
-    if (look_load(a.look + kLookFailed)) return;
 
     const int lane = threadIdx.x & 31;
     const K *const keys = reinterpret_cast<const K *>(a.keys);
-    for (uint64_t base = uint64_t(blockIdx.x) * a.tile; base < a.n;
-         base += uint64_t(gridDim.x) * a.tile) {
-        if (threadIdx.x == 0) {
-            s_drawn = 0;
-            s_found = 0;
-        }
-        __syncthreads();
-        const int m = int(a.n - base < a.tile ? a.n - base : a.tile);
-        for (int i0 = 0; i0 < m; i0 += kMultiThreads) {
-            const int i = i0 + int(threadIdx.x);
-            unsigned long long begin = 0, room = 0;
-            if (i < m) {
-                const unsigned long long end = a.end_out[base + uint64_t(i)];
-                begin = a.begin_out ? a.begin_out[base + uint64_t(i)]
-                                    : a.begin_first[base + uint64_t(i)];
-                room = end - begin;
+    if (a.begin_first && blockIdx.x == 0 && threadIdx.x == 0) *a.begin_first = 0;
+    const uint64_t ntiles = (a.n + a.tile - 1) / a.tile;
+    for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const uint64_t tile_base = tile * a.tile;
+        const int tile_m = int(a.n - tile_base < a.tile ? a.n - tile_base : a.tile);
+        const unsigned long long before = a.look[kLookTiles + tile];
+        unsigned long long part_begin = 0; /* of the part, within the tile */
+        for (int part = 0; part < tile_m; part += kMultiTile) {
+            const uint64_t base = tile_base + uint64_t(part);
+            const int m = tile_m - part < kMultiTile ? tile_m - part : kMultiTile;
+            if (threadIdx.x == 0) {
+                s_drawn = 0;
+                s_found = 0;
             }
-            const unsigned found = __ballot_sync(kFull, room != 0);
-            int p = 0;
-            if (lane == 0 && found) p = atomicAdd(&s_found, __popc(found));
-            p = __shfl_sync(kFull, p, 0) + __popc(found & ((1u << lane) - 1u));
-            if (room) {
-                s_key[p] = ld_stream(keys + base + uint64_t(i));
-                s_begin[p] = begin;
-                s_room[p] = room;
+            /* ends within the tile; the loads of all rows before any store */
+            constexpr int kPer = kMultiTile / kMultiThreads;
+            unsigned long long begin[kPer], end[kPer];
+            const unsigned long long part_end = a.end_out[base + uint64_t(m - 1)];
+#pragma unroll
+            for (int j = 0; j < kPer; ++j) {
+                const int i = int(threadIdx.x) + j * kMultiThreads;
+                end[j] = i < m ? a.end_out[base + uint64_t(i)] : 0ull;
+                begin[j] = i > 0 && i < m ? a.end_out[base + uint64_t(i) - 1] : part_begin;
             }
-        }
-        __syncthreads();
-        const int n = s_found;
-        bool has = false, left = n > 0;
-        int at = 0;
-        K key = 0;
-        V *out = nullptr;
-        uint64_t room = 0;
-        typename Walk::State s;
-        while (left || __any_sync(kFull, has)) {
-            if (draw_key(has, n, &s_drawn, left, at)) {
-                key = s_key[at];
-                out = reinterpret_cast<V *>(a.values_out) + s_begin[at];
-                room = s_room[at];
-                has = true;
-                Walk::start(a, key, s);
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < kPer; ++j) {
+                const int i = int(threadIdx.x) + j * kMultiThreads;
+                const unsigned long long room = i < m ? end[j] - begin[j] : 0ull;
+                if (i < m) {
+                    a.end_out[base + uint64_t(i)] = before + end[j];
+                    if (a.begin_out) a.begin_out[base + uint64_t(i)] = before + begin[j];
+                }
+                const unsigned found = __ballot_sync(kFull, room != 0);
+                int p = 0;
+                if (lane == 0 && found) p = atomicAdd(&s_found, __popc(found));
+                p = __shfl_sync(kFull, p, 0) + __popc(found & ((1u << lane) - 1u));
+                if (room) {
+                    s_key[p] = ld_stream(keys + base + uint64_t(i));
+                    s_begin[p] = before + begin[j];
+                    s_room[p] = room;
+                }
             }
-            if (has && Walk::value_step(a, key, s, out, room)) has = false;
+            part_begin = part_end;
+            __syncthreads();
+            const int n = s_found;
+            bool has = false, left = n > 0;
+            int at = 0;
+            K key = 0;
+            V *out = nullptr;
+            uint64_t room = 0;
+            typename Walk::State s;
+            while (left || __any_sync(kFull, has)) {
+                if (draw_key(has, n, &s_drawn, left, at)) {
+                    key = s_key[at];
+                    out = reinterpret_cast<V *>(a.values_out) + s_begin[at];
+                    room = s_room[at];
+                    has = true;
+                    Walk::start(a, key, s);
+                }
+                if (has && Walk::value_step(a, key, s, out, room)) has = false;
+            }
+            __syncthreads(); /* the shared rows are rewritten by the next part */
         }
-        __syncthreads(); /* the shared rows are rewritten by the next tile */
     }
 }
 

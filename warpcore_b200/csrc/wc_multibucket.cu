@@ -29,7 +29,7 @@ struct wc_mbht {
     void *vals = nullptr;
     uint32_t *status = nullptr;           /* device Status word */
     unsigned long long *counters = nullptr; /* device: num_keys, num_occupied, scratch */
-    void *scan = nullptr;                 /* look-back words, grown on demand */
+    void *scan = nullptr;                 /* tiles of a retrieve, grown on demand */
     uint64_t scan_bytes = 0;
     bool initialized = false;
 };
