@@ -816,6 +816,10 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_insert_kernel(const 
                 finish(kStDuplicateKey);
                 continue;
             }
+            /* a fingerprint seen before the key it was written after: the
+             * slot's claim decides */
+            if (slot_key<L>(sw, 0) == empty)
+                free |= 1u << FpWords<W>::slot_of(__ffs(cand) - 1);
             cand &= cand - 1u;
             advance = cand == 0 && free == 0;
         } else if (claiming) {
