@@ -686,18 +686,45 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS_READ) fp_find_kernel(con
 /* Insert on tables with fingerprints, in the form of fp_find_kernel: the
  * lanes' fingerprint loads, slot reads and claims are in flight together.
  * Claims take the lowest slot with an empty fingerprint first, as in
- * fp_op_kernel; equal keys in one wave meet on that slot, so they need no
- * merging.  Against fp_op_kernel, which ran the
+ * fp_op_kernel.  Against fp_op_kernel, which ran the
  * three steps one after the other: u64 set of 134 MB at load 0.9, 15 M keys
  * 727 -> 597 us; u64 pairs of 161 MB, 9 M 491 -> 444; u32 pairs of 269 MB, 30 M
- * 1612 -> 1423; 65 536 updates of 575 MB of u64 pairs 41 -> 33. */
+ * 1612 -> 1423; 65 536 updates of 575 MB of u64 pairs 41 -> 33.
+ *
+ * Equal keys that meet in one refill are merged, with the value of the last:
+ * a call of at most 32 keys stores each key's last value, and a frequent key
+ * sends one claim or store per refill instead of up to 32 that queue at one
+ * address.  A warp that found no equal keys in kMergeQuiet refills in a row
+ * looks through one refill of eight, so distinct keys pay little: 4 M
+ * keys, without / with merging, u64 set 176 / 184 us, u32 pairs 224 / 225, u64
+ * pairs 215 / 201; one key 4 M times 2 645 / 117, 2 617 / 565, 4 110 / 566;
+ * Zipf(1.4) 780 / 216, 3 346 / 2 146, 3 528 / 2 095.
+ *
+ * In tables with values the merged lanes wait for the lane that has their key
+ * (kHold), unless they are most of a refill.  Their places would be filled
+ * with one or two keys at a time, and a frequent key that comes in more
+ * and smaller refills reads and writes its slot's line more often: 4 M
+ * Zipf(1.1) updates of u64 pairs 10.2 ms without waiting, 6.8 with it (and
+ * without merging); keys in runs of 16 125 us with waiting always, 87 so.
+ * Sets, which write nothing for a key that is there, gain nothing by it. */
+constexpr uint32_t kMergeQuiet = 4;
+
+/* one more block than the other kernels where 48 registers do: 4 M u32 pairs
+ * 238 -> 225 us, u64 set 204 -> 184 */
+template <class L>
+constexpr int fp_insert_min_blocks()
+{
+    return L::kSlotBytes <= 8 ? WC_FP_MIN_BLOCKS + 1 : WC_FP_MIN_BLOCKS;
+}
+
 template <class L, int W>
-__global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_insert_kernel(const TableOpArgs a)
+__global__ void __launch_bounds__(256, fp_insert_min_blocks<L>()) fp_insert_kernel(const TableOpArgs a)
 {
     using K = typename L::key_t;
     using V = typename L::val_t;
     constexpr int SB = L::kSlotBytes;
     constexpr bool kValueIn = L::kHasValue;
+    constexpr bool kHold = kValueIn;
     const uint64_t pol_keep = l2_policy_evict_last(); /* fingerprint lines */
 
     const TableView &t = a.t;
@@ -731,6 +758,10 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_insert_kernel(const 
      * fingerprints are due */
     bool has = false;
     uint32_t cand = 0, free = 0, at = 0;
+    uint32_t quiet = 0; /* refills since the last one with equal keys */
+    /* waits: lane `first` inserts this lane's key too; held: some lane waits */
+    bool waits = false, held = false;
+    int first = 0;
     uint64_t bucket = 0, step = 0, wins = 0;
     K key = empty;
     V val = 0, expect = 0;
@@ -750,6 +781,12 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_insert_kernel(const 
     };
 
     for (;;) {
+        /* ---- lanes whose key another lane inserts wait for it ---- */
+        if (kHold && held) {
+            const unsigned done = __ballot_sync(kFull, !has);
+            if (waits && ((done >> first) & 1u)) has = waits = false;
+            held = __any_sync(kFull, waits);
+        }
         /* ---- refill lanes whose key is done, in input order ---- */
         const unsigned need = __ballot_sync(kFull, !has);
         const uint32_t idle = uint32_t(__popc(need)), avail = m - cursor;
@@ -758,6 +795,7 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_insert_kernel(const 
         if (take) {
             const uint32_t r = uint32_t(__popc(need & lanemask_lt));
             const uint32_t off = cursor - pf_base + r; /* < 64 for refilling lanes */
+            bool fresh = false;
             const K ka = shfl_any(pfA, int(off & 31u));
             const K kb = shfl_any(pfB, int(off & 31u));
             V va = 0, vb = 0;
@@ -774,9 +812,27 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_insert_kernel(const 
                 free = 0;
                 wins = 0;
                 step = 0;
-                if (key == empty || key == tomb) finish(kStInvalidKey);
-                else bucket = probe_begin<K>(t, key);
+                fresh = key != empty && key != tomb;
+                if (!fresh) finish(kStInvalidKey);
             }
+            bool merged = false;
+            if (quiet < kMergeQuiet || (quiet & 7u) == 0) {
+                const unsigned peers = merge_equal_keys<K, V, kValueIn>(fresh, key, empty, val);
+                merged = fresh && (peers & lanemask_lt);
+                const uint32_t gone = uint32_t(__popc(__ballot_sync(kFull, merged)));
+                if (gone) quiet = 0;
+                if constexpr (kHold) {
+                    if (merged && gone * 4 <= take * 3) {
+                        waits = true;
+                        first = __ffs(peers) - 1;
+                    }
+                    held |= gone != 0;
+                }
+            }
+            ++quiet;
+            if (merged) finish(kStDuplicateKey);
+            else if (fresh) bucket = probe_begin<K>(t, key);
+            if constexpr (kHold) has |= waits;
             cursor += take;
             if (cursor - pf_base >= 32) {
                 pf_base += 32;
@@ -800,14 +856,14 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_insert_kernel(const 
                                 : base_slot + uint64_t(free ? __ffs(free) - 1 : 0);
         unsigned char *const sp = slots + s * SB;
         const bool checking = cand != 0, claiming = !checking && free != 0;
-        if (has) {
+        if (has && !waits) {
             /* slots are read where the claims' atomics land (L2): an L1 copy
              * may predate the claim of an equal key by another lane */
             if (checking) sw = load_lane<SB>(sp);
             else if (claiming) old = cas_slot<L>(sp, empty, expect, key, val, &old_payload);
             else f.load(t.fps + base_slot, pol_keep);
         }
-        if (!has) continue;
+        if (!has || waits) continue;
 
         bool advance = false;
         if (checking) {

@@ -487,6 +487,22 @@ __device__ __forceinline__ void group_range(const TableOpArgs &a, const uint64_t
     }
 }
 
+/* Equal keys among those the lanes of a warp have just taken, in input order
+ * by lane (`fresh`: lanes with a valid new key): returns the lanes that have
+ * this lane's key.  The value of the last of them replaces every one's.
+ * Whole warps call it. */
+template <class K, class V, bool kValue>
+__device__ __forceinline__ unsigned merge_equal_keys(bool fresh, K key, K empty, V &val)
+{
+    const unsigned peers = __match_any_sync(kFull, fresh ? key : empty) &
+                           __ballot_sync(kFull, fresh);
+    if constexpr (kValue) {
+        const V last = shfl_any(val, fresh ? 31 - __clz(peers) : 0);
+        if (fresh) val = last;
+    }
+    return peers;
+}
+
 template <class L, int W, int OP>
 __global__ void __launch_bounds__(256, WC_TABLE_MIN_BLOCKS) table_op_kernel(const TableOpArgs a)
 {
