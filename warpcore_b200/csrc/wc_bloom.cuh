@@ -63,10 +63,6 @@ __device__ __forceinline__ T atomic_or_any(T *p, T v)
         return T(atomicOr(reinterpret_cast<unsigned int *>(p), (unsigned int)v));
 }
 
-#ifndef WC_BLOOM_INSERT_READS_BLOCK
-#define WC_BLOOM_INSERT_READS_BLOCK 1
-#endif
-
 /* bit masks of the CG words of key's block, computed once by the lane that
  * owns the key */
 template <class K, class S, int CG>
@@ -104,8 +100,8 @@ __device__ __forceinline__ void block_masks(K key, K seed, uint32_t hasher, uint
  * this thread's row in shared memory (cp.reduce.async.bulk), for blocks of
  * 16 to 128 bytes.  Inserts are bound by their ORs at L2: one per word that
  * misses bits, 4.3 per key with 8 bits in 64 bytes, after a read of the
- * block to find those words.  A bulk reduction needs no read and is one
- * request per key.  2^28 keys into the 2^32-bit filter of 64-byte blocks:
+ * block to find those words.  A bulk reduction needs no read (see LookFirst)
+ * and is one request per key.  2^28 keys into the 2^32-bit filter of 64-byte blocks:
  * 13.17 -> 12.12 ms; 6 M keys into a 16 MiB filter of 32-byte blocks, which
  * stays in L2: 191 -> 174 us.  Sending a quarter or half of the warps'
  * masks this way and the others as word ORs measured 15.2 / 13.9 ms and
@@ -118,10 +114,10 @@ struct BulkOr {
      * lanes' 16-byte stores over all banks */
     static constexpr int kRow = BB > 16 ? BB + 16 : 16;
 
-    static __device__ __forceinline__ void reduce(S *block, unsigned char *row, const S (&m)[CG])
+    /* the mask into this thread's row, once the row's last reduction has
+     * been read */
+    static __device__ __forceinline__ void put(unsigned char *row, const S (&m)[CG])
     {
-        const uint32_t sa = uint32_t(__cvta_generic_to_shared(row));
-        /* the row's last reduction has been read */
         asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         constexpr int WPV = 16 / int(sizeof(S));
 #pragma unroll
@@ -130,6 +126,27 @@ struct BulkOr {
             memcpy(&q, &m[v * WPV], 16);
             *reinterpret_cast<uint4 *>(row + 16 * v) = q;
         }
+    }
+    /* whether the block misses bits of the row's mask.  (The mask is read
+     * back, so that it and the block are never both in registers.) */
+    static __device__ __forceinline__ bool misses(const S *block, const unsigned char *row)
+    {
+        uint32_t w[BB / 4], miss = 0;
+        load_window<BB>(reinterpret_cast<const unsigned char *>(block), w);
+#pragma unroll
+        for (int v = 0; v < BB / 16; ++v) {
+            uint32_t q[4];
+            asm volatile("ld.volatile.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3])
+                         : "r"(uint32_t(__cvta_generic_to_shared(row)) + 16u * v) : "memory");
+#pragma unroll
+            for (int i = 0; i < 4; ++i) miss |= q[i] & ~w[4 * v + i];
+        }
+        return miss != 0;
+    }
+    static __device__ __forceinline__ void send(S *block, unsigned char *row)
+    {
+        const uint32_t sa = uint32_t(__cvta_generic_to_shared(row));
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.or.b64 [%0], [%1], %2;"
                      :: "l"(block), "r"(sa), "r"(BB) : "memory");
@@ -197,6 +214,87 @@ __device__ __forceinline__ bool block_has_all(K key, K seed, uint32_t hasher, ui
     return ok & 1u;
 }
 
+/* When a warp's inserts read a block before its bulk OR, so that a key whose
+ * bits are all set sends nothing.  ORs of one block queue at its place in
+ * L2, about 1 ns each, so a stream of repeated keys needs the read; for
+ * distinct keys it is a second access for nothing.  A warp looks at its first
+ * kSample keys, goes on looking while at least one of kFew looked at was there,
+ * and else looks again after kSkip rounds.  2^32-bit filter of 64-byte
+ * blocks, never / always / this: 2^28 distinct keys 12.13 / 12.82 / 12.31 ms,
+ * inserted again 12.13 / 9.31 / 9.88, 2^27 Zipf(0.8) keys 10.0 / 5.3 / 5.4,
+ * Zipf(1.1) 32.2 / 5.0 / 5.1, 2^24 times one key 17.2 / 0.53 / 0.48; 6 M keys into a
+ * 16 MiB filter of 32-byte blocks: 171 / 197 / 179 us, 169 / 116 / 120, 171 / 155 /
+ * 155, 478 / 186 / 152, 3 077 / 271 / 170.  Few keys sampled per look would not do:
+ * regions hold some 16 keys of a tile, and with "two present in the last
+ * round" Zipf(1.1) took 14.6 ms. */
+struct LookFirst {
+    static constexpr uint32_t kSample = 64, kFew = 32, kSkip = 15;
+    uint32_t keys = 0, there = 0, skip = 0;
+
+    __device__ __forceinline__ bool now() const { return skip == 0; }
+    /* ends a round: lanes with a key, and (looked at) with one that was there */
+    __device__ __forceinline__ void next(bool in, bool present)
+    {
+        if (skip) {
+            --skip;
+            return;
+        }
+        keys += uint32_t(__popc(__ballot_sync(kFull, in)));
+        there += uint32_t(__popc(__ballot_sync(kFull, present)));
+        if (keys >= kSample && there * kFew < keys) skip = kSkip;
+        if (keys >= 4 * kSample) {
+            keys /= 2;
+            there /= 2;
+        }
+    }
+};
+
+constexpr uint64_t kNoBlock = ~0ull;
+
+/* ORs one key per lane into the block that starts at word `first` (kNoBlock:
+ * no key).  Whole warps call it. */
+template <class K, class S, int CG, bool kBulk>
+__device__ __forceinline__ void bloom_or(const BloomArgs &a, K key, uint64_t first,
+                                         unsigned char *row, LookFirst &look)
+{
+    S *const words = reinterpret_cast<S *>(a.words);
+    const bool whole = first != kNoBlock && first + CG <= a.num_slots;
+    const bool read = !kBulk || look.now();
+    bool there = false;
+    if (first != kNoBlock) {
+        S w[CG];
+        if constexpr (!kBulk) {
+            if (whole) {
+                load_block<S, CG>(words + first, w);
+            } else {
+                /* ragged last block: words wrap to the front */
+#pragma unroll
+                for (int s = 0; s < CG; ++s) w[s] = __ldcg(words + (first + s) % a.num_slots);
+            }
+        }
+        S m[CG];
+        block_masks<K, S, CG>(key, K(a.seed), a.hasher, a.k, m);
+        if (kBulk && whole) {
+            if constexpr (kBulk) {
+                using Bulk = BulkOr<S, CG>;
+                Bulk::put(row, m);
+                there = read && !Bulk::misses(words + first, row);
+                if (!there) Bulk::send(words + first, row);
+            }
+        } else {
+#pragma unroll
+            for (int s = 0; s < CG; ++s) {
+                if (kBulk ? m[s] != 0 : (w[s] & m[s]) != m[s]) {
+                    uint64_t wi = first + uint64_t(s);
+                    if (wi >= a.num_slots) wi -= a.num_slots;
+                    atomic_or_any(words + wi, m[s]);
+                }
+            }
+        }
+    }
+    if constexpr (kBulk) look.next(first != kNoBlock, there);
+}
+
 template <class K, class S, int CG, bool INSERT>
 __global__ void __launch_bounds__(256) bloom_kernel(const BloomArgs a)
 {
@@ -231,7 +329,6 @@ __global__ void __launch_bounds__(256) bloom_kernel(const BloomArgs a)
         S own_mask[kOwnerMasks ? CG : 1];
         if constexpr (kOwnerMasks) block_masks<K, S, CG>(key, seed, a.hasher, a.k, own_mask);
 
-        constexpr bool kRead = !INSERT || WC_BLOOM_INSERT_READS_BLOCK;
         LaneWords win[TPK];
 #pragma unroll
         for (int r = 0; r < TPK; ++r) {
@@ -239,7 +336,7 @@ __global__ void __launch_bounds__(256) bloom_kernel(const BloomArgs a)
             const uint64_t b = shfl_any(blk, o);
             const uint64_t w0 = b * CG + uint64_t(q) * SPL;
             win[r] = LaneWords{{0u, 0u, 0u, 0u}};
-            if (kRead && (base + o) < a.n) {
+            if ((base + o) < a.n) {
                 if (b * CG + CG <= a.num_slots) {
                     win[r] = load_lane<LB>(words + w0);
                 } else {
@@ -287,7 +384,7 @@ __global__ void __launch_bounds__(256) bloom_kernel(const BloomArgs a)
                 const S w = lane_word<S>(win[r], s);
                 const bool missing = (w & mask[s]) != mask[s];
                 ok &= !missing;
-                if (INSERT && own_ok && mask[s] && (!kRead || missing)) {
+                if (INSERT && own_ok && missing) {
                     uint64_t wi = b * CG + uint64_t(q) * SPL + s;
                     if (wi >= a.num_slots) wi -= a.num_slots; /* ragged last block */
                     atomic_or_any(words + wi, mask[s]);
@@ -310,8 +407,9 @@ __global__ void __launch_bounds__(256) bloom_kernel(const BloomArgs a)
 
 /* One key per lane, for blocks of at most 128 bytes: the lane computes its
  * key's masks, reads its own block with 32-byte vector loads and tests it.
- * An insert of blocks of 16 bytes or more ORs the masks without a read
- * (BulkOr), of smaller ones only the words that miss bits.  Against the
+ * An insert of blocks of 16 bytes or more ORs the whole mask (BulkOr) and
+ * reads the block only where keys repeat (LookFirst); of smaller ones it ORs
+ * only the words that miss bits.  Against the
  * cooperative kernel above it spends no shuffles on block indices and masks.
  * It serves the keys whose block lies in [region_lo, region_hi) (one pass:
  * the whole filter).
@@ -333,8 +431,6 @@ __global__ void __launch_bounds__(256) bloom_lane_kernel(const BloomArgs a)
     static_assert(CG * sizeof(S) <= 128, "block of one lane");
     using Bulk = BulkOr<S, CG>;
     constexpr bool kBulk = INSERT && Bulk::kUsed;
-    constexpr bool kRead = (!INSERT || WC_BLOOM_INSERT_READS_BLOCK) && !kBulk;
-    constexpr uint64_t kNone = ~0ull;
 
     S *const words = reinterpret_cast<S *>(a.words);
     const K *const keys = reinterpret_cast<const K *>(a.keys);
@@ -342,11 +438,12 @@ __global__ void __launch_bounds__(256) bloom_lane_kernel(const BloomArgs a)
     __shared__ alignas(16) unsigned char s_rows[kBulk ? 256 * Bulk::kRow : 16];
     __shared__ uint32_t s_words[INSERT ? 1 : CG * sizeof(S) / 4 * 256];
     const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-    for (uint64_t i0 = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i0 < a.n;
-         i0 += stride * U) {
+    LookFirst look;
+    /* (whole warps stay in the loop) */
+    for (uint64_t i0 = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+         i0 - (threadIdx.x & 31) < a.n; i0 += stride * U) {
         K key[U];
-        uint64_t w0[U]; /* first word of the key's block, kNone: not served */
-        S w[U][CG];
+        uint64_t w0[U]; /* first word of the key's block, kNoBlock: not served */
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const uint64_t i = i0 + uint64_t(u) * stride;
@@ -358,13 +455,21 @@ __global__ void __launch_bounds__(256) bloom_lane_kernel(const BloomArgs a)
             const uint64_t blk = mod_hash<K>(hash_key<K>(a.hasher, K(key[u] + seed)),
                                              a.num_blocks, a.magic_blocks) - a.block_base;
             w0[u] = i < a.n && blk < a.local_blocks && blk >= a.region_lo && blk < a.region_hi
-                        ? blk * CG : kNone;
+                        ? blk * CG : kNoBlock;
             if constexpr (!INSERT) {
                 if (i < a.n && blk >= a.local_blocks && a.region_lo == 0) a.flags_out[i] = 0;
             }
+        }
+        if constexpr (INSERT) {
 #pragma unroll
-            for (int s = 0; s < CG; ++s) w[u][s] = 0;
-            if (kRead && w0[u] != kNone) {
+            for (int u = 0; u < U; ++u)
+                bloom_or<K, S, CG, kBulk>(a, key[u], w0[u],
+                                          s_rows + (kBulk ? threadIdx.x * Bulk::kRow : 0), look);
+        } else {
+            S w[U][CG];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (w0[u] == kNoBlock) continue;
                 if (w0[u] + CG <= a.num_slots) {
                     load_block<S, CG>(words + w0[u], w[u]);
                 } else {
@@ -374,33 +479,12 @@ __global__ void __launch_bounds__(256) bloom_lane_kernel(const BloomArgs a)
                         w[u][s] = __ldcg(words + (w0[u] + s) % a.num_slots);
                 }
             }
-        }
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (w0[u] == kNone) continue;
-            if constexpr (!INSERT) {
-                a.flags_out[i0 + uint64_t(u) * stride] =
-                    (unsigned char)block_has_all<K, S, CG>(key[u], seed, a.hasher, a.k, w[u],
-                                                           s_words + threadIdx.x);
-            } else {
-                S m[CG];
-                block_masks<K, S, CG>(key[u], seed, a.hasher, a.k, m);
-                if constexpr (kBulk) {
-                    if (w0[u] + CG <= a.num_slots) {
-                        Bulk::reduce(words + w0[u], s_rows + threadIdx.x * Bulk::kRow, m);
-                        continue;
-                    }
-                }
-#pragma unroll
-                for (int s = 0; s < CG; ++s) {
-                    const bool missing = (w[u][s] & m[s]) != m[s];
-                    if (m[s] && (!kRead || missing)) {
-                        uint64_t wi = w0[u] + uint64_t(s);
-                        if (wi >= a.num_slots) wi -= a.num_slots;
-                        atomic_or_any(words + wi, m[s]);
-                    }
-                }
-            }
+            for (int u = 0; u < U; ++u)
+                if (w0[u] != kNoBlock)
+                    a.flags_out[i0 + uint64_t(u) * stride] =
+                        (unsigned char)block_has_all<K, S, CG>(key[u], seed, a.hasher, a.k, w[u],
+                                                               s_words + threadIdx.x);
         }
     }
     if constexpr (kBulk) Bulk::finish();
@@ -420,9 +504,8 @@ __global__ void __launch_bounds__(256) bloom_lane_kernel(const BloomArgs a)
  * region_kpl x 32 keys (region_kpl coalesced loads per lane in flight),
  * computes their blocks, and compacts the keys of its region into a list
  * in shared memory (ballot + prefix count, input order kept).  The lanes
- * then take the list densely, kRegionU entries per lane at a time, issue
- * all their block reads before testing any, and write flags / OR words as
- * the one-key-per-lane kernel does.  One entry per lane with four resident
+ * then take the list densely, one entry per lane at a time, and write flags /
+ * OR words as the one-key-per-lane kernel does.  One entry per lane with four resident
  * blocks per SM (64-byte blocks; two for 128-byte blocks, whose words take
  * twice the registers) keeps more warps issuing than four entries per lane
  * with two blocks: on the 2^32-bit filter of 64-byte blocks, 2^28 keys,
@@ -435,7 +518,6 @@ __global__ void __launch_bounds__(256) bloom_lane_kernel(const BloomArgs a)
 /* keys per lane per warp tile (the rows of 128-byte blocks leave shared
  * memory for half as many) */
 constexpr int region_kpl(int block_bytes) { return block_bytes <= 64 ? 8 : 4; }
-constexpr int kRegionU = 1;     /* compacted keys per lane in flight */
 constexpr int kRegionWarps = 8; /* 256 threads */
 
 template <class K, class S, int CG, bool INSERT>
@@ -447,7 +529,6 @@ __global__ void __launch_bounds__(256, CG * sizeof(S) <= 64 ? 4 : 2) bloom_regio
     constexpr int WT = 32 * kRegionKpl; /* keys per warp tile */
     static_assert(BB <= 128, "block of one lane");
     static_assert(WT <= 256, "tile offsets are one byte");
-    constexpr bool kRead = !INSERT || WC_BLOOM_INSERT_READS_BLOCK;
 
     __shared__ K s_key[kRegionWarps][WT];
     __shared__ uint32_t s_rel[kRegionWarps][WT];       /* block - region_lo */
@@ -466,6 +547,7 @@ __global__ void __launch_bounds__(256, CG * sizeof(S) <= 64 ? 4 : 2) bloom_regio
     const uint64_t gwarp = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
 
+    LookFirst look;
     for (uint64_t base = gwarp * WT; base < a.n; base += nwarps * WT) {
         K kk[kRegionKpl];
 #pragma unroll
@@ -495,53 +577,24 @@ __global__ void __launch_bounds__(256, CG * sizeof(S) <= 64 ? 4 : 2) bloom_regio
             cnt += __popc(m);
         }
         __syncwarp();
-        for (int e0 = 0; e0 < cnt; e0 += 32 * kRegionU) {
-            S w[kRegionU][CG];
-#pragma unroll
-            for (int u = 0; u < kRegionU; ++u) {
-                const int e = e0 + u * 32 + lane;
-                if (kRead && !kBulk && e < cnt) {
-                    const uint64_t w0 = (a.region_lo + s_rel[wib][e]) * CG;
-                    if (w0 + CG <= a.num_slots) {
-                        load_block<S, CG>(words + w0, w[u]);
-                    } else {
-#pragma unroll
-                        for (int s = 0; s < CG; ++s) w[u][s] = __ldcg(words + (w0 + s) % a.num_slots);
-                    }
+        for (int e0 = 0; e0 < cnt; e0 += 32) {
+            const int e = e0 + lane;
+            const K key = e < cnt ? s_key[wib][e] : K(0);
+            const uint64_t w0 = e < cnt ? (a.region_lo + s_rel[wib][e]) * CG : kNoBlock;
+            if constexpr (INSERT) {
+                bloom_or<K, S, CG, kBulk>(a, key, w0,
+                                          s_rows + (kBulk ? threadIdx.x * Bulk::kRow : 0), look);
+            } else if (e < cnt) {
+                S w[CG];
+                if (w0 + CG <= a.num_slots) {
+                    load_block<S, CG>(words + w0, w);
                 } else {
 #pragma unroll
-                    for (int s = 0; s < CG; ++s) w[u][s] = 0;
+                    for (int s = 0; s < CG; ++s) w[s] = __ldcg(words + (w0 + s) % a.num_slots);
                 }
-            }
-#pragma unroll
-            for (int u = 0; u < kRegionU; ++u) {
-                const int e = e0 + u * 32 + lane;
-                if (e >= cnt) continue;
-                const K key = s_key[wib][e];
-                const uint64_t w0 = (a.region_lo + s_rel[wib][e]) * CG;
-                if constexpr (!INSERT) {
-                    a.flags_out[base + s_off[wib][e]] =
-                        (unsigned char)block_has_all<K, S, CG>(key, seed, a.hasher, a.k, w[u],
-                                                               s_words + threadIdx.x);
-                } else {
-                    S m[CG];
-                    block_masks<K, S, CG>(key, seed, a.hasher, a.k, m);
-                    if constexpr (kBulk) {
-                        if (w0 + CG <= a.num_slots) {
-                            Bulk::reduce(words + w0, s_rows + threadIdx.x * Bulk::kRow, m);
-                            continue;
-                        }
-                    }
-#pragma unroll
-                    for (int s = 0; s < CG; ++s) {
-                        const bool missing = (w[u][s] & m[s]) != m[s];
-                        if (m[s] && (!kRead || missing)) {
-                            uint64_t wi = w0 + uint64_t(s);
-                            if (wi >= a.num_slots) wi -= a.num_slots;
-                            atomic_or_any(words + wi, m[s]);
-                        }
-                    }
-                }
+                a.flags_out[base + s_off[wib][e]] =
+                    (unsigned char)block_has_all<K, S, CG>(key, seed, a.hasher, a.k, w,
+                                                           s_words + threadIdx.x);
             }
         }
         __syncwarp();
