@@ -16,11 +16,15 @@
  *     needed for the wrap check only, is looked at one step later.
  *   - The cached keys take the same way when the input is used up.
  * A warp whose first kCountSample keys hit the cache in less than one of
- * kCountMinHits stops using it: in a stream of nearly distinct keys the
- * cache only delays them.
+ * kCountMinHits leaves it out for a while: in a stream of nearly distinct
+ * keys the cache only delays them.  Keys left for the queue are merged with
+ * equal ones of the same 32, so that a stream in runs, or one whose frequent
+ * keys found the cache full, sends one add for each.  (A warp that found no
+ * equal keys four times looks at one 32 of eight.)  2^26 u32 keys in runs of
+ * four 2 030 -> 955 us, 2^26 sorted Zipf(1.1) u64 keys 1 670 -> 987.
  *
  * Measured against table_op_kernel and its caches of 32 KiB per block, which
- * merged equal keys with __match_any_sync, probed the table in the same
+ * merged all equal keys with __match_any_sync, probed the table in the same
  * loop and counted the cached keys slot by slot at the end: u32 pairs, 2^27
  * Zipf(1.1) keys over 2^23 (84 MB) 2496 -> 1252 us (107 G keys/s); 2^25
  * Zipf(1.1) over 2^20 679 -> 330; u64 keys, 3 M Zipf(0.5) over 1 M 199 ->
@@ -41,12 +45,82 @@ namespace b200 {
 constexpr int kCountThreads = 1024; /* one block per SM, at most 64 registers */
 constexpr int kCountWarps = kCountThreads / 32;
 constexpr int kCountQueue = 64;     /* keys a warp's queue holds */
-/* when a warp leaves the cache out.  Even few early hits pay later, when the
+/* When a warp leaves the cache out: fewer than one of kCountMinHits of the
+ * first kCountSample keys hit it.  Even few early hits pay later, when the
  * cache holds the frequent keys: Zipf(0.8), 2^25 u32 keys over 2^22, ran
  * 1757 / 792 / 703 / 692 us with one hit of 6 / 16 / 32 / 64 of the first 128
- * keys, 666 with one of 64 of the first 256. */
-constexpr uint32_t kCountSample = 256;
+ * keys.  A stream may begin with rare keys, so the warp tries the cache again
+ * for kCountResample keys after every kCountAgain: where each warp's first 300
+ * keys were distinct and the others 16 hot ones, 2^24 u32 keys took 2 440 us
+ * without that and 357 with it, u64 keys 3 430 and 590. */
+constexpr uint32_t kCountSample = 128;
 constexpr uint32_t kCountMinHits = 64;
+constexpr uint32_t kCountAgain = 512, kCountResample = 64;
+
+/* What a warp remembers from one 32 keys to the next: keys of the present
+ * sample and its hits, for how many times 32 keys the cache is still left out,
+ * and times since equal keys were found.  In one register where keys take 8
+ * bytes, whose kernels have none left (2^24 Zipf(0.5) keys over 2^20: 455 us
+ * with each in its own, 438 so); for 4-byte keys that costs more than it saves
+ * (2^26 Zipf(1.4) keys over 2^24 406 and 417). */
+template <bool kPacked>
+struct CountWarp;
+
+template <>
+struct CountWarp<false> {
+    uint32_t seen = 0, hits = 0, off = 0, quiet = 0;
+    bool on = true;
+
+    __device__ __forceinline__ bool cache() const { return on; }
+    __device__ __forceinline__ bool sampling() const { return seen < kCountSample; }
+    /* 32 more keys of the sample, `more` of them hits */
+    __device__ __forceinline__ void sampled(uint32_t more)
+    {
+        seen += 32;
+        hits += more;
+        if (seen >= kCountSample && hits * kCountMinHits < seen) {
+            on = false;
+            off = kCountAgain / 32;
+        }
+    }
+    __device__ __forceinline__ void left_out()
+    {
+        if (--off == 0) {
+            on = true;
+            seen = kCountSample - kCountResample;
+            hits = 0;
+        }
+    }
+    __device__ __forceinline__ bool look_for_equal() const { return quiet < 4 || (quiet & 7) == 0; }
+    __device__ __forceinline__ void equal(bool found) { quiet = found ? 1 : quiet + 1; }
+};
+
+template <>
+struct CountWarp<true> {
+    /* bits 0 to 3 seen / 32, 4 to 13 hits, 14 to 21 off, 22 on quiet (4 to 15,
+     * going back to 8) */
+    uint32_t bits = 0;
+
+    __device__ __forceinline__ bool cache() const { return (bits >> 14 & 0xffu) == 0; }
+    __device__ __forceinline__ bool sampling() const { return (bits & 0xfu) < kCountSample / 32; }
+    __device__ __forceinline__ void sampled(uint32_t more)
+    {
+        bits += 1u + (more << 4);
+        if (!sampling() && (bits >> 4 & 0x3ffu) * kCountMinHits < kCountSample)
+            bits = (bits & ~0x3fffffu) | (kCountSample - kCountResample) / 32 |
+                   (kCountAgain / 32) << 14;
+    }
+    __device__ __forceinline__ void left_out() { bits -= 1u << 14; }
+    __device__ __forceinline__ bool look_for_equal() const
+    {
+        return bits >> 22 < 4 || bits >> 22 == 8;
+    }
+    __device__ __forceinline__ void equal(bool found)
+    {
+        if (found) bits &= 0x3fffffu;
+        bits += bits >> 22 == 15 ? uint32_t(-7) << 22 : 1u << 22;
+    }
+};
 
 struct CountArgs {
     TableView t;
@@ -250,8 +324,7 @@ __global__ void __launch_bounds__(kCountThreads, 1) count_insert_kernel(const Co
         uint64_t at = 0;
         K pfA = uint64_t(lane) < m ? ld_stream(keys + lane) : empty;
         K pfB = 32 + uint64_t(lane) < m ? ld_stream(keys + 32 + lane) : empty;
-        uint32_t seen = 0, hits = 0;
-        bool cache = true;
+        CountWarp<sizeof(K) == 8> mem;
         probe([&]() {
             if (at >= m) return false;
             const K key = pfA;
@@ -264,7 +337,7 @@ __global__ void __launch_bounds__(kCountThreads, 1) count_insert_kernel(const Co
                 join |= kStInvalidKey;
                 in = false;
             }
-            if (cache) {
+            if (mem.cache()) {
                 bool known = false;
                 if (in) {
                     const uint32_t set =
@@ -295,13 +368,23 @@ __global__ void __launch_bounds__(kCountThreads, 1) count_insert_kernel(const Co
                     }
                     if (known) join |= kStDuplicateKey;
                 }
-                if (seen < kCountSample) {
-                    seen += 32;
-                    hits += uint32_t(__popc(__ballot_sync(kFull, known)));
-                    if (seen >= kCountSample && hits * kCountMinHits < seen) cache = false;
-                }
+                if (mem.sampling()) mem.sampled(uint32_t(__popc(__ballot_sync(kFull, known))));
+            } else {
+                mem.left_out();
             }
-            enqueue(in, key, 1u);
+            /* equal keys among those left for the table */
+            uint32_t c = 1;
+            bool equal = false;
+            if (mem.look_for_equal()) {
+                const unsigned peers = __match_any_sync(kFull, in ? key : empty) &
+                                       __ballot_sync(kFull, in);
+                const bool merged = in && (peers & lanemask_lt);
+                equal = __any_sync(kFull, merged);
+                c = uint32_t(__popc(peers));
+                in &= !merged;
+            }
+            mem.equal(equal);
+            enqueue(in, key, c);
             return at < m;
         });
     }
