@@ -598,11 +598,13 @@ int wc_fingerprint_policy(int mode, int *previous);
  * default. */
 int wc_fingerprint_ops(uint32_t op_mask, uint32_t *previous);
 /* Which operations may probe whole windows with one key per lane (each
- * lane reads its key's window with 32-byte loads; bit 0 insert, 2 retrieve,
- * 3 erase, default all three) instead of with groups of lanes per window
- * and ballots.  Applies to tables whose slot array fits in L2 and whose
- * window is at most 128 bytes; counting inserts
- * (bit 1) have kernels of their own.  Results are the same either way. */
+ * lane reads its key's window with 32-byte loads; bit 0 insert, 1 counting
+ * insert, 2 retrieve, 3 erase, default all four) instead of with groups of
+ * lanes per window and ballots.  Applies to windows of at most 128 bytes:
+ * for bits 0, 2 and 3 to tables whose slot array fits in L2; for bit 1 to
+ * counting inserts without statuses, into these tables and into larger ones
+ * whose windows are short (on tables with fingerprints too: with the bit
+ * clear they follow wc_fingerprint_ops).  Results are the same either way. */
 int wc_lane_ops(uint32_t op_mask, uint32_t *previous);
 
 /* ------------------------------------------------------------------ */

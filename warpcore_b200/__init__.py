@@ -442,9 +442,9 @@ def set_fingerprint_policy(mode):
 
 
 def set_lane_ops(op_mask):
-    """Operations (bit 0 insert, 2 retrieve, 3 erase) whose whole-window
-    probing reads one key's window per lane (wc_lane_ops); returns the
-    previous mask"""
+    """Operations (bit 0 insert, 1 counting insert, 2 retrieve, 3 erase) whose
+    whole-window probing reads one key's window per lane (wc_lane_ops);
+    returns the previous mask"""
     prev = ctypes.c_uint32(0)
     _check(lib().wc_lane_ops(int(op_mask), ctypes.byref(prev)))
     return prev.value

@@ -156,8 +156,10 @@ std::atomic<uint32_t> g_fp_ops{0xFu};
 
 /* Operations (bit kOp*) whose whole-window probing runs the one-key-per-lane
  * kernel (wc_lane_kernels.cuh) where a window is at most 128 bytes; the
- * others run table_op_kernel.  Counting inserts always run table_op_kernel. */
-std::atomic<uint32_t> g_lane_ops{0xDu};
+ * others run table_op_kernel.  Bit kOpCount: counting inserts without
+ * statuses may run count_insert_kernel (wc_count.cuh); all others run
+ * table_op_kernel or the fingerprint kernel. */
+std::atomic<uint32_t> g_lane_ops{0xFu};
 
 /* Random-access regions of the multi-pass kernels, for inserts and for
  * queries (bytes; 0 = one pass).  Random 64-byte reads on B200 measured
@@ -807,7 +809,8 @@ int check_table(const wc_table *t, int kind_mask)
  * the group kernel. */
 TableKernel pick_lane_kernel(const wc_table *t, int op)
 {
-    if (!((g_lane_ops.load(std::memory_order_relaxed) >> op) & 1u)) return nullptr;
+    if (op == kOpCount || !((g_lane_ops.load(std::memory_order_relaxed) >> op) & 1u))
+        return nullptr;
     if (t->capacity * t->slot_bytes > uint64_t(device_props().l2_bytes)) return nullptr;
     const int W = int(t->cfg.cg_size);
     switch (t->layout) {
@@ -866,6 +869,7 @@ TableKernel pick_table_kernel(const wc_table *t, int op)
 CountInsertKernel pick_count_insert_kernel(const wc_table *t, int op, uint64_t n, int handler)
 {
     if (op != kOpCount || handler != WC_HANDLER_NOTHING || (n >> 32)) return nullptr;
+    if (!((g_lane_ops.load(std::memory_order_relaxed) >> kOpCount) & 1u)) return nullptr;
     const uint64_t slots = t->capacity * t->slot_bytes;
     const uint64_t window = uint64_t(t->cfg.cg_size) * t->slot_bytes;
     if (slots > uint64_t(device_props().l2_bytes) &&
@@ -1561,7 +1565,7 @@ int wc_fingerprint_ops(uint32_t op_mask, uint32_t *previous)
 
 int wc_lane_ops(uint32_t op_mask, uint32_t *previous)
 {
-    const uint32_t prev = g_lane_ops.exchange(op_mask & 0xDu);
+    const uint32_t prev = g_lane_ops.exchange(op_mask & 0xFu);
     if (previous) *previous = prev;
     return WC_OK;
 }
