@@ -590,9 +590,9 @@ int wc_fingerprint_policy(int mode, int *previous);
 /* Which operations read fingerprints first on tables that have them: bit
  * 0 insert, 1 counting insert, 2 retrieve, 3 erase (default: all four;
  * an operation whose bit is clear probes whole windows and keeps the
- * fingerprints up to date).  Bit 4: a fingerprint-first counting insert
- * loads the slot it is about to claim before the compare-and-swap.  Bit 5: never
- * replace a large insert (more than 1/8 of a table whose fingerprints
+ * fingerprints up to date).  Bit 4: a fingerprint-first insert (counting
+ * or not) loads the slot it is about to claim before the compare-and-swap.
+ * Bit 5: never replace a large insert (more than 1/8 of a table whose fingerprints
  * exceed half of L2) by a whole-window insert without fingerprint writes
  * followed by a streaming rebuild of all fingerprints, which is the
  * default. */

@@ -72,6 +72,33 @@ def test_equal_keys_of_one_call(kb, vb, cg):
         assert t.size() == len(stored)
 
 
+@pytest.mark.parametrize("preload", [False, True])
+@pytest.mark.parametrize("kb,vb", [(4, 4), (8, 8), (4, 8), (8, 4)])
+def test_claims_over_stale_payloads(kb, vb, preload):
+    # free slots whose payload is not zero, with and without a load of the
+    # slot before its claim (bit 4): every key is stored once
+    n = 50_021
+    keys, vals = o.gen_unique_keys(kb, n, 25), o.gen_uniform(vb, n, 27)
+    at = np.concatenate([np.arange(n), np.arange(0, n, 3)])
+    prev = wc.set_fingerprint_ops(0x1F if preload else 0xF)
+    try:
+        t = wc.SingleValueHashTable(2 * n, key_bytes=kb, value_bytes=vb)
+        inf = t.info()
+        slots = bytes_view(inf.slots, t.capacity * inf.slot_bytes).view(t.capacity, inf.slot_bytes)
+        first = inf.slot_bytes // 2  # the payload follows the key
+        slots[::2, first:first + vb] = 7
+        for claims in (n, 0):
+            st = empty_dev(len(at), 4)
+            t.insert(dev(keys[at]), dev(vals[at]), status_out=st)
+            assert np.count_nonzero(host(st) == o.ST_NONE) == claims
+            assert t.size() == t.size_scan() == n
+            out = empty_dev(n, vb)
+            t.retrieve(dev(keys), out)
+            assert np.array_equal(host(out), vals)
+    finally:
+        wc.set_fingerprint_ops(prev)
+
+
 @pytest.mark.parametrize("kind", ["pairs32", "pairs64", "set32", "set64"])
 @pytest.mark.parametrize("skew", ["zipf", "runs", "one", "late"])
 def test_repeated_keys(kind, skew):

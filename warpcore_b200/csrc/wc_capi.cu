@@ -146,8 +146,8 @@ std::atomic<int> g_fp_mode{-1}; /* -1: not yet read from the environment */
 
 /* Operations (bit kOp*) that run the fingerprint-first kernel on tables
  * with fingerprints; the others run the whole-window kernel, which keeps
- * the fingerprints up to date.  Bit 4 makes the counting
- * fingerprint kernel load a claim's slot before its compare-and-swap.  Measured on B200 with u64
+ * the fingerprints up to date.  Bit 4 makes the inserting fingerprint
+ * kernels load a claim's slot before its compare-and-swap.  Measured on B200 with u64
  * pairs at load 0.9, 2^27 keys: retrieve 13.0 -> 20.5 G/s on fingerprints;
  * the window insert slows down on a fingerprint table (9.1 G/s, its
  * fingerprint byte writes miss L2) more than the fingerprint insert does

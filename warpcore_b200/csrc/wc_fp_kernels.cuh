@@ -725,6 +725,7 @@ __global__ void __launch_bounds__(256, fp_insert_min_blocks<L>()) fp_insert_kern
     constexpr int SB = L::kSlotBytes;
     constexpr bool kValueIn = L::kHasValue;
     constexpr bool kHold = kValueIn;
+    const bool preload = (a.flags & kFlagPreloadClaim) != 0;
     const uint64_t pol_keep = l2_policy_evict_last(); /* fingerprint lines */
 
     const TableView &t = a.t;
@@ -757,6 +758,7 @@ __global__ void __launch_bounds__(256, fp_insert_min_blocks<L>()) fp_insert_kern
      * with `free` the lowest slot of it is to be claimed, else the bucket's
      * fingerprints are due */
     bool has = false;
+    bool peeked = false; /* the claim's slot has been read (preload) */
     uint32_t cand = 0, free = 0, at = 0;
     uint32_t quiet = 0; /* refills since the last one with equal keys */
     /* waits: lane `first` inserts this lane's key too; held: some lane waits */
@@ -810,6 +812,7 @@ __global__ void __launch_bounds__(256, fp_insert_min_blocks<L>()) fp_insert_kern
                 has = true;
                 cand = 0;
                 free = 0;
+                peeked = false;
                 wins = 0;
                 step = 0;
                 fresh = key != empty && key != tomb;
@@ -856,10 +859,11 @@ __global__ void __launch_bounds__(256, fp_insert_min_blocks<L>()) fp_insert_kern
                                 : base_slot + uint64_t(free ? __ffs(free) - 1 : 0);
         unsigned char *const sp = slots + s * SB;
         const bool checking = cand != 0, claiming = !checking && free != 0;
+        const bool peeking = preload && claiming && !peeked;
         if (has && !waits) {
             /* slots are read where the claims' atomics land (L2): an L1 copy
              * may predate the claim of an equal key by another lane */
-            if (checking) sw = load_lane<SB>(sp);
+            if (checking || peeking) sw = load_lane<SB>(sp);
             else if (claiming) old = cas_slot<L>(sp, empty, expect, key, val, &old_payload);
             else f.load(t.fps + base_slot, pol_keep);
         }
@@ -879,18 +883,25 @@ __global__ void __launch_bounds__(256, fp_insert_min_blocks<L>()) fp_insert_kern
             cand &= cand - 1u;
             advance = cand == 0 && free == 0;
         } else if (claiming) {
-            if (old == empty && old_payload == expect) {
+            if (peeking) {
+                old = slot_key<L>(sw, 0);
+                old_payload = slot_val<L>(sw, 0);
+                peeked = old == empty;
+            } else if (old == empty && old_payload == expect) {
                 st_hint_u8(t.fps + s, fingerprint(key), pol_keep);
                 ++live_delta;
                 finish(kStNone);
-            } else if (old == key) {
+                continue;
+            }
+            if (old == key) {
                 store_value<L>(sp, val);
                 finish(kStDuplicateKey);
             } else if (old == empty) {
-                expect = old_payload; /* free slot, stale payload: again */
+                expect = old_payload; /* free slot, its payload known now */
             } else {
                 free &= free - 1u;
                 expect = 0;
+                peeked = false;
                 advance = free == 0;
             }
         } else {
