@@ -47,6 +47,9 @@ namespace b200 {
 #ifndef WC_MULTI_INSERT_BLOCKS
 #define WC_MULTI_INSERT_BLOCKS 4
 #endif
+/* (count: u64 keys spill up to 120 bytes with 6 and are no slower for it: 2^22
+ * lookups of multi-value u64 pairs 487 / 487 / 504 us with 6 / 5 / 4, multi-bucket
+ * at CG 4 319 / 335 / 358, bucket list 293 / 294 / 309) */
 #ifndef WC_MULTI_COUNT_BLOCKS
 #define WC_MULTI_COUNT_BLOCKS 6
 #endif
@@ -78,12 +81,16 @@ struct MultiArgs {
 constexpr int kMultiTile = 1024;
 /* keys per tile of multi_find_kernel, whose last walks leave lanes idle at a
  * barrier (a quarter of its stalls at 1024 keys).  2048 where keys take 4
- * bytes and windows at most 64; with more, the shared memory of six blocks
- * leaves L1 too small for the windows in flight (1024 / 2048: u32 pairs 380 /
- * 357 us, multi-bucket of u32 keys 586 / 550, u64 pairs 280 / 436). */
+ * bytes and windows, of a width known here, at most 64; with more, the shared
+ * memory of six blocks leaves L1 too small for the windows in flight (1024 /
+ * 2048: u32 pairs 380 / 357 us, multi-bucket of u32 keys 586 / 550, u64 pairs
+ * 280 / 436).  A run-time width (window_bytes 0) may be up to 128 bytes of
+ * 4-byte keys: retrieves of multi-bucket tables at CG 4 / 16 / 32 259 / 283 / 370
+ * us with 1024, 261 / 291 / 384 with 2048, of bucket lists 298 / 295 / 393 and
+ * 306 / 305 / 407. */
 constexpr int multi_find_tile(int key_bytes, int window_bytes)
 {
-    return key_bytes == 4 && window_bytes <= 64 ? 2 * kMultiTile : kMultiTile;
+    return key_bytes == 4 && window_bytes > 0 && window_bytes <= 64 ? 2 * kMultiTile : kMultiTile;
 }
 constexpr int kMultiThreads = 256;
 
