@@ -192,7 +192,8 @@ __global__ void __launch_bounds__(kMultiThreads, WC_MULTI_INSERT_BLOCKS)
                 c.count < v.max_values)
                 size[j] = bl_header_size(v, bl_load(v.pool + c.index));
         }
-        /* try[j]: the swap that takes a place or blocks the handle */
+        /* the swap that takes a place or blocks the handle, where the list may
+         * grow */
         bool tried[kPer];
 #pragma unroll
         for (int j = 0; j < kPer; ++j) {

@@ -1,5 +1,5 @@
 /*
- * wc_fp_kernels.cuh -- fingerprint-first bulk kernel for tables that keep
+ * wc_fp_kernels.cuh -- fingerprint-first bulk kernels for tables that keep
  * one fingerprint byte per slot (b200_core.cuh, "fingerprints").
  *
  * The bucket sequence, the slot order of claims and every per-key status
@@ -18,16 +18,14 @@
  *     erase: its compare-and-swap on the slot follows, with the words read
  *     as the expected value).
  *
- * Counting inserts run fp_op_kernel, inserts fp_insert_kernel, retrieve and
- * erase fp_find_kernel.
+ * Inserts run fp_insert_kernel, retrieve and erase fp_find_kernel, counting
+ * inserts fp_count_kernel (or count_insert_kernel, wc_count.cuh).
  *
  * Each lane owns one key and issues one memory operation per wave: a
  * fingerprint load, a candidate slot load, or a compare-and-swap claim.
  * The 32 lanes' operations are independent, so a warp keeps 32 requests in
  * flight.  Keys are refilled in input order from a double-buffered
- * prefetch, duplicates in one refill are merged with __match_any_sync, and
- * counting inserts go through the per-block count cache, as in
- * table_op_kernel.
+ * prefetch; inserts merge equal keys of a refill.
  */
 #ifndef WC_FP_KERNELS_CUH
 #define WC_FP_KERNELS_CUH
@@ -53,9 +51,6 @@ namespace b200 {
  * random slot traffic of a table larger than L2 evicts slot lines before
  * fingerprint lines (a fingerprint byte written into an evicted sector
  * costs a DRAM read to merge). */
-#ifndef WC_FP_L2_HINTS
-#define WC_FP_L2_HINTS 1
-#endif
 
 __device__ __forceinline__ uint64_t l2_policy_evict_last()
 {
@@ -125,18 +120,15 @@ __device__ __forceinline__ void fp_masks(const unsigned char *p, uint32_t fp, ui
         constexpr int NW = W / 4;
         uint32_t w[NW];
         if constexpr (W == 4) {
-            w[0] = WC_FP_L2_HINTS ? ld_hint_u32(p, pol)
-                                  : __ldcg(reinterpret_cast<const unsigned int *>(p));
+            w[0] = ld_hint_u32(p, pol);
         } else if constexpr (W == 8) {
-            const uint2 v = WC_FP_L2_HINTS ? ld_hint_v2(p, pol)
-                                           : __ldcg(reinterpret_cast<const uint2 *>(p));
+            const uint2 v = ld_hint_v2(p, pol);
             w[0] = v.x;
             w[1] = v.y;
         } else {
 #pragma unroll
             for (int h = 0; h < W / 16; ++h) {
-                const uint4 v = WC_FP_L2_HINTS ? ld_hint_v4(p + 16 * h, pol)
-                                               : __ldcg(reinterpret_cast<const uint4 *>(p) + h);
+                const uint4 v = ld_hint_v4(p + 16 * h, pol);
                 w[4 * h + 0] = v.x;
                 w[4 * h + 1] = v.y;
                 w[4 * h + 2] = v.z;
@@ -151,10 +143,7 @@ __device__ __forceinline__ void fp_masks(const unsigned char *p, uint32_t fp, ui
             empty |= pack_bytes4(__vcmpeq4(w[k], 0u)) << (4 * k);
         }
     } else {
-        const uint32_t x =
-            WC_FP_L2_HINTS ? (W == 2 ? ld_hint_u16(p, pol) : ld_hint_u8(p, pol))
-                           : (W == 2 ? uint32_t(__ldcg(reinterpret_cast<const unsigned short *>(p)))
-                                     : uint32_t(__ldcg(p)));
+        const uint32_t x = W == 2 ? ld_hint_u16(p, pol) : ld_hint_u8(p, pol);
         constexpr uint32_t lim = (1u << W) - 1u; /* the zero bytes above W are not slots */
         match = pack_bytes4(__vcmpeq4(x, pat)) & lim;
         empty = pack_bytes4(__vcmpeq4(x, 0u)) & lim;
@@ -178,10 +167,13 @@ __device__ __forceinline__ LaneWords load_slot_once(const unsigned char *sp)
     return r;
 }
 
-template <class L, int W, int OP>
-__global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_op_kernel(const TableOpArgs a)
+/* Counting insert.  The steps of a wave (fingerprints, slot, claim) run one
+ * after the other; duplicates in one refill are merged with __match_any_sync,
+ * and without per-key statuses keys go through the per-block count cache, both
+ * as in table_op_kernel. */
+template <class L, int W>
+__global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_count_kernel(const TableOpArgs a)
 {
-    static_assert(OP == kOpCount, "operation");
     using K = typename L::key_t;
     using V = typename L::val_t;
     constexpr int SB = L::kSlotBytes;
@@ -220,10 +212,10 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_op_kernel(const Tabl
     uint32_t st = kStNone, join = 0, cnt_add = 1;
     int live_delta = 0; /* claims minus erases of this lane */
 
-    constexpr int kCache = OP == kOpCount ? (1 << count_cache_bits<L>()) : 1;
+    constexpr int kCache = 1 << count_cache_bits<L>();
     __shared__ K sc_key[kCache];
     __shared__ V sc_cnt[kCache];
-    const bool use_cache = OP == kOpCount && a.handler == kHandlerNothing;
+    const bool use_cache = a.handler == kHandlerNothing;
     if (use_cache) {
         for (int c = threadIdx.x; c < kCache; c += blockDim.x) {
             sc_key[c] = empty;
@@ -284,28 +276,26 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_op_kernel(const Tabl
                 }
             }
         }
-        if constexpr (OP == kOpCount) {
-            if (use_cache && refill && pending) {
-                using CW = typename std::conditional<sizeof(K) == 8, unsigned long long,
-                                                     unsigned int>::type;
-                const uint32_t h = uint32_t((uint64_t(key) * 0x9E3779B97F4A7C15ull) >> (64 - count_cache_bits<L>()));
+        if (use_cache && refill && pending) {
+            using CW = typename std::conditional<sizeof(K) == 8, unsigned long long,
+                                                 unsigned int>::type;
+            const uint32_t h = uint32_t((uint64_t(key) * 0x9E3779B97F4A7C15ull) >> (64 - count_cache_bits<L>()));
 #pragma unroll
-                for (int p = 0; p < 4; ++p) {
-                    const int c = int((h + p) & (kCache - 1));
-                    K cur = *reinterpret_cast<volatile K *>(&sc_key[c]);
-                    bool first = false;
-                    if (cur == empty) {
-                        cur = K(atomicCAS(reinterpret_cast<CW *>(&sc_key[c]), CW(empty), CW(key)));
-                        first = cur == empty;
-                        if (first) cur = key;
-                    }
-                    if (cur == key) {
-                        atomic_add_any(&sc_cnt[c], V(cnt_add));
-                        if (!first) join |= kStDuplicateKey;
-                        st = kStNone;
-                        pending = false;
-                        break;
-                    }
+            for (int p = 0; p < 4; ++p) {
+                const int c = int((h + p) & (kCache - 1));
+                K cur = *reinterpret_cast<volatile K *>(&sc_key[c]);
+                bool first = false;
+                if (cur == empty) {
+                    cur = K(atomicCAS(reinterpret_cast<CW *>(&sc_key[c]), CW(empty), CW(key)));
+                    first = cur == empty;
+                    if (first) cur = key;
+                }
+                if (cur == key) {
+                    atomic_add_any(&sc_cnt[c], V(cnt_add));
+                    if (!first) join |= kStDuplicateKey;
+                    st = kStNone;
+                    pending = false;
+                    break;
                 }
             }
         }
@@ -374,11 +364,7 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_op_kernel(const Tabl
                     /* (atom.cas takes no L2 cache hint) */
                     const K old = cas_slot<L>(sp, empty, claim_expect, key, payload, &old_payload);
                     if (old == empty && old_payload == claim_expect) {
-#if WC_FP_L2_HINTS
                         st_hint_u8(t.fps + base_slot + uint64_t(s), fp, pol_keep);
-#else
-                        fp_store(t, base_slot + uint64_t(s), fp);
-#endif
                         ++live_delta;
                         st = kStNone;
                         pending = false;
@@ -437,14 +423,12 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS) fp_op_kernel(const Tabl
             has = false;
         }
     }
-    if constexpr (OP == kOpCount) {
-        if (use_cache) {
-            __syncthreads();
-            for (int c = threadIdx.x; c < kCache; c += blockDim.x) {
-                const K ck = sc_key[c];
-                if (ck != empty)
-                    count_one<L, W>(t, ck, uint32_t(sc_cnt[c]), a.max_windows, join, live_delta);
-            }
+    if (use_cache) {
+        __syncthreads();
+        for (int c = threadIdx.x; c < kCache; c += blockDim.x) {
+            const K ck = sc_key[c];
+            if (ck != empty)
+                count_one<L, W>(t, ck, uint32_t(sc_cnt[c]), a.max_windows, join, live_delta);
         }
     }
     const uint32_t wjoin = __reduce_or_sync(kFull, join);
@@ -520,8 +504,8 @@ struct FpWords {
     }
 };
 
-/* Retrieve and erase on tables with fingerprints.  What fp_op_kernel was
- * bound by here is instruction issue (28 warp instructions per query, 77 %
+/* Retrieve and erase on tables with fingerprints.  What a kernel in the form of
+ * fp_count_kernel was bound by here is instruction issue (28 warp instructions per query, 77 %
  * issue-active): a wave ran the fingerprint and the slot step one after the
  * other, each waiting for its own load, built masks byte by byte and carried
  * 64-bit places.  Here the lanes' fingerprint and slot loads are in flight
@@ -686,7 +670,7 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS_READ) fp_find_kernel(con
 /* Insert on tables with fingerprints, in the form of fp_find_kernel: the
  * lanes' fingerprint loads, slot reads and claims are in flight together.
  * Claims take the lowest slot with an empty fingerprint first, as in
- * fp_op_kernel.  Against fp_op_kernel, which ran the
+ * fp_count_kernel.  Against a kernel in the form of that one, which ran the
  * three steps one after the other: u64 set of 134 MB at load 0.9, 15 M keys
  * 727 -> 597 us; u64 pairs of 161 MB, 9 M 491 -> 444; u32 pairs of 269 MB, 30 M
  * 1612 -> 1423; 65 536 updates of 575 MB of u64 pairs 41 -> 33.

@@ -26,8 +26,8 @@
  * compare-and-swap that loses sees the key.  A claim that loses its slot to
  * another key reads the window again.
  *
- * Insert, retrieve and erase; counting inserts keep table_op_kernel and its
- * shared-memory count cache.
+ * Insert, retrieve and erase; counting inserts without statuses have a kernel
+ * of this form with a count cache (wc_count.cuh), the others table_op_kernel.
  */
 #ifndef WC_LANE_KERNELS_CUH
 #define WC_LANE_KERNELS_CUH

@@ -17,7 +17,7 @@ TableKernel pick_table_op(int op, bool fp)
 {
     switch (op) {
     case kOpInsert: return fp ? fp_insert_kernel<L, W> : table_op_kernel<L, W, kOpInsert>;
-    case kOpCount: return fp ? fp_op_kernel<L, W, kOpCount> : table_op_kernel<L, W, kOpCount>;
+    case kOpCount: return fp ? fp_count_kernel<L, W> : table_op_kernel<L, W, kOpCount>;
     case kOpRetrieve: return fp ? fp_find_kernel<L, W, kOpRetrieve> : table_op_kernel<L, W, kOpRetrieve>;
     case kOpErase: return fp ? fp_find_kernel<L, W, kOpErase> : table_op_kernel<L, W, kOpErase>;
     default: return nullptr;
