@@ -829,19 +829,22 @@ TableKernel pick_window_kernel(const wc_table *t, int op)
     if (TableKernel k = pick_lane_kernel(t, op)) return k;
     const int W = int(t->cfg.cg_size);
     switch (t->layout) {
-    case kLayoutKV32: return table_kernel_kv32(W, op, false);
-    case kLayoutKV64: return table_kernel_kv64(W, op, false);
-    case kLayoutSet32: return table_kernel_set32(W, op, false);
-    case kLayoutK32V64: return table_kernel_k32v64(W, op, false);
-    case kLayoutK64V32: return table_kernel_k64v32(W, op, false);
-    default: return table_kernel_set64(W, op, false);
+    case kLayoutKV32: return table_kernel_kv32(W, op, kFpNone);
+    case kLayoutKV64: return table_kernel_kv64(W, op, kFpNone);
+    case kLayoutSet32: return table_kernel_set32(W, op, kFpNone);
+    case kLayoutK32V64: return table_kernel_k32v64(W, op, kFpNone);
+    case kLayoutK64V32: return table_kernel_k64v32(W, op, kFpNone);
+    default: return table_kernel_set64(W, op, kFpNone);
     }
 }
 
 TableKernel pick_table_kernel(const wc_table *t, int op)
 {
     const int W = int(t->cfg.cg_size);
-    const bool fp = t->fps != nullptr && ((g_fp_ops.load(std::memory_order_relaxed) >> op) & 1u);
+    const uint32_t ops = g_fp_ops.load(std::memory_order_relaxed);
+    const int fp = t->fps == nullptr || !((ops >> op) & 1u) ? kFpNone
+                   : ops & 0x10u                             ? kFpPreload
+                                                             : kFpFirst;
     if (!fp) return pick_window_kernel(t, op);
     switch (t->layout) {
     case kLayoutKV32: return table_kernel_kv32(W, op, fp);

@@ -690,7 +690,9 @@ __global__ void __launch_bounds__(256, WC_FP_MIN_BLOCKS_READ) fp_find_kernel(con
  * and smaller refills reads and writes its slot's line more often: 4 M
  * Zipf(1.1) updates of u64 pairs 10.2 ms without waiting, 6.8 with it (and
  * without merging); keys in runs of 16 125 us with waiting always, 87 so.
- * Sets, which write nothing for a key that is there, gain nothing by it. */
+ * Sets, which write nothing for a key that is there, gain nothing by it.
+ *
+ * kPreload: a claim's slot is loaded before its compare-and-swap. */
 constexpr uint32_t kMergeQuiet = 4;
 
 /* one more block than the other kernels where 48 registers do: 4 M u32 pairs
@@ -701,7 +703,7 @@ constexpr int fp_insert_min_blocks()
     return L::kSlotBytes <= 8 ? WC_FP_MIN_BLOCKS + 1 : WC_FP_MIN_BLOCKS;
 }
 
-template <class L, int W>
+template <class L, int W, bool kPreload>
 __global__ void __launch_bounds__(256, fp_insert_min_blocks<L>()) fp_insert_kernel(const TableOpArgs a)
 {
     using K = typename L::key_t;
@@ -709,7 +711,6 @@ __global__ void __launch_bounds__(256, fp_insert_min_blocks<L>()) fp_insert_kern
     constexpr int SB = L::kSlotBytes;
     constexpr bool kValueIn = L::kHasValue;
     constexpr bool kHold = kValueIn;
-    const bool preload = (a.flags & kFlagPreloadClaim) != 0;
     const uint64_t pol_keep = l2_policy_evict_last(); /* fingerprint lines */
 
     const TableView &t = a.t;
@@ -742,7 +743,7 @@ __global__ void __launch_bounds__(256, fp_insert_min_blocks<L>()) fp_insert_kern
      * with `free` the lowest slot of it is to be claimed, else the bucket's
      * fingerprints are due */
     bool has = false;
-    bool peeked = false; /* the claim's slot has been read (preload) */
+    bool peeked = false; /* the claim's slot has been read (kPreload) */
     uint32_t cand = 0, free = 0, at = 0;
     uint32_t quiet = 0; /* refills since the last one with equal keys */
     /* waits: lane `first` inserts this lane's key too; held: some lane waits */
@@ -843,7 +844,7 @@ __global__ void __launch_bounds__(256, fp_insert_min_blocks<L>()) fp_insert_kern
                                 : base_slot + uint64_t(free ? __ffs(free) - 1 : 0);
         unsigned char *const sp = slots + s * SB;
         const bool checking = cand != 0, claiming = !checking && free != 0;
-        const bool peeking = preload && claiming && !peeked;
+        const bool peeking = kPreload && claiming && !peeked;
         if (has && !waits) {
             /* slots are read where the claims' atomics land (L2): an L1 copy
              * may predate the claim of an equal key by another lane */

@@ -33,12 +33,12 @@ using DumpKernel = void (*)(const void *, uint64_t, uint64_t, uint64_t, void *, 
                             unsigned long long *);
 
 /* kernel for (window width W, op); nullptr if the combination is not built */
-TableKernel table_kernel_kv32(int W, int op, bool fingerprints);
-TableKernel table_kernel_kv64(int W, int op, bool fingerprints);
-TableKernel table_kernel_set32(int W, int op, bool fingerprints);
-TableKernel table_kernel_set64(int W, int op, bool fingerprints);
-TableKernel table_kernel_k32v64(int W, int op, bool fingerprints);
-TableKernel table_kernel_k64v32(int W, int op, bool fingerprints);
+TableKernel table_kernel_kv32(int W, int op, int fp);
+TableKernel table_kernel_kv64(int W, int op, int fp);
+TableKernel table_kernel_set32(int W, int op, int fp);
+TableKernel table_kernel_set64(int W, int op, int fp);
+TableKernel table_kernel_k32v64(int W, int op, int fp);
+TableKernel table_kernel_k64v32(int W, int op, int fp);
 /* the one-key-per-lane window kernel of (W, op), nullptr if not built */
 TableKernel lane_kernel_kv32(int W, int op);
 TableKernel lane_kernel_kv64(int W, int op);

@@ -47,8 +47,10 @@ struct TableOpArgs {
     uint32_t flags;       /* kFlag* */
 };
 
-/* fingerprint kernel: before the compare-and-swap of a claim, read the
- * target slot with a plain load (into L2), then CAS on the resident line */
+/* which kernel: whole windows, fingerprints first, and of the inserting ones
+ * that which reads a claim's slot with a plain load (into L2) before its
+ * compare-and-swap on the resident line (the counting kernel: a flag) */
+enum : int { kFpNone = 0, kFpFirst = 1, kFpPreload = 2 };
 constexpr uint32_t kFlagPreloadClaim = 1u;
 
 constexpr unsigned kFull = 0xffffffffu;

@@ -13,10 +13,13 @@ namespace warpcore {
 namespace b200 {
 
 template <class L, int W>
-TableKernel pick_table_op(int op, bool fp)
+TableKernel pick_table_op(int op, int fp)
 {
     switch (op) {
-    case kOpInsert: return fp ? fp_insert_kernel<L, W> : table_op_kernel<L, W, kOpInsert>;
+    case kOpInsert:
+        return fp == kFpPreload ? fp_insert_kernel<L, W, true>
+               : fp             ? fp_insert_kernel<L, W, false>
+                                : table_op_kernel<L, W, kOpInsert>;
     case kOpCount: return fp ? fp_count_kernel<L, W> : table_op_kernel<L, W, kOpCount>;
     case kOpRetrieve: return fp ? fp_find_kernel<L, W, kOpRetrieve> : table_op_kernel<L, W, kOpRetrieve>;
     case kOpErase: return fp ? fp_find_kernel<L, W, kOpErase> : table_op_kernel<L, W, kOpErase>;
@@ -25,7 +28,7 @@ TableKernel pick_table_op(int op, bool fp)
 }
 
 template <class L>
-TableKernel pick_table_kernel_for(int W, int op, bool fp)
+TableKernel pick_table_kernel_for(int W, int op, int fp)
 {
     switch (W) {
     case 1: return pick_table_op<L, 1>(op, fp);

@@ -4,7 +4,7 @@
 namespace warpcore {
 namespace b200 {
 
-TableKernel table_kernel_set32(int W, int op, bool fp) { return pick_table_kernel_for<LayoutSet32>(W, op, fp); }
+TableKernel table_kernel_set32(int W, int op, int fp) { return pick_table_kernel_for<LayoutSet32>(W, op, fp); }
 TableKernel lane_kernel_set32(int W, int op) { return pick_lane_kernel_for<LayoutSet32>(W, op); }
 
 } // namespace b200
