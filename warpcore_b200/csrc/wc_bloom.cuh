@@ -223,24 +223,29 @@ __device__ __forceinline__ bool block_has_all(K key, K seed, uint32_t hasher, ui
  * blocks, never / always / this: 2^28 distinct keys 12.13 / 12.82 / 12.31 ms,
  * inserted again 12.13 / 9.31 / 9.88, 2^27 Zipf(0.8) keys 10.0 / 5.3 / 5.4,
  * Zipf(1.1) 32.2 / 5.0 / 5.1, 2^24 times one key 17.2 / 0.53 / 0.48; 6 M keys into a
- * 16 MiB filter of 32-byte blocks: 171 / 197 / 179 us, 169 / 116 / 120, 171 / 155 /
- * 155, 478 / 186 / 152, 3 077 / 271 / 170.  Few keys sampled per look would not do:
- * regions hold some 16 keys of a tile, and with "two present in the last
+ * 16 MiB filter of 32-byte blocks: 171 / 197 / 177 us, 169 / 116 / 116, 171 / 155 /
+ * 151, 478 / 186 / 145, 3 077 / 271 / 150.  The share is taken over several rounds:
+ * a region holds some 16 keys of a tile, and with "two present in the last
  * round" Zipf(1.1) took 14.6 ms. */
 struct LookFirst {
     static constexpr uint32_t kSample = 64, kFew = 32, kSkip = 15;
     uint32_t keys = 0, there = 0, skip = 0;
 
     __device__ __forceinline__ bool now() const { return skip == 0; }
-    /* ends a round: lanes with a key, and (looked at) with one that was there */
-    __device__ __forceinline__ void next(bool in, bool present)
+    /* keys of a round that was looked at: which lanes had one, and had one
+     * that was there */
+    __device__ __forceinline__ void looked(bool in, bool present)
+    {
+        keys += uint32_t(__popc(__ballot_sync(kFull, in)));
+        there += uint32_t(__popc(__ballot_sync(kFull, present)));
+    }
+    /* ends a round */
+    __device__ __forceinline__ void next()
     {
         if (skip) {
             --skip;
             return;
         }
-        keys += uint32_t(__popc(__ballot_sync(kFull, in)));
-        there += uint32_t(__popc(__ballot_sync(kFull, present)));
         if (keys >= kSample && there * kFew < keys) skip = kSkip;
         if (keys >= 4 * kSample) {
             keys /= 2;
@@ -251,15 +256,15 @@ struct LookFirst {
 
 constexpr uint64_t kNoBlock = ~0ull;
 
-/* ORs one key per lane into the block that starts at word `first` (kNoBlock:
- * no key).  Whole warps call it. */
+/* ORs a key into the block that starts at word `first` (kNoBlock: no key);
+ * whether its bits were all there (bulk ORs with `read`: the block is read
+ * first) */
 template <class K, class S, int CG, bool kBulk>
-__device__ __forceinline__ void bloom_or(const BloomArgs &a, K key, uint64_t first,
-                                         unsigned char *row, LookFirst &look)
+__device__ __forceinline__ bool bloom_or(const BloomArgs &a, K key, uint64_t first,
+                                         unsigned char *row, bool read)
 {
     S *const words = reinterpret_cast<S *>(a.words);
     const bool whole = first != kNoBlock && first + CG <= a.num_slots;
-    const bool read = !kBulk || look.now();
     bool there = false;
     if (first != kNoBlock) {
         S w[CG];
@@ -292,7 +297,7 @@ __device__ __forceinline__ void bloom_or(const BloomArgs &a, K key, uint64_t fir
             }
         }
     }
-    if constexpr (kBulk) look.next(first != kNoBlock, there);
+    return there;
 }
 
 template <class K, class S, int CG, bool INSERT>
@@ -424,8 +429,17 @@ constexpr int bloom_keys_per_lane()
     return INSERT && BulkOr<S, CG>::kUsed && CG * int(sizeof(S)) <= 32 ? 2 : 1;
 }
 
+/* resident blocks: inserts of blocks of up to 32 bytes keep the six they have
+ * at 40 registers (43 without the bound: 182 us, 176 with it) */
+template <class S, int CG, bool INSERT>
+constexpr int bloom_lane_min_blocks()
+{
+    return INSERT && CG * sizeof(S) <= 32 ? 6 : 1;
+}
+
 template <class K, class S, int CG, bool INSERT>
-__global__ void __launch_bounds__(256) bloom_lane_kernel(const BloomArgs a)
+__global__ void __launch_bounds__(256, bloom_lane_min_blocks<S, CG, INSERT>())
+    bloom_lane_kernel(const BloomArgs a)
 {
     constexpr int U = bloom_keys_per_lane<S, CG, INSERT>();
     static_assert(CG * sizeof(S) <= 128, "block of one lane");
@@ -439,9 +453,10 @@ __global__ void __launch_bounds__(256) bloom_lane_kernel(const BloomArgs a)
     __shared__ uint32_t s_words[INSERT ? 1 : CG * sizeof(S) / 4 * 256];
     const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
     LookFirst look;
-    /* (whole warps stay in the loop) */
-    for (uint64_t i0 = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-         i0 - (threadIdx.x & 31) < a.n; i0 += stride * U) {
+    /* (whole warps stay in the loop where look has its ballots) */
+    const uint64_t end = kBulk ? a.n + (threadIdx.x & 31) : a.n;
+    for (uint64_t i0 = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i0 < end;
+         i0 += stride * U) {
         K key[U];
         uint64_t w0[U]; /* first word of the key's block, kNoBlock: not served */
 #pragma unroll
@@ -461,10 +476,19 @@ __global__ void __launch_bounds__(256) bloom_lane_kernel(const BloomArgs a)
             }
         }
         if constexpr (INSERT) {
+            const bool read = look.now();
+            bool there[U];
 #pragma unroll
             for (int u = 0; u < U; ++u)
-                bloom_or<K, S, CG, kBulk>(a, key[u], w0[u],
-                                          s_rows + (kBulk ? threadIdx.x * Bulk::kRow : 0), look);
+                there[u] = bloom_or<K, S, CG, kBulk>(
+                    a, key[u], w0[u], s_rows + (kBulk ? threadIdx.x * Bulk::kRow : 0), read);
+            if constexpr (kBulk) {
+                if (read) {
+#pragma unroll
+                    for (int u = 0; u < U; ++u) look.looked(w0[u] != kNoBlock, there[u]);
+                }
+                look.next();
+            }
         } else {
             S w[U][CG];
 #pragma unroll
@@ -582,8 +606,13 @@ __global__ void __launch_bounds__(256, CG * sizeof(S) <= 64 ? 4 : 2) bloom_regio
             const K key = e < cnt ? s_key[wib][e] : K(0);
             const uint64_t w0 = e < cnt ? (a.region_lo + s_rel[wib][e]) * CG : kNoBlock;
             if constexpr (INSERT) {
-                bloom_or<K, S, CG, kBulk>(a, key, w0,
-                                          s_rows + (kBulk ? threadIdx.x * Bulk::kRow : 0), look);
+                const bool read = look.now();
+                const bool there = bloom_or<K, S, CG, kBulk>(
+                    a, key, w0, s_rows + (kBulk ? threadIdx.x * Bulk::kRow : 0), read);
+                if constexpr (kBulk) {
+                    if (read) look.looked(w0 != kNoBlock, there);
+                    look.next();
+                }
             } else if (e < cnt) {
                 S w[CG];
                 if (w0 + CG <= a.num_slots) {
