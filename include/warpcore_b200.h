@@ -629,13 +629,13 @@ int wc_region_bytes(int op, uint64_t bytes, uint64_t *previous);
 /* reference)                                                            */
 /* ------------------------------------------------------------------ */
 
-/* A table or filter whose slot array fits the device's persisting-L2
- * maximum (cudaDevAttrMaxPersistingL2CacheSize) launches its kernels with an
- * access-policy window over that array: its lines persist in L2 while keys
- * and outputs stream past, and while other work runs between calls.  Arrays
- * get windows at creation, in order, while no larger than the persisting
- * set-aside (a sixth of L2) and, with the windows of all live arrays on the
- * device, within twice that; the others launch without one.  The first such array sets this process's persisting-L2
+/* A table or filter whose slot array fits the persisting-L2 set-aside, a sixth
+ * of L2 (21 MB; B200 grants 24), launches its kernels with an access-policy
+ * window over that array: its lines persist in L2 while keys and outputs
+ * stream past, and while other work runs between calls.  Arrays get windows
+ * at creation, in order, while the windows of all live arrays on the device
+ * stay within twice the set-aside; the others, and larger arrays, launch
+ * without one.  The first such array sets this process's persisting-L2
  * limit once per device.  On by default (environment variable
  * WARPCORE_B200_L2_PERSIST=0 in the Python binding turns it off);
  * `enable` = 0 turns the windows off for later launches and creations

@@ -1,7 +1,9 @@
-"""The one-pass lookup of the multi-value, multi-bucket and bucket-list
-tables at the edges of its tiles: query counts around a block's threads, a
-full tile and a full wave, more windows with values than a tile can note,
-and a key with more values than a note's position holds."""
+"""The lookups and inserts of the multi-value, multi-bucket and bucket-list
+tables at the edges of their tiles: query counts around a block's threads, a
+full tile and a full wave, keys whose values fill many windows, a key with
+tens of thousands of values, input counts around warps, queues and waves.
+(Two tests are named after notes of the windows found, which an earlier form
+of the lookup kept.)"""
 import numpy as np
 import pytest
 import torch

@@ -119,8 +119,8 @@ const DeviceProps &device_props()
 }
 
 /* ---- L2 persistence for tables that fit in L2 ----
- * A table (or filter) whose slot array fits the device's persisting-L2
- * maximum gets an access-policy window over that array on each of its own
+ * A table (or filter) whose slot array fits the persisting-L2 set-aside
+ * gets an access-policy window over that array on each of its own
  * launches (a launch attribute, so the caller's streams are untouched):
  * its lines are kept as persisting and the streamed keys and outputs cannot
  * evict them.  The set-aside is this process's context limit
@@ -135,7 +135,10 @@ const DeviceProps &device_props()
  * 24.05 with 71 MB; a filter or table fill falls from 5.4 to 2.7 TB/s.  So
  * the set-aside asked for is a sixth of L2 (21 MB, 24 MB granted), the
  * largest size that costs the others nothing; one small table used to
- * halve the inserts of every large one beside it. */
+ * halve the inserts of every large one beside it.  Tables of 24 to 79 MB have
+ * no window since: 2^20 lookups of a 40 MB u32 table after a 1 GiB copy took 40
+ * us with a window and 49 without when the set-aside was 71 MB, and take 34
+ * now without one. */
 constexpr int kL2SetAsideFraction = 6;
 std::atomic<int> g_l2_mode{1};
 
