@@ -161,3 +161,34 @@ def test_one_key_many_times_is_not_slow(kind):
             ms.append(a.elapsed_time(b))
         times.append(min(ms[1:]))
     assert times[1] < 6 * times[0], times
+
+
+@pytest.mark.parametrize("kind", ["count32", "count64", "count64_32", "set32"])
+def test_rebuild_keeps_fingerprints_of_other_claims(kind):
+    # a large insert writes no fingerprints and has them recomputed after; a
+    # slot that it reads as empty may be claimed by another stream's insert
+    # before it writes, and that one's fingerprint must stay.  Here every
+    # empty slot is in that state.
+    if kind == "set32":  # (sets rebuild where fingerprints exceed half of L2)
+        kb = 4
+        cap = torch.cuda.get_device_properties(0).L2_cache_size // 2 + (1 << 20)
+        t = wc.HashSet(cap, key_bytes=4)
+    else:
+        kb, vb = {"count32": (4, 4), "count64": (8, 8), "count64_32": (8, 4)}[kind]
+        t = wc.CountingHashTable(1_000_003, key_bytes=kb, value_bytes=vb)
+    n = t.capacity // 4
+    keys = torch.empty(n, dtype={4: torch.int32, 8: torch.int64}[kb], device="cuda")
+    wc.gen_unique(keys, 39)
+    fps = bytes_view(t.info().fingerprints, t.capacity)
+    fps.fill_(255)
+    t.insert(keys)
+    assert t.size() == t.size_scan() == n
+    assert bool((fps != 0).all())
+    assert int((fps != 255).sum()) > n * 9 // 10  # the stored keys' were written
+    if kind == "set32":
+        out = torch.zeros(n, dtype=torch.uint8, device="cuda")
+        t.retrieve(keys, out)
+    else:
+        out = empty_dev(n, vb)
+        t.retrieve(keys, out)
+    assert bool((out == 1).all())

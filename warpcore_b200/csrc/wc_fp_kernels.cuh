@@ -919,7 +919,15 @@ __global__ void __launch_bounds__(256, fp_insert_min_blocks<L>()) fp_insert_kern
  * large insert runs the whole-window kernel without fingerprint writes and
  * then this pass: streaming the slot array costs less than one random byte
  * write per key once a batch covers more than about 1/8 of a table larger
- * than L2. */
+ * than L2.
+ *
+ * A slot read as empty leaves its fingerprint alone: an insert on another
+ * stream may claim it and store its fingerprint between the read and the
+ * write here, and a cleared fingerprint would hide its key for good.  (A
+ * fingerprint never has to be cleared, since no slot becomes empty again.)
+ * The stores of mixed vectors byte by byte cost under 1 % of an insert: 2^27
+ * u64 pairs 8.76 -> 8.79 ms, 135 M u32 pairs 8.37 -> 8.40, 180 M keys into a
+ * u32 set 9.42 -> 9.47. */
 template <class L>
 __device__ __forceinline__ uint32_t fp_of_slot_key(typename L::key_t k, typename L::key_t e,
                                                    typename L::key_t tb)
@@ -956,16 +964,25 @@ __global__ void __launch_bounds__(256) fp_rebuild_kernel(const void *slots, uint
             uint32_t f = 0;
 #pragma unroll
             for (int s = 0; s < SPV; ++s) f |= fp_of_slot_key<L>(slot_key<L>(lw, s), e, tb) << (8 * s);
-            if constexpr (SPV == 1) fps[v] = (unsigned char)f;
-            else if constexpr (SPV == 2) reinterpret_cast<unsigned short *>(fps)[v] = (unsigned short)f;
-            else reinterpret_cast<uint32_t *>(fps)[v] = f;
+            bool all = true;
+#pragma unroll
+            for (int s = 0; s < SPV; ++s) all &= (f >> (8 * s) & 0xffu) != kFpEmpty;
+            if (all) {
+                if constexpr (SPV == 1) fps[v] = (unsigned char)f;
+                else if constexpr (SPV == 2) reinterpret_cast<unsigned short *>(fps)[v] = (unsigned short)f;
+                else reinterpret_cast<uint32_t *>(fps)[v] = f;
+            } else if constexpr (SPV > 1) {
+#pragma unroll
+                for (int s = 0; s < SPV; ++s)
+                    if (f >> (8 * s) & 0xffu) fps[v * SPV + s] = (unsigned char)(f >> (8 * s));
+            }
         }
     }
     /* ragged tail: capacity need not be a multiple of SPV */
     if (blockIdx.x == 0 && threadIdx.x < capacity % SPV) {
         const uint64_t si = nvec * SPV + threadIdx.x;
         const K k = *reinterpret_cast<const K *>(reinterpret_cast<const unsigned char *>(slots) + si * SB);
-        fps[si] = (unsigned char)fp_of_slot_key<L>(k, e, tb);
+        if (k != e) fps[si] = (unsigned char)fp_of_slot_key<L>(k, e, tb);
     }
 }
 
