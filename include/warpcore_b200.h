@@ -173,7 +173,11 @@ int wc_table_destroy(wc_table *t);
  * counting tables too (hash_set.cuh:161-175, counting_hash_table.cuh:114-124) */
 int wc_table_init(wc_table *t, uint64_t seed, wc_stream_t stream);
 /* insert(keys_in, values_in, num_in, stream, probing_length, status_out)
- * (single_value_hash_table.cuh:241-258) */
+ * (single_value_hash_table.cuh:241-258).  Equal keys in one call take one
+ * slot, and all but one of them report duplicate_key; the slot ends with the
+ * value of any of them, as their writes race (in calls of at most 32 keys of
+ * the last one, except in tables that L2 holds with windows of at most 64
+ * bytes). */
 int wc_svht_insert(wc_table *t, const void *keys_in, const void *values_in,
                    uint64_t num_in, wc_stream_t stream,
                    uint64_t probing_length, void *status_out,
