@@ -1,6 +1,7 @@
-"""Lookups of several values per key where one key's walk visits the whole
-table: an absent key in a full table.  Its tile of the lookup is then far
-behind all others, and the call is slow but answers as any other."""
+"""Walks far longer than their neighbours: lookups of several values per key
+where one key's walk visits the whole table (an absent key in a full one; its
+tile of the lookup is then far behind all others, and the call is slow but
+answers as any other), and inserts of thousands of values of one key."""
 import numpy as np
 import pytest
 import torch
@@ -47,3 +48,36 @@ def test_absent_key_in_a_full_table(kind):
     assert np.array_equal(host(begin).astype(np.int64), np.maximum(np.arange(n) - 1, 0))
     assert np.array_equal(host(out).view(np.uint32), values)
     assert np.array_equal(host(st), np.where(np.arange(n) == 0, o.ST_PROBING_LENGTH_EXCEEDED, 0))
+
+
+@pytest.mark.parametrize("kind", ["mv", "mb1", "mb4"])
+@pytest.mark.parametrize("kb,vb,cg", [(4, 4, 8), (8, 8, 8), (4, 8, 1)])
+def test_many_values_of_one_key_in_one_batch(kind, kb, vb, cg):
+    # a list of more than 128 windows, filled by many warps at once between
+    # other keys: every value stored once, one first value per key
+    hot, others = 9000 // (8 // cg if cg < 8 else 1), 20_011
+    keys = o.gen_unique_keys(kb, others + 1, 107)
+    at = np.concatenate([np.full(hot, others), np.arange(others)])
+    at = at[np.random.default_rng(17).permutation(len(at))]
+    n = len(at)
+    vals = (np.arange(n) + 1).astype({4: np.uint32, 8: np.uint64}[vb])
+    if kind == "mv":
+        t = wc.MultiValueHashTable(2 * n, key_bytes=kb, value_bytes=vb, cg_size=cg)
+    else:
+        if int(kind[2:]) > cg:
+            pytest.skip("buckets are no larger than windows")
+        t = wc.MultiBucketHashTable(2 * n, key_bytes=kb, value_bytes=vb, cg_size=cg,
+                                    bucket_size=int(kind[2:]))
+    st = empty_dev(n, 4)
+    t.insert(dev(keys[at]), dev(vals), status_out=st)
+    assert t.num_keys() == others + 1
+    assert np.count_nonzero(host(st) == o.ST_NONE) == others + 1
+    assert np.count_nonzero(host(st) == o.ST_DUPLICATE_KEY) == hot - 1
+    begin, end = (torch.zeros(others + 1, dtype=torch.int64, device="cuda") for _ in range(2))
+    out = empty_dev(n, vb)
+    assert t.retrieve(dev(keys), begin, end, out) == n
+    b, e, got = (host(x).astype(np.int64) for x in (begin, end, out))
+    owner = np.repeat(np.arange(others + 1), e - b)
+    order = np.argsort(got)
+    assert np.array_equal(got[order], np.arange(n) + 1)
+    assert np.array_equal(owner[order], at)

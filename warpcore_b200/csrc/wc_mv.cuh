@@ -68,10 +68,19 @@ struct MvWalk {
      * has one; a claim that loses tries the next free slot it saw ---- */
     static constexpr int WB = W * L::kSlotBytes;
     static constexpr int kInsertBlocks = WB <= 64 ? WC_MULTI_INSERT_BLOCKS : 3;
+    /* Many values of one key in one batch queue at the end of its walk, where
+     * each step's compare-and-swaps of all its lanes but one are lost.  Past
+     * kCrowd windows a lane that lost to its own key sits out up to kCrowdSkip
+     * steps: 2^20 Zipf(0.8) keys over 2^20 (the most frequent 14 000 times) 13.6
+     * -> 11.1 ms in u32 pairs, 13.4 -> 12.0 in u64; 2^17 Zipf(1.01) 9.2 -> 7.5,
+     * 10.1 -> 8.4.  Shorter lists are left alone: from 32 windows on, 2^20
+     * Zipf(0.5) keys took 397 us, 307 without any and 315 so. */
+    static constexpr uint32_t kCrowd = 128, kCrowdSkip = 31;
     struct InsertState {
         uint64_t bucket, step, wins, num;
         uint32_t free; /* free slots still to be tried; 0: the window is due */
         val_t expect;  /* payload the slot is expected to hold */
+        uint32_t skip; /* steps to sit out (kCrowd) */
     };
     struct InsertIo {
         uint32_t w[WB <= 128 ? WB / 4 : 1];
@@ -93,6 +102,7 @@ struct MvWalk {
         s.num = 0;
         s.free = 0;
         s.expect = 0;
+        s.skip = 0;
         return kStNone;
     }
 
@@ -105,6 +115,7 @@ struct MvWalk {
     static __device__ __forceinline__ void issue(const Args &a, key_t key, val_t val,
                                                  const InsertState &s, InsertIo &io)
     {
+        if (s.skip) return;
         if (s.free) {
             io.old = cas_slot<L>(slot_of(a, s), key_t(a.t.empty_key), s.expect, key, val,
                                  &io.old_payload);
@@ -123,6 +134,10 @@ struct MvWalk {
     {
         const key_t empty = key_t(a.t.empty_key);
         bool advance = false;
+        if (s.skip) {
+            --s.skip;
+            return false;
+        }
         if (s.free) {
             if (io.old == empty && io.old_payload == s.expect) {
                 counts.fresh += s.num == 0;
@@ -138,6 +153,9 @@ struct MvWalk {
                 join |= st;
                 return true;
             }
+            if (io.old == key && s.wins >= kCrowd)
+                s.skip = (threadIdx.x * 7u + blockIdx.x * 5u + uint32_t(s.num) * 3u) &
+                         kCrowdSkip;
             s.free &= s.free - 1u;
             s.expect = 0;
             advance = s.free == 0;
